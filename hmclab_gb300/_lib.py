@@ -269,6 +269,8 @@ SIGNATURES = {
     "hmc_ess_work_size": [I64, I64, I],
     "hmc_moments": [I, I64, I64, I64, P, P, P, S],
     "hmc_rank_normalize": [I, I64, I64, I64, P, P, S],
+    "hmc_rank_normalize_table": [I, I64, I64, I64, P, P, P, S],
+    "hmc_rank_scores_size": [I64, I64],
     "hmc_graph_begin": [S],
     "hmc_graph_end": [S, _ct.POINTER(c_void_p)],
     "hmc_graph_launch": [P, S],
@@ -278,6 +280,7 @@ _RESTYPES = {
     "hmc_last_error": c_char_p,
     "hmc_launch_count": c_int64,
     "hmc_ess_work_size": c_int64,
+    "hmc_rank_scores_size": c_int64,
     "hmc_tc_partials_size": c_int64,
 }
 

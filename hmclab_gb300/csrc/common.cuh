@@ -147,6 +147,18 @@ __device__ inline void philox_scalars(uint64_t seed, uint32_t chain, uint64_t pr
   *u_acc = u01d(r.z, r.w);
 }
 
+// FP32 to FP64, exact.  The conversion instruction issues at 2 lanes per cycle
+// and SM (measured), like the FP64 pipe it feeds, so sums of FP32 terms in
+// FP64 spent most of their time converting; a normal FP32 value is rebuilt
+// with five integer instructions at 64 lanes per cycle instead: exponent
+// rebased by 1023 - 127, fraction shifted into the high word and the low.
+__device__ __forceinline__ double f64_of(float v) {
+  const uint32_t b = __float_as_uint(v);
+  if ((b & 0x7f800000u) - 0x00800000u >= 0x7f000000u) return (double)v;  // zero, subnormal, inf, NaN
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double f64_of(double v) { return v; }
+
 // ---------------------------------------------------------------------------
 // Per-chain reductions over the [d][C] layout: a block owns 32 consecutive
 // chains (threadIdx.x) and RY row lanes (threadIdx.y); rows are strided by RY

@@ -20,8 +20,11 @@ def rank_normalize(samples, stream=None):
     device tensor of the samples' shape [N][d][C])."""
     N, d, C = samples.shape
     z = _dev.empty((N, d, C), "float64", samples.device)
-    _lib.call("hmc_rank_normalize", _dev.dtype_code(_dev.normalise_dtype(samples.dtype)), N, d, C,
-              samples.data_ptr(), z.data_ptr(), _dev.stream_handle(stream))
+    scores = _dev.empty((_lib.load().hmc_rank_scores_size(N, C),), "float64", samples.device)
+    _lib.call("hmc_rank_normalize_table", _dev.dtype_code(_dev.normalise_dtype(samples.dtype)), N, d, C,
+              samples.data_ptr(), scores.data_ptr(), z.data_ptr(), _dev.stream_handle(stream))
+    if stream is not None:
+        scores.record_stream(stream)  # allocated on the current stream, read on this one
     return z
 
 
