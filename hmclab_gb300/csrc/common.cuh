@@ -147,15 +147,24 @@ __device__ inline void philox_scalars(uint64_t seed, uint32_t chain, uint64_t pr
   *u_acc = u01d(r.z, r.w);
 }
 
-// FP32 to FP64, exact.  The conversion instruction issues at 2 lanes per cycle
-// and SM (measured), like the FP64 pipe it feeds, so sums of FP32 terms in
-// FP64 spent most of their time converting; a normal FP32 value is rebuilt
-// with five integer instructions at 64 lanes per cycle instead: exponent
-// rebased by 1023 - 127, fraction shifted into the high word and the low.
+// FP32 to FP64, exact.  The conversion instruction occupies the FP64 pipe (2
+// lanes per cycle and SM measured, and for its full time when its predicate is
+// false), so FP64 sums of FP32 terms spent most of their time converting.  The
+// words are built with integer instructions at 64 lanes per cycle instead:
+// exponent rebased by 1023 - 127, fraction shifted into the high word and the
+// low; subnormals are scaled by 2^64 first, and zero, infinity and NaN keep
+// their meaning.
 __device__ __forceinline__ double f64_of(float v) {
-  const uint32_t b = __float_as_uint(v);
-  if ((b & 0x7f800000u) - 0x00800000u >= 0x7f000000u) return (double)v;  // zero, subnormal, inf, NaN
-  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+  uint32_t b = __float_as_uint(v), add = 0x38000000u;
+  if ((b & 0x7f800000u) - 0x00800000u >= 0x7f000000u) {
+    if (b & 0x7f800000u) {
+      add = 0x70000000u;  // infinity, NaN: exponent 255 becomes 2047
+    } else {
+      b = __float_as_uint(v * 18446744073709551616.f);
+      add = (b & 0x7fffffffu) ? 0x34000000u : 0u;  // 2^64 less, or zero
+    }
+  }
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + add)), (int)(b << 29));
 }
 __device__ __forceinline__ double f64_of(double v) { return v; }
 

@@ -58,10 +58,9 @@ __device__ __forceinline__ double warp_sum8(const double v[ESS_LAGS], int lane) 
 // eight lags of every half-chain in registers and slides one window of
 // deviations past them, and lags are computed in rounds (8, 16, 32, ...)
 // until every parameter has truncated.  600 parameters x 128 half-chains of
-// 50 draws, 50 lags: 237 us for the rounds of 8, 16 and 26 lags (a first
-// round of 16: 224 us + one round less, but half the parameters stop at 8)
-// against 1242 us with one warp per block converting and centring both
-// factors of every product.  98 M products of all lags take 185 us.
+// 50 draws, 50 lags: 237 us in rounds of 8, 16 and 26 lags against 1242 us
+// with one warp per block that converts and centres both factors of every
+// product; the 98 M products of all lags alone would take 185 us.
 template <typename T, int MODE>
 __global__ void ess_lags_kernel(const T* __restrict__ x, int64_t d, int64_t C, int n, int lag0, int lag1, int lags,
                                 double* __restrict__ part, const double* __restrict__ done) {

@@ -13,7 +13,7 @@
 
 #include <type_traits>
 
-#include "common.cuh"
+#include "columns.cuh"
 
 namespace hmc {
 int gemm_dispatch(int dtype, int64_t m, int64_t n, int64_t k, double alpha, const void* A, const void* B,
@@ -177,29 +177,53 @@ __global__ void draw_z_kernel(ChainView<T> s) {
   }
 }
 
+// (T)(coeff * (double)e).  An FP32 coefficient (1 and 1/2 of the leapfrog) makes
+// the FP64 product exact, so its rounding to FP32 is the FP32 product.
+template <typename T>
+__device__ __forceinline__ T scaled_step(double coeff, bool single, T e) {
+  return single ? (T)coeff * e : (T)(coeff * (double)e);
+}
+inline bool is_single(double coeff) { return (double)(float)coeff == coeff; }
+
+// sqrt of a mass: FP32 through the correctly rounded single-precision root,
+// which equals the FP64 root rounded to FP32.
+__device__ __forceinline__ float mass_root(float m) { return sqrtf(m); }
+__device__ __forceinline__ double mass_root(double m) { return sqrt(m); }
+
 // Momentum (UNIT/DIAG; FULL has p and v = M^-1 p already), K0 in FP64, step
-// size of this trajectory, first drift and reflection.
+// size of this trajectory, first drift and reflection.  Bound by issue (Philox
+// and Box-Muller, 43 % ALU) once the step size is formed once per chain and
+// block and the mass's root in FP32: d = 4096, 1024 chains, diagonal mass,
+// cold cache: 36 us against 561 us with one 8-warp block per 32 chains and an
+// FP64 root and three conversions per element.
 template <typename T, int MASS>
-__global__ void begin_kernel(ChainView<T> s, double drift) {
-  __shared__ double sh[RED_Y][RED_X + 1];
-  const int64_t c = blockIdx.x * (int64_t)RED_X + threadIdx.x;
-  const bool live = c < s.C;
-  const int64_t n = s.control[0];
-  T e = (T)0;
-  if (live) {
-    e = s.eps[c];
-    if (s.randomize) e = (T)((double)step_factor(s, c, n) * (double)e);
+__global__ void __launch_bounds__(COL_THREADS) begin_kernel(ChainView<T> s, double drift, bool single,
+                                                            ColumnShape shape) {
+  __shared__ ColumnShared sh;
+  __shared__ T step[32], first_drift[32];
+  const ColumnTile t = column_tile(shape, s.C);
+  const int64_t n = s.control[0], c = t.c;
+  if ((int)threadIdx.x < (1 << shape.log_x)) {
+    T e = (T)0;
+    if (t.live) {
+      e = s.eps[c];
+      if (s.randomize) e *= step_factor(s, c, n);  // the FP64 product of two T rounds to the product in T
+    }
+    step[t.x] = e;
+    first_drift[t.x] = scaled_step(drift, single, e);  // (drift * eps), then times M^-1 p
+    sh.flag[t.x] = 0;
   }
-  const T ce = (T)(drift * (double)e);  // (drift * eps), then times M^-1 p
+  __syncthreads();
+  const T e = step[t.x], ce = first_drift[t.x];
   double k = 0.0;
   bool oob = false;
-  if (live) {
+  if (t.live) {
     if (MASS == HMC_MASS_FULL) {
-      for (int64_t i = threadIdx.y; i < s.d; i += RED_Y) {
+      for (int64_t i = t.row; i < s.d; i += t.rows) {
         const int64_t idx = i * s.C + c;
         T p = s.p[idx];
         const T mp = s.v[idx];
-        k += (double)p * (double)mp;
+        k += f64_of(p) * f64_of(mp);
         T q = s.q_cur[idx] + ce * mp;
         oob |= reflect(s, i, q, p);
         s.q[idx] = q;
@@ -207,18 +231,21 @@ __global__ void begin_kernel(ChainView<T> s, double drift) {
       }
     } else {
       const int64_t quads = (s.d + 3) / 4;
-      for (int64_t qd = threadIdx.y; qd < quads; qd += RED_Y) {
-        T z[4];
+      for (int64_t qd = t.row; qd < quads; qd += t.rows) {
+        const int64_t i0 = 4 * qd, k0 = i0 * s.C + c;
+        T qc[4], z[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) qc[j] = i0 + j < s.d ? s.q_cur[k0 + j * s.C] : (T)0;
         draw_z4(s, qd, c, n, z);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int64_t i = 4 * qd + j;
+          const int64_t i = i0 + j;
           if (i < s.d) {
-            const int64_t idx = i * s.C + c;
-            T p = MASS == HMC_MASS_DIAG ? (T)sqrt((double)s.mdiag[i]) * z[j] : z[j];
+            const int64_t idx = k0 + j * s.C;
+            T p = MASS == HMC_MASS_DIAG ? mass_root(s.mdiag[i]) * z[j] : z[j];
             const T mp = minv_p<T, MASS>(s, i, idx, p);
-            k += (double)p * (double)mp;
-            T q = s.q_cur[idx] + ce * mp;
+            k += f64_of(p) * f64_of(mp);
+            T q = qc[j] + ce * mp;
             oob |= reflect(s, i, q, p);
             s.q[idx] = q;
             s.p[idx] = p;
@@ -227,79 +254,117 @@ __global__ void begin_kernel(ChainView<T> s, double drift) {
       }
     }
   }
-  const double ksum = block_chain_sum(k, sh);
-  __shared__ int oob_any[RED_X];
-  if (threadIdx.y == 0) oob_any[threadIdx.x] = 0;
-  __syncthreads();
-  if (oob) atomicOr(&oob_any[threadIdx.x], 1);
-  __syncthreads();
-  if (live && threadIdx.y == 0) {
+  if (oob) atomicOr(&sh.flag[t.x], 1);
+  const double ksum = column_total(shape, k, sh);  // orders the flags too
+  if (t.first && t.live) {
+    int out = 0;
+    for (int r = 0; r < shape.cluster; ++r) out |= column_flag(shape, sh, t.x, r);
     s.k_cur[c] = 0.5 * ksum;
     s.eps_local[c] = e;
-    s.flags[c] = oob_any[threadIdx.x] ? HMC_FLAG_OUT_OF_BOUNDS : 0;
+    s.flags[c] = out ? HMC_FLAG_OUT_OF_BOUNDS : 0;
   }
+  if (shape.cluster > 1) column_sync(shape);
 }
 
+// VEC consecutive chains in one access of 16 bytes.
+template <typename T, int VEC>
+struct alignas(sizeof(T) * VEC) Pack {
+  T v[VEC];
+};
+constexpr int KICK_ROWS = 2;  // rows of a thread loaded together
+
 // p -= kick * eps * g; q += drift * eps * M^-1 p; reflect.  For FULL the kick
-// and the drift are split around the host-issued v = M^-1 p product.
-template <typename T, int MASS, int DO_KICK, int DO_DRIFT>
-__global__ void kick_drift_kernel(ChainView<T> s, double kick, double drift) {
-  const int64_t total = s.d * s.C;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = idx % s.C, i = idx / s.C;
-    const T e = s.eps_local[c];
-    T p = s.p[idx];
-    if (DO_KICK) {
-      const T ck = (T)(kick * (double)e * (s.beta ? s.beta[c] : 1.0));
-      p -= ck * s.g[idx];
+// and the drift are split around the host-issued v = M^-1 p product.  A thread
+// owns VEC chains and walks rows, so the step sizes and the index arithmetic
+// are paid per chain instead of per element (where FP64 products and 64-bit
+// divisions bounded it); d = 4096, 1024 chains, cold
+// cache: 15 us for 84 MB (5.6 TB/s) against 41 us.
+template <typename T, int MASS, int DO_KICK, int DO_DRIFT, int VEC>
+__global__ void __launch_bounds__(256, 4) kick_drift_kernel(ChainView<T> s, double kick, double drift, bool single) {
+  using V = Pack<T, VEC>;
+  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * VEC;
+  if (c >= s.C) return;
+  T ck[VEC], cd[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) {
+    const T e = s.eps_local[c + v];
+    if (DO_KICK) ck[v] = s.beta ? (T)(kick * (double)e * s.beta[c + v]) : scaled_step(kick, single, e);
+    if (DO_DRIFT) cd[v] = scaled_step(drift, single, e);
+  }
+  const int64_t stride = (int64_t)gridDim.y * blockDim.y;
+  for (int64_t r0 = blockIdx.y * (int64_t)blockDim.y + threadIdx.y; r0 < s.d; r0 += KICK_ROWS * stride) {
+    V p[KICK_ROWS], q[KICK_ROWS], w[KICK_ROWS];  // w: the gradient, or v = M^-1 p of a full mass
+#pragma unroll
+    for (int u = 0; u < KICK_ROWS; ++u) {
+      const int64_t i = r0 + u * stride;
+      if (i >= s.d) break;
+      const int64_t idx = i * s.C + c;
+      p[u] = *(const V*)(s.p + idx);
+      if (DO_KICK) w[u] = *(const V*)(s.g + idx);
+      if (DO_DRIFT) q[u] = *(const V*)(s.q + idx);
+      if (DO_DRIFT && MASS == HMC_MASS_FULL) w[u] = *(const V*)(s.v + idx);
     }
-    if (DO_DRIFT) {
-      const T cd = (T)(drift * (double)e);
-      T q = s.q[idx] + cd * minv_p<T, MASS>(s, i, idx, p);
-      if (s.lo || s.hi) {
-        if (reflect(s, i, q, p)) atomicOr(&s.flags[c], HMC_FLAG_OUT_OF_BOUNDS);
+#pragma unroll
+    for (int u = 0; u < KICK_ROWS; ++u) {
+      const int64_t i = r0 + u * stride;
+      if (i >= s.d) break;
+      const int64_t idx = i * s.C + c;
+      const T mi = DO_DRIFT && MASS == HMC_MASS_DIAG ? s.minv[i] : (T)1;
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        if (DO_KICK) p[u].v[v] -= ck[v] * w[u].v[v];
+        if (DO_DRIFT) {
+          const T mp = MASS == HMC_MASS_FULL ? w[u].v[v] : (MASS == HMC_MASS_DIAG ? mi * p[u].v[v] : p[u].v[v]);
+          q[u].v[v] = q[u].v[v] + cd[v] * mp;
+          if (s.lo || s.hi) {
+            if (reflect(s, i, q[u].v[v], p[u].v[v])) atomicOr(&s.flags[c + v], HMC_FLAG_OUT_OF_BOUNDS);
+          }
+        }
       }
-      s.q[idx] = q;
+      if (DO_DRIFT) *(V*)(s.q + idx) = q[u];
+      if (DO_KICK || s.lo || s.hi) *(V*)(s.p + idx) = p[u];
     }
-    s.p[idx] = p;
   }
 }
 
 // FP64 kinetic energy of p (MASS != FULL) or of (p, v = M^-1 p) (FULL).
 template <typename T, int MASS>
-__device__ __forceinline__ double kinetic_partial(const ChainView<T>& s, const T* p, const T* mp_full, int64_t c) {
+__device__ __forceinline__ double kinetic_partial(const ChainView<T>& s, const T* __restrict__ p,
+                                                  const T* __restrict__ mp_full, const ColumnTile& t) {
   double k = 0.0;
-  for (int64_t i = threadIdx.y; i < s.d; i += RED_Y) {
-    const int64_t idx = i * s.C + c;
+#pragma unroll 8
+  for (int64_t i = t.row; i < s.d; i += t.rows) {
+    const int64_t idx = i * s.C + t.c;
     const T pi = p[idx];
     const T mp = MASS == HMC_MASS_UNIT ? pi : (MASS == HMC_MASS_DIAG ? s.minv[i] * pi : mp_full[idx]);
-    k += (double)pi * (double)mp;
+    k += f64_of(pi) * f64_of(mp);
   }
   return k;
 }
 
 template <typename T, int MASS>
-__global__ void kinetic_kernel(ChainView<T> s, const T* p, const T* mp_full, double* out) {
-  __shared__ double sh[RED_Y][RED_X + 1];
-  const int64_t c = blockIdx.x * (int64_t)RED_X + threadIdx.x;
-  const double k = c < s.C ? kinetic_partial<T, MASS>(s, p, mp_full, c) : 0.0;
-  const double ks = block_chain_sum(k, sh);
-  if (c < s.C && threadIdx.y == 0) out[c] = 0.5 * ks;
+__global__ void __launch_bounds__(COL_THREADS) kinetic_kernel(ChainView<T> s, const T* p, const T* mp_full, double* out,
+                                                              ColumnShape shape) {
+  __shared__ ColumnShared sh;
+  const ColumnTile t = column_tile(shape, s.C);
+  const double ks = column_total(shape, t.live ? kinetic_partial<T, MASS>(s, p, mp_full, t) : 0.0, sh);
+  if (t.first && t.live) out[t.c] = 0.5 * ks;
+  if (shape.cluster > 1) column_sync(shape);
 }
 
+// K1, the accept test (FP64, one thread per chain), and the accepted or kept
+// position into q_cur and the sample ring.  Bound by memory latency; d = 4096,
+// 1024 chains, cold cache: 37 us against 565 us.
 template <typename T, int MASS>
-__global__ void end_kernel(ChainView<T> s) {
-  __shared__ double sh[RED_Y][RED_X + 1];
-  __shared__ int acc_flag[RED_X];
-  const int64_t c = blockIdx.x * (int64_t)RED_X + threadIdx.x;
-  const bool live = c < s.C;
+__global__ void __launch_bounds__(COL_THREADS) end_kernel(ChainView<T> s, ColumnShape shape) {
+  __shared__ ColumnShared sh;
+  const ColumnTile t = column_tile(shape, s.C);
+  const int64_t c = t.c;
   const int64_t n = s.control[0];
-  const double k = live ? kinetic_partial<T, MASS>(s, s.p, s.v, c) : 0.0;
-  const double ks = block_chain_sum(k, sh);
-  if (threadIdx.y == 0) {
+  const double ks = column_total(shape, t.live ? kinetic_partial<T, MASS>(s, s.p, s.v, t) : 0.0, sh);
+  if (t.first) {
     int accept = 0;
-    if (live) {
+    if (t.live) {
       const double k1 = 0.5 * ks;
       s.k_prop[c] = k1;
       double x1 = s.x_prop[c];
@@ -336,39 +401,43 @@ __global__ void end_kernel(ChainView<T> s) {
         s.accepted[c] += 1;
       }
     }
-    acc_flag[threadIdx.x] = accept;
+    sh.flag[t.x] = accept;
   }
-  __syncthreads();
+  column_sync(shape);
   const bool record = s.ring_q != nullptr && (n % s.thin) == 0;
   const int64_t slot = record ? (n / s.thin) % s.ring_slots : 0;
-  if (live) {
-    const bool acc = acc_flag[threadIdx.x] != 0;
-    for (int64_t i = threadIdx.y; i < s.d; i += RED_Y) {
-      const int64_t idx = i * s.C + c;
-      T qv;
-      if (acc) {
-        qv = s.q[idx];
-        s.q_cur[idx] = qv;
-      } else if (record) {
-        qv = s.q_cur[idx];
+  const bool acc = column_flag(shape, sh, t.x, 0) != 0;
+  if (t.live && (acc || record)) {
+    const T* __restrict__ from = acc ? s.q : s.q_cur;
+    T* ring = record ? s.ring_q + slot * s.d * s.C : nullptr;
+    constexpr int U = 8;  // rows loaded together
+    for (int64_t i0 = t.row; i0 < s.d; i0 += U * t.rows) {
+      T qv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = i0 + u * t.rows;
+        if (i < s.d) qv[u] = from[i * s.C + c];
       }
-      if (record) s.ring_q[slot * s.d * s.C + idx] = qv;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = i0 + u * t.rows;
+        if (i >= s.d) break;
+        if (acc) s.q_cur[i * s.C + c] = qv[u];
+        if (record) ring[i * s.C + c] = qv[u];
+      }
     }
-    if (record && threadIdx.y == 0) s.ring_x[slot * s.C + c] = s.beta ? s.beta[c] * s.x_cur[c] : s.x_cur[c];
   }
+  if (record && t.first && t.live) s.ring_x[slot * s.C + c] = s.beta ? s.beta[c] * s.x_cur[c] : s.x_cur[c];
   // The last block to finish advances the proposal counter.
-  __shared__ bool last;
   __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
+  column_sync(shape);  // and no block of the tile leaves while its flags are read
+  if (threadIdx.x == 0) {
     const unsigned long long prev = atomicAdd((unsigned long long*)&s.control[1], 1ull);
-    last = prev == (unsigned long long)(gridDim.x - 1);
-  }
-  __syncthreads();
-  if (last && threadIdx.x == 0 && threadIdx.y == 0) {
-    s.control[0] = n + 1;
-    s.control[1] = 0;
-    __threadfence();
+    if (prev == (unsigned long long)(gridDim.x - 1)) {
+      s.control[0] = n + 1;
+      s.control[1] = 0;
+      __threadfence();
+    }
   }
 }
 
@@ -401,14 +470,13 @@ template <typename T>
 int begin_impl(const hmc_chains* s, double drift, cudaStream_t st) {
   HMC_TRY(check_state<T>(s, "hmc_begin_trajectory"));
   ChainView<T> v = view<T>(s);
-  const dim3 grid = red_grid(s->chains), block = red_block();
+  const ColumnShape shape = column_shape(s->chains, s->dims);
+  const char* who = "begin_kernel";
   switch (s->mass_kind) {
     case HMC_MASS_UNIT:
-      begin_kernel<T, HMC_MASS_UNIT><<<grid, block, 0, st>>>(v, drift);
-      break;
+      return launch_columns(who, begin_kernel<T, HMC_MASS_UNIT>, shape, s->chains, st, v, drift, is_single(drift), shape);
     case HMC_MASS_DIAG:
-      begin_kernel<T, HMC_MASS_DIAG><<<grid, block, 0, st>>>(v, drift);
-      break;
+      return launch_columns(who, begin_kernel<T, HMC_MASS_DIAG>, shape, s->chains, st, v, drift, is_single(drift), shape);
     default: {
       const int64_t quads = (s->dims + 3) / 4;
       draw_z_kernel<T><<<ew_grid(quads * s->chains), 256, 0, st>>>(v);
@@ -417,10 +485,42 @@ int begin_impl(const hmc_chains* s, double drift, cudaStream_t st) {
       // p = L z, then v = M^-1 p.
       HMC_TRY(gemm_dispatch(dt, s->dims, s->chains, s->dims, 1.0, s->mass_chol, s->v, nullptr, s->p, 0, st));
       HMC_TRY(gemm_dispatch(dt, s->dims, s->chains, s->dims, 1.0, s->mass_inv, s->p, nullptr, s->v, 0, st));
-      begin_kernel<T, HMC_MASS_FULL><<<grid, block, 0, st>>>(v, drift);
+      return launch_columns(who, begin_kernel<T, HMC_MASS_FULL>, shape, s->chains, st, v, drift, is_single(drift), shape);
     }
   }
-  return check_launch("begin_kernel");
+}
+
+// Threads (x over chains, y over rows) and grid of the kick: at least the
+// rows a thread loads together, which also share the per-chain work.
+template <typename T, int MASS, int VEC>
+int kick_drift_launch(const ChainView<T>& v, bool do_kick, bool do_drift, double kick, double drift,
+                      cudaStream_t st) {
+  const int64_t cols = (v.C + VEC - 1) / VEC;
+  unsigned bx = 1;
+  while (bx < 256 && bx < cols) bx *= 2;
+  const dim3 block(bx, 256 / bx);
+  int64_t gy = (v.d + KICK_ROWS * block.y - 1) / (KICK_ROWS * block.y);
+  const int64_t gx = (cols + bx - 1) / bx;
+  while (gy > 1 && gx * gy > 152 * 16) gy = (gy + 1) / 2;
+  HMC_REQUIRE(gx <= 0x7FFFFFFF, "hmc_kick_drift: too many chains");
+  const dim3 grid((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535));
+  const bool single = is_single(kick) && is_single(drift);
+  if (do_kick && do_drift)
+    kick_drift_kernel<T, MASS, 1, 1, VEC><<<grid, block, 0, st>>>(v, kick, drift, single);
+  else if (do_kick)
+    kick_drift_kernel<T, MASS, 1, 0, VEC><<<grid, block, 0, st>>>(v, kick, drift, single);
+  else
+    kick_drift_kernel<T, MASS, 0, 1, VEC><<<grid, block, 0, st>>>(v, kick, drift, single);
+  return check_launch("kick_drift_kernel");
+}
+
+template <typename T, int MASS>
+int kick_drift_any(const ChainView<T>& v, bool do_kick, bool do_drift, double kick, double drift, cudaStream_t st) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  // 16-byte accesses need every row of the [d][C] state on a 16-byte boundary
+  const bool vec = v.C % VEC == 0 && ((uintptr_t)v.q | (uintptr_t)v.p | (uintptr_t)v.g | (uintptr_t)v.v) % 16 == 0;
+  return vec ? kick_drift_launch<T, MASS, VEC>(v, do_kick, do_drift, kick, drift, st)
+             : kick_drift_launch<T, MASS, 1>(v, do_kick, do_drift, kick, drift, st);
 }
 
 template <typename T>
@@ -428,60 +528,43 @@ int kick_drift_impl(const hmc_chains* s, double kick, double drift, cudaStream_t
   HMC_TRY(check_state<T>(s, "hmc_kick_drift"));
   HMC_REQUIRE(s->g != nullptr, "hmc_kick_drift: missing gradient buffer");
   ChainView<T> v = view<T>(s);
-  const unsigned grid = ew_grid(s->dims * s->chains);
   const bool do_drift = drift != 0.0;
   const bool do_kick = kick != 0.0;
   HMC_REQUIRE(do_kick || do_drift, "hmc_kick_drift: kick and drift are both zero");
   switch (s->mass_kind) {
     case HMC_MASS_UNIT:
-      if (do_kick && do_drift)
-        kick_drift_kernel<T, HMC_MASS_UNIT, 1, 1><<<grid, 256, 0, st>>>(v, kick, drift);
-      else if (do_kick)
-        kick_drift_kernel<T, HMC_MASS_UNIT, 1, 0><<<grid, 256, 0, st>>>(v, kick, drift);
-      else
-        kick_drift_kernel<T, HMC_MASS_UNIT, 0, 1><<<grid, 256, 0, st>>>(v, kick, drift);
-      break;
+      return kick_drift_any<T, HMC_MASS_UNIT>(v, do_kick, do_drift, kick, drift, st);
     case HMC_MASS_DIAG:
-      if (do_kick && do_drift)
-        kick_drift_kernel<T, HMC_MASS_DIAG, 1, 1><<<grid, 256, 0, st>>>(v, kick, drift);
-      else if (do_kick)
-        kick_drift_kernel<T, HMC_MASS_DIAG, 1, 0><<<grid, 256, 0, st>>>(v, kick, drift);
-      else
-        kick_drift_kernel<T, HMC_MASS_DIAG, 0, 1><<<grid, 256, 0, st>>>(v, kick, drift);
-      break;
+      return kick_drift_any<T, HMC_MASS_DIAG>(v, do_kick, do_drift, kick, drift, st);
     default: {
       if (do_kick) {
-        kick_drift_kernel<T, HMC_MASS_FULL, 1, 0><<<grid, 256, 0, st>>>(v, kick, drift);
-        if (!do_drift) break;
-        HMC_TRY(check_launch("kick_kernel"));
+        HMC_TRY((kick_drift_any<T, HMC_MASS_FULL>(v, true, false, kick, drift, st)));
+        if (!do_drift) return HMC_OK;
       }
       const int dt = std::is_same<T, double>::value ? HMC_F64 : HMC_F32;
       HMC_TRY(gemm_dispatch(dt, s->dims, s->chains, s->dims, 1.0, s->mass_inv, s->p, nullptr, s->v, 0, st));
-      kick_drift_kernel<T, HMC_MASS_FULL, 0, 1><<<grid, 256, 0, st>>>(v, kick, drift);
+      return kick_drift_any<T, HMC_MASS_FULL>(v, false, true, kick, drift, st);
     }
   }
-  return check_launch("kick_drift_kernel");
 }
 
 template <typename T>
 int end_impl(const hmc_chains* s, cudaStream_t st) {
   HMC_TRY(check_state<T>(s, "hmc_end_trajectory"));
   ChainView<T> v = view<T>(s);
-  const dim3 grid = red_grid(s->chains), block = red_block();
+  const ColumnShape shape = column_shape(s->chains, s->dims);
+  const char* who = "end_kernel";
   switch (s->mass_kind) {
     case HMC_MASS_UNIT:
-      end_kernel<T, HMC_MASS_UNIT><<<grid, block, 0, st>>>(v);
-      break;
+      return launch_columns(who, end_kernel<T, HMC_MASS_UNIT>, shape, s->chains, st, v, shape);
     case HMC_MASS_DIAG:
-      end_kernel<T, HMC_MASS_DIAG><<<grid, block, 0, st>>>(v);
-      break;
+      return launch_columns(who, end_kernel<T, HMC_MASS_DIAG>, shape, s->chains, st, v, shape);
     default: {
       const int dt = std::is_same<T, double>::value ? HMC_F64 : HMC_F32;
       HMC_TRY(gemm_dispatch(dt, s->dims, s->chains, s->dims, 1.0, s->mass_inv, s->p, nullptr, s->v, 0, st));
-      end_kernel<T, HMC_MASS_FULL><<<grid, block, 0, st>>>(v);
+      return launch_columns(who, end_kernel<T, HMC_MASS_FULL>, shape, s->chains, st, v, shape);
     }
   }
-  return check_launch("end_kernel");
 }
 
 template <typename T>
@@ -489,23 +572,25 @@ int kinetic_impl(const hmc_chains* s, const void* p, double* out, cudaStream_t s
   HMC_REQUIRE(s && p && out, "hmc_kinetic_energy: null argument");
   HMC_REQUIRE(s->dims > 0 && s->chains > 0, "hmc_kinetic_energy: bad sizes");
   ChainView<T> v = view<T>(s);
-  const dim3 grid = red_grid(s->chains), block = red_block();
+  const ColumnShape shape = column_shape(s->chains, s->dims);
+  const char* who = "kinetic_kernel";
+  const T* pt = (const T*)p;
   switch (s->mass_kind) {
     case HMC_MASS_UNIT:
-      kinetic_kernel<T, HMC_MASS_UNIT><<<grid, block, 0, st>>>(v, (const T*)p, nullptr, out);
-      break;
+      return launch_columns(who, kinetic_kernel<T, HMC_MASS_UNIT>, shape, s->chains, st, v, pt, (const T*)nullptr, out,
+                            shape);
     case HMC_MASS_DIAG:
       HMC_REQUIRE(s->mass_inv_diag, "hmc_kinetic_energy: missing inverse diagonal");
-      kinetic_kernel<T, HMC_MASS_DIAG><<<grid, block, 0, st>>>(v, (const T*)p, nullptr, out);
-      break;
+      return launch_columns(who, kinetic_kernel<T, HMC_MASS_DIAG>, shape, s->chains, st, v, pt, (const T*)nullptr, out,
+                            shape);
     default: {
       HMC_REQUIRE(s->mass_inv && s->v, "hmc_kinetic_energy: full mass needs inverse and v");
       const int dt = std::is_same<T, double>::value ? HMC_F64 : HMC_F32;
       HMC_TRY(gemm_dispatch(dt, s->dims, s->chains, s->dims, 1.0, s->mass_inv, p, nullptr, s->v, 0, st));
-      kinetic_kernel<T, HMC_MASS_FULL><<<grid, block, 0, st>>>(v, (const T*)p, (const T*)s->v, out);
+      return launch_columns(who, kinetic_kernel<T, HMC_MASS_FULL>, shape, s->chains, st, v, pt, (const T*)s->v, out,
+                            shape);
     }
   }
-  return check_launch("kinetic_kernel");
 }
 
 template <typename T>
