@@ -501,7 +501,7 @@ extern "C" HMC_API int hmc_rank_normalize_table(int dtype, int64_t N, int64_t d,
   HMC_REQUIRE(S < (1ll << 31) / 2, "hmc_rank_normalize: too many draws per parameter");
   // the documented size limit of the entry point
   HMC_REQUIRE((double)S * (double)S * (double)d <= 1.1e12,
-              "hmc_rank_normalize: S^2 d = %.3g is beyond this estimator's limit (1.1e12)",
+              "hmc_rank_normalize: S^2 d = %.3g is beyond this estimator's budget (1.1e12)",
               (double)S * (double)S * (double)d);
   return HMC_DISPATCH(dtype, T, [&] {
     return rank_normalize<T>(N, d, C, (const T*)samples, scores, z, as_stream(stream));
