@@ -610,11 +610,11 @@ def dominant_kernel_timing(post, smp, n_iter=20):
     lik = post.separate_distributions[1] if hasattr(post, "separate_distributions") else post
     if getattr(smp, "_persistent", None) is not None:
         B = smp.proposals_per_graph
-        if smp._persistent.warps is None:
+        if smp._persistent.shape is None:
             smp._persistent.autotune(h)
 
         def launch():  # one block of proposals, writing no state
-            smp._persistent._call(B, smp._persistent.warps, True, h)
+            smp._persistent._call(B, smp._persistent.shape, True, h)
     elif smp._fused is not None:
         smp._fused.after_begin(h)
 
@@ -1337,7 +1337,7 @@ def run_profile_case(a):
                                             proposals_per_graph=10, persistent=True)
         smp.run(10 * (a.repeat + 1))
         smp.finish()
-        print(f"persistent: d={d} chains={a.chains} warps={smp._persistent.warps} ok")
+        print(f"persistent: d={d} chains={a.chains} shape={smp._persistent.shape} ok")
     elif a.case in ("tomo", "srcloc"):
         import numpy as np
 

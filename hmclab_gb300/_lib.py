@@ -29,6 +29,8 @@ HMC_MASS_FULL = 2
 
 HMC_FLAG_OUT_OF_BOUNDS = 1
 
+HMC_PERSISTENT_WARPS, HMC_PERSISTENT_LANES, HMC_PERSISTENT_ROWS = 0, 1, 2
+
 HMC_CSR_GATHER, HMC_CSR_GATHER4, HMC_CSR_SLAB = 0, 1, 2
 
 c_void_p = _ct.c_void_p
@@ -231,6 +233,7 @@ SIGNATURES = {
     "hmc_gemm": [I, I64, I64, I64, D, P, P, P, P, I, S],
     "hmc_exchange": [P, I64, P, P, P, P, S],
     "hmc_persistent_dense": [P, P, P, D, I, P, P, P, I64, I, I, S],
+    "hmc_persistent_dense_shaped": [P, P, P, D, I, P, P, P, I64, I, I, I, I, S],
     "hmc_persistent_dense_groups": [P, I, P, I64, I, I, S],
     "hmc_gemm_splitk": [I, I64, I64, I64, D, P, P, P, I, P, I64, S],
     "hmc_split_bf16": [I64, I64, P, I64, P, P, S],

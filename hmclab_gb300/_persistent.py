@@ -1,6 +1,8 @@
 """Persistent fused proposals (csrc/persistent.cu) for small dense
-linear-Gaussian posteriors: whole blocks of proposals in one launch, one warp
-per chain, with an autotuner that picks the chains per block.
+linear-Gaussian posteriors: whole blocks of proposals in one launch.  The
+kernel follows from the problem (`kernel_of`), because the kernels add the
+energies of a chain in different orders; the autotuner picks its launch shape,
+which does not change results.
 
 Applies when the target is a premultiplied dense `LinearMatrix` with
 d <= 128, alone or in a `BayesRule` with one diagonal `Normal` or `Laplace`
@@ -21,6 +23,52 @@ def _smem(d, full, warps, esize):
     """Shared memory of one block: GtG (and M^-1, L for a full mass) with an
     odd row stride, plus one vector per warp (as in csrc/persistent.cu)."""
     return ((3 if full else 1) * d * (d | 1) + warps * d) * esize
+
+
+def _lanes_smem(d, steps, chains_per_warp, warps, esize):
+    """Upper bound of one block's shared memory in csrc/persistent_lanes.cu:
+    the chains' vectors and step coefficients, and GtG."""
+    return ((d + 16 + 2 * steps) * warps * chains_per_warp + d * (d | 1)) * esize
+
+
+def _cluster(d, chains, esize):
+    """Blocks per chain of the rows kernel: one per 16 FP64 or 32 FP32 rows, as
+    long as every block has an SM of its own; FP64 products of more than 64
+    rows need two blocks of 512 threads.  Measured per proposal (10 steps,
+    FP64): d = 50, one chain 28.9 / 21.6 / 19.0 / 20.1 us on 1 / 2 / 4 / 8
+    blocks, 64 chains 28.9 / 21.7 / 25.8 / 42.5; d = 100, one chain 39.1 /
+    25.1 / 23.3 us on 2 / 4 / 8; FP32, d = 128, one chain 16.8 / 15.6 / 14.1 /
+    14.7 us on 1 / 2 / 4 / 8."""
+    rows = 16 if esize == 8 else 32
+    r = 1
+    while r < 8 and r * rows < d and 2 * r * chains <= 152:
+        r *= 2
+    return max(r, 2) if esize == 8 and d > 64 else r
+
+
+def _rows_kernel(d, chains, esize):
+    """Whether several lanes per row (one chain per cluster) beat one lane per
+    row.  FP64: while the chains leave SMs without one; a lone warp issues
+    FP64 at a quarter of its SM's rate (d = 50, one chain: 19 us per proposal
+    against 64 us; 304 chains 52 against 64, 1024 chains 177 against 90; d =
+    30, 304 chains 34 against 28).  FP32: beyond the 64 columns that the lanes
+    kernel holds in registers (d = 100, 152 chains 15 against 26 us, 304
+    chains 29 against 26; d = 50, one chain 11.4 against 6.4)."""
+    if esize == 8:
+        return chains <= (152 if d <= 32 else 304)
+    return d > 64 and chains <= 152
+
+
+def kernel_of(d, chains, esize, full, steps):
+    """(kernel, launch shapes the autotuner may choose from) of one problem."""
+    if full:
+        return [(_lib.HMC_PERSISTENT_WARPS, w, 0) for w in _WARPS if _smem(d, full, w, esize) <= _SMEM]
+    if _rows_kernel(d, chains, esize):
+        return [(_lib.HMC_PERSISTENT_ROWS, _cluster(d, chains, esize), 0)]
+    return [(_lib.HMC_PERSISTENT_LANES, ct, w) for ct in ((1, 2, 4) if esize == 4 else (1, 2)) for w in (1, 2, 4, 8)
+            if _lanes_smem(d, steps, ct, w, esize) <= _SMEM]
+
+
 # chosen launch shapes, per (dimension, chains, dtype, mass, prior, schedule length)
 _tuned = {}
 
@@ -91,38 +139,38 @@ class PersistentDense:
         self.schedule = _schedule(first, steps)
         self._sched_ref = _ct.byref(self.schedule)
         self.key = (sampler.dimensions, sampler.chains, dt, sampler.mass_matrix.kind, self.prior_kind, len(steps))
-        self.warps = _tuned.get(self.key)
+        self.shape = _tuned.get(self.key)
 
-    def _call(self, n, warps, dry, h):
-        _lib.call("hmc_persistent_dense", self.smp._state_ref, self.GtG.data_ptr(), self.Gtd0.data_ptr(), self.dtd,
-                  self.prior_kind, self.pmean.data_ptr() if self.pmean is not None else None,
-                  self.pw.data_ptr() if self.pw is not None else None, self._sched_ref, n, warps, int(dry), h)
+    def _call(self, n, shape, dry, h):
+        _lib.call("hmc_persistent_dense_shaped", self.smp._state_ref, self.GtG.data_ptr(), self.Gtd0.data_ptr(),
+                  self.dtd, self.prior_kind, self.pmean.data_ptr() if self.pmean is not None else None,
+                  self.pw.data_ptr() if self.pw is not None else None, self._sched_ref, n, *shape, int(dry), h)
 
     def autotune(self, h, proposals=4):
-        """Time every chains-per-block choice on dry runs (which write no
-        state) of the live chains and keep the fastest (cached per problem
-        shape by hmclab_gb300.autotune, in memory and on disk)."""
+        """Time the launch shapes of this problem's kernel on dry runs (which
+        write no state) of the live chains and keep the fastest (cached per
+        problem shape by hmclab_gb300.autotune, in memory and on disk)."""
         from hmclab_gb300 import autotune as _autotune
 
-        if self.warps is not None:
-            return self.warps
+        if self.shape is not None:
+            return self.shape
         slen = self.smp._state.stream_len
         if slen > 0:
             proposals = min(proposals, slen)
         full = self.smp.mass_matrix.kind == _lib.HMC_MASS_FULL
         esize = 8 if self.smp.dtype == "float64" else 4
-        cands = [(w,) for w in _WARPS if _smem(self.smp.dimensions, full, w, esize) <= _SMEM]
+        cands = kernel_of(self.key[0], self.key[1], esize, full, self.key[5])
         shape = {"d": self.key[0], "C": self.key[1], "dtype": self.key[2], "mass": int(self.key[3]),
                  "prior": self.key[4], "steps": self.key[5]}
-        (self.warps,) = _autotune.choose("persistent_dense", shape, cands,
-                                         lambda c: self._call(proposals, c[0], True, h), self.smp.device, h, reps=1)
-        _tuned[self.key] = self.warps
-        return self.warps
+        self.shape = cands[0] if len(cands) == 1 else _autotune.choose(
+            "persistent_shapes", shape, cands, lambda c: self._call(proposals, c, True, h), self.smp.device, h, reps=1)
+        _tuned[self.key] = self.shape
+        return self.shape
 
     def run(self, n, h):
-        if self.warps is None:
+        if self.shape is None:
             self.autotune(h)
-        self._call(n, self.warps, False, h)
+        self._call(n, self.shape, False, h)
 
 
 def run_groups(samplers, n_proposals, warps=None):

@@ -98,42 +98,64 @@ __device__ inline double u01d(uint32_t a, uint32_t b) {
   return ((double)v + 0.5) * (1.0 / 9007199254740992.0);
 }
 
-// Four standard normals for (row quad, chain, proposal) by Box-Muller.
+// Four uniforms for (row quad, chain, proposal), and the two halves of
+// Box-Muller: z = radius(u0) (cos, sin)(angle(u1)), radius(u2) (cos, sin)(angle(u3)).
 template <typename T>
-__device__ inline void philox_normal4(uint64_t seed, uint32_t quad, uint32_t chain, uint64_t proposal,
-                                      uint32_t purpose, T out[4]);
+__device__ inline void philox_uniforms4(uint64_t seed, uint32_t quad, uint32_t chain, uint64_t proposal,
+                                        uint32_t purpose, T u[4]);
 
 template <>
-__device__ inline void philox_normal4<float>(uint64_t seed, uint32_t quad, uint32_t chain,
-                                             uint64_t proposal, uint32_t purpose, float out[4]) {
+__device__ inline void philox_uniforms4<float>(uint64_t seed, uint32_t quad, uint32_t chain, uint64_t proposal,
+                                               uint32_t purpose, float u[4]) {
   const uint4 r = philox4x32_10(
       make_uint4(quad, chain, (uint32_t)proposal, ((uint32_t)(proposal >> 32) & 0x0FFFFFFFu) | (purpose << 28)),
       make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
-  const float u1 = u01f(r.x), u2 = u01f(r.y), u3 = u01f(r.z), u4 = u01f(r.w);
-  const float a = sqrtf(-2.0f * logf(u1)), b = sqrtf(-2.0f * logf(u3));
-  const float t1 = 6.283185307179586f * u2, t2 = 6.283185307179586f * u4;
-  out[0] = a * cosf(t1);
-  out[1] = a * sinf(t1);
-  out[2] = b * cosf(t2);
-  out[3] = b * sinf(t2);
+  u[0] = u01f(r.x);
+  u[1] = u01f(r.y);
+  u[2] = u01f(r.z);
+  u[3] = u01f(r.w);
 }
 
 template <>
-__device__ inline void philox_normal4<double>(uint64_t seed, uint32_t quad, uint32_t chain,
-                                              uint64_t proposal, uint32_t purpose, double out[4]) {
+__device__ inline void philox_uniforms4<double>(uint64_t seed, uint32_t quad, uint32_t chain, uint64_t proposal,
+                                                uint32_t purpose, double u[4]) {
   // Two Philox blocks give 53-bit uniforms for the FP64 verification mode.
   const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
   const uint32_t w = ((uint32_t)(proposal >> 32) & 0x07FFFFFFu) | (purpose << 28);
   const uint4 r0 = philox4x32_10(make_uint4(quad, chain, (uint32_t)proposal, w), key);
   const uint4 r1 = philox4x32_10(make_uint4(quad, chain, (uint32_t)proposal, w | 0x08000000u), key);
-  const double u1 = u01d(r0.x, r0.y), u2 = u01d(r0.z, r0.w);
-  const double u3 = u01d(r1.x, r1.y), u4 = u01d(r1.z, r1.w);
-  const double a = sqrt(-2.0 * log(u1)), b = sqrt(-2.0 * log(u3));
-  const double t1 = 6.283185307179586 * u2, t2 = 6.283185307179586 * u4;
-  out[0] = a * cos(t1);
-  out[1] = a * sin(t1);
-  out[2] = b * cos(t2);
-  out[3] = b * sin(t2);
+  u[0] = u01d(r0.x, r0.y);
+  u[1] = u01d(r0.z, r0.w);
+  u[2] = u01d(r1.x, r1.y);
+  u[3] = u01d(r1.z, r1.w);
+}
+
+__device__ __forceinline__ float normal_radius(float u) { return sqrtf(-2.0f * logf(u)); }
+__device__ __forceinline__ double normal_radius(double u) { return sqrt(-2.0 * log(u)); }
+__device__ __forceinline__ void normal_angle(float u, float& c, float& s) {
+  const float t = 6.283185307179586f * u;
+  c = cosf(t);
+  s = sinf(t);
+}
+__device__ __forceinline__ void normal_angle(double u, double& c, double& s) {
+  const double t = 6.283185307179586 * u;
+  c = cos(t);
+  s = sin(t);
+}
+
+// Four standard normals for (row quad, chain, proposal) by Box-Muller.
+template <typename T>
+__device__ inline void philox_normal4(uint64_t seed, uint32_t quad, uint32_t chain, uint64_t proposal,
+                                      uint32_t purpose, T out[4]) {
+  T u[4], c, s;
+  philox_uniforms4<T>(seed, quad, chain, proposal, purpose, u);
+  const T a = normal_radius(u[0]), b = normal_radius(u[2]);
+  normal_angle(u[1], c, s);
+  out[0] = a * c;
+  out[1] = a * s;
+  normal_angle(u[3], c, s);
+  out[2] = b * c;
+  out[3] = b * s;
 }
 
 // Per-chain scalar uniforms for proposal n: step factor and accept uniform.
@@ -167,6 +189,19 @@ __device__ __forceinline__ double f64_of(float v) {
   return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + add)), (int)(b << 29));
 }
 __device__ __forceinline__ double f64_of(double v) { return v; }
+
+// (T)(coeff * (double)e).  An FP32 coefficient (1 and 1/2 of the leapfrog) makes
+// the FP64 product exact, so its rounding to FP32 is the FP32 product.
+template <typename T>
+__device__ __forceinline__ T scaled_step(double coeff, bool single, T e) {
+  return single ? (T)coeff * e : (T)(coeff * (double)e);
+}
+inline bool is_single(double coeff) { return (double)(float)coeff == coeff; }
+
+// sqrt of a mass: FP32 through the correctly rounded single-precision root,
+// which equals the FP64 root rounded to FP32.
+__device__ __forceinline__ float mass_root(float m) { return sqrtf(m); }
+__device__ __forceinline__ double mass_root(double m) { return sqrt(m); }
 
 // ---------------------------------------------------------------------------
 // Per-chain reductions over the [d][C] layout: a block owns 32 consecutive

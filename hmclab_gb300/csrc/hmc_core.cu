@@ -177,19 +177,6 @@ __global__ void draw_z_kernel(ChainView<T> s) {
   }
 }
 
-// (T)(coeff * (double)e).  An FP32 coefficient (1 and 1/2 of the leapfrog) makes
-// the FP64 product exact, so its rounding to FP32 is the FP32 product.
-template <typename T>
-__device__ __forceinline__ T scaled_step(double coeff, bool single, T e) {
-  return single ? (T)coeff * e : (T)(coeff * (double)e);
-}
-inline bool is_single(double coeff) { return (double)(float)coeff == coeff; }
-
-// sqrt of a mass: FP32 through the correctly rounded single-precision root,
-// which equals the FP64 root rounded to FP32.
-__device__ __forceinline__ float mass_root(float m) { return sqrtf(m); }
-__device__ __forceinline__ double mass_root(double m) { return sqrt(m); }
-
 // Momentum (UNIT/DIAG; FULL has p and v = M^-1 p already), K0 in FP64, step
 // size of this trajectory, first drift and reflection.  Bound by issue (Philox
 // and Box-Muller, 43 % ALU) once the step size is formed once per chain and

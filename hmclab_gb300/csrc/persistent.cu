@@ -1,81 +1,28 @@
 // Persistent fused proposals for small dense linear-Gaussian targets: one
-// launch runs many whole HMC proposals for every chain, one warp per chain,
-// with the d x d GtG of the premultiplied LinearMatrix in shared memory.
-// Everything a proposal needs — Philox momenta (or injected streams), every
-// kick and drift of the integrator, the misfit at the end point, the FP64
-// accept test, the thinned sample record — happens in registers and shared
-// memory, so a chain of d <= 128 costs a handful of microseconds per
-// proposal instead of four launches per leapfrog step.
+// launch runs many whole HMC proposals for every chain.  Everything a proposal
+// needs — Philox momenta (or injected streams), every kick and drift of the
+// integrator, the misfit at the end point, the FP64 accept test, the thinned
+// sample record — happens in registers and shared memory, so a chain of d <=
+// 128 costs a handful of microseconds per proposal instead of four launches
+// per leapfrog step.  Three kernels share the work:
 //
-// Each lane owns the rows lane, lane + 32, ... of the chain's state.  The
-// arithmetic follows the launch-per-step path operation by operation (same
+//   persistent_lanes_kernel  (persistent_lanes.cu) many chains, unit or diagonal mass: a warp per
+//                            1, 2 or 4 chains, a lane per row
+//   persistent_rows_kernel   (persistent_rows.cu) few chains, unit or diagonal mass: a cluster of
+//                            blocks per chain, several lanes per row
+//   persistent_dense_kernel  full mass, and several targets in one launch: a
+//                            warp per chain
+//
+// The arithmetic follows the launch-per-step path operation by operation (same
 // random draws, the same (GtG q - Gtd0) + prior-gradient composition, the
 // same casts); the sums of the products and of the energies are taken in a
-// different order, so the two paths agree to rounding of those sums.
-#include "common.cuh"
+// different order, so the two paths agree to rounding of those sums.  FP32
+// products are summed by column modulo 4 in all three kernels, so FP32 states
+// are bitwise the same in each.
+#include "persistent.cuh"
 
 namespace hmc {
 namespace pers {
-
-constexpr int MAX_D = 128;
-enum PriorKind { PRIOR_NONE = 0, PRIOR_NORMAL = 1, PRIOR_LAPLACE = 2 };
-
-template <typename T>
-struct Target {
-  int d, ld;  // dimension, odd row stride of GtG in shared memory
-  int prior;  // PriorKind
-  const T* GtG;
-  const T* Gtd0;
-  double dtd;
-  const T* pmean;
-  const T* pw;
-};
-
-template <typename T>
-struct State {
-  int64_t C;
-  int mass;  // HMC_MASS_*
-  T* q_cur;
-  double* x_cur;
-  const T* eps;
-  int64_t* accepted;
-  const int64_t* control;
-  uint64_t seed;
-  int randomize;
-  const T* mdiag;
-  const T* minv;
-  const T* mchol;      // FULL: lower Cholesky factor of M, [d][d]
-  const T* mfull_inv;  // FULL: M^-1, [d][d]
-  const T* sz;
-  const T* seps;
-  const double* su;
-  int64_t slen;
-  T* ring_q;
-  double* ring_x;
-  int64_t ring_slots, thin;
-};
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-template <typename T>
-__device__ __forceinline__ T sign_of(T x) {
-  return x > (T)0 ? (T)1 : (x < (T)0 ? (T)-1 : (T)0);
-}
-
-// Standard normal for row i of chain c at proposal n: the injected stream or
-// the Philox quad (i / 4) that the launch-per-step path draws.
-template <typename T>
-__device__ __forceinline__ T momentum_draw(const State<T>& s, int d, int i, int64_t c, int64_t n) {
-  if (s.sz) return s.sz[((n % s.slen) * d + i) * s.C + c];
-  T z[4];
-  philox_normal4<T>(s.seed, (uint32_t)(i >> 2), (uint32_t)c, (uint64_t)n, PURPOSE_MOMENTUM, z);
-  const int j = i & 3;  // select without a local-memory array index
-  return j == 0 ? z[0] : (j == 1 ? z[1] : (j == 2 ? z[2] : z[3]));
-}
 
 // out[k] = sum_j GtG[row][j] q[j] for the lane's rows (q published in qw).
 // Four partial sums per row (j mod 4) keep four independent FMA chains in
@@ -116,16 +63,6 @@ __device__ __forceinline__ void apply_minv(int mass, const T* Mi, int ld, int d,
   } else {
 #pragma unroll
     for (int k = 0; k < E; ++k) mp[k] = mass == HMC_MASS_DIAG ? minv[k] * p[k] : p[k];
-  }
-}
-
-// Shared-memory matrices of one block: GtG, and for a full mass its
-// inverse and Cholesky factor, each [d][ld]; then one q vector per warp.
-template <typename T>
-__device__ __forceinline__ void load_matrix(T* dst, const T* src, int d, int ld) {
-  for (int e = threadIdx.x; e < d * d; e += blockDim.x) {
-    const int r = e / d;
-    dst[r * ld + (e - r * d)] = src[e];
   }
 }
 
@@ -433,23 +370,43 @@ int check_common(const char* who, const hmc_schedule* sch, int64_t nprop, int wa
   return HMC_OK;
 }
 
+// kernel HMC_PERSISTENT_WARPS: a = warps per block; _LANES: a = chains per warp,
+// b = warps per block; _ROWS: a = blocks per chain.
 template <typename T>
 int persistent_impl(const hmc_chains* s, const void* GtG, const void* Gtd0, double dtd, int prior,
-                    const void* pmean, const void* pw, const hmc_schedule* sch, int64_t nprop, int warps, int dry,
-                    cudaStream_t stream) {
+                    const void* pmean, const void* pw, const hmc_schedule* sch, int64_t nprop, int kernel, int a, int b,
+                    int dry, cudaStream_t stream) {
   const char* who = "hmc_persistent_dense";
+  const int warps = kernel == HMC_PERSISTENT_WARPS ? a : (kernel == HMC_PERSISTENT_LANES ? b : 1);
   HMC_TRY(check_common(who, sch, nprop, warps));
   State<T> st;
   Target<T> tg;
   HMC_TRY(fill_target<T>(who, s, GtG, Gtd0, dtd, prior, pmean, pw, nprop, warps, st, tg));
+  HMC_REQUIRE(kernel >= HMC_PERSISTENT_WARPS && kernel <= HMC_PERSISTENT_ROWS, "%s: unknown kernel %d", who, kernel);
+  HMC_REQUIRE(kernel == HMC_PERSISTENT_WARPS || st.mass != HMC_MASS_FULL,
+              "%s: a full mass runs one chain per warp", who);
   if (nprop == 0) return HMC_OK;
-  const int E = (tg.d + 31) / 32;
   int rc;
-  switch (E) {
-    case 1: rc = launch_single<T, 1>(st, tg, *sch, nprop, dry, warps, stream); break;
-    case 2: rc = launch_single<T, 2>(st, tg, *sch, nprop, dry, warps, stream); break;
-    case 3: rc = launch_single<T, 3>(st, tg, *sch, nprop, dry, warps, stream); break;
-    default: rc = launch_single<T, 4>(st, tg, *sch, nprop, dry, warps, stream); break;
+  if (kernel != HMC_PERSISTENT_WARPS) {
+    bool single = is_single(sch->first_drift);
+    for (int k = 0; k < sch->steps; ++k) single = single && is_single(sch->kick[k]) && is_single(sch->drift[k]);
+    if (kernel == HMC_PERSISTENT_LANES) {
+      HMC_REQUIRE(a == 1 || a == 2 || (a == 4 && sizeof(T) == 4), "%s: %d chains per warp", who, a);
+      HMC_REQUIRE(warps <= 8, "%s: at most 8 warps per block", who);
+      HMC_REQUIRE(lanes_smem<T>(tg.d, sch->steps, a, warps) <= 227 * 1024, "%s: d = %d does not fit in shared memory", who,
+                  tg.d);
+      rc = launch_lanes<T>(st, tg, *sch, nprop, dry, single, a, warps, stream);
+    } else {
+      rc = launch_rows<T>(st, tg, *sch, nprop, dry, single, a, stream);
+    }
+  } else {
+    const int E = (tg.d + 31) / 32;
+    switch (E) {
+      case 1: rc = launch_single<T, 1>(st, tg, *sch, nprop, dry, warps, stream); break;
+      case 2: rc = launch_single<T, 2>(st, tg, *sch, nprop, dry, warps, stream); break;
+      case 3: rc = launch_single<T, 3>(st, tg, *sch, nprop, dry, warps, stream); break;
+      default: rc = launch_single<T, 4>(st, tg, *sch, nprop, dry, warps, stream); break;
+    }
   }
   HMC_TRY(rc);
   if (dry) return HMC_OK;
@@ -521,8 +478,19 @@ extern "C" HMC_API int hmc_persistent_dense(const hmc_chains* s, const void* GtG
                                             int dry, void* stream) {
   if (!s) return fail(HMC_ERR_INVALID_ARG, "hmc_persistent_dense: null state");
   return HMC_DISPATCH(s->dtype, T, [&] {
-    return persistent_impl<T>(s, GtG, Gtd0, dtd, prior, prior_mean, prior_w, schedule, proposals, warps_per_block,
-                              dry, as_stream(stream));
+    return persistent_impl<T>(s, GtG, Gtd0, dtd, prior, prior_mean, prior_w, schedule, proposals, HMC_PERSISTENT_WARPS,
+                              warps_per_block, 0, dry, as_stream(stream));
+  });
+}
+
+extern "C" HMC_API int hmc_persistent_dense_shaped(const hmc_chains* s, const void* GtG, const void* Gtd0, double dtd,
+                                                   int prior, const void* prior_mean, const void* prior_w,
+                                                   const hmc_schedule* schedule, int64_t proposals, int kernel, int a,
+                                                   int b, int dry, void* stream) {
+  if (!s) return fail(HMC_ERR_INVALID_ARG, "hmc_persistent_dense: null state");
+  return HMC_DISPATCH(s->dtype, T, [&] {
+    return persistent_impl<T>(s, GtG, Gtd0, dtd, prior, prior_mean, prior_w, schedule, proposals, kernel, a, b, dry,
+                              as_stream(stream));
   });
 }
 

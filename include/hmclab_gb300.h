@@ -725,6 +725,20 @@ HMC_API int hmc_persistent_dense(const hmc_chains* s, const void* GtG,
                                  const hmc_schedule* schedule,
                                  int64_t proposals, int warps_per_block,
                                  int dry, void* stream);
+/* The same with the kernel and its launch shape named: _WARPS (a = warps per
+ * block; the kernel of hmc_persistent_dense), and for unit and diagonal mass
+ * _LANES (a = 1, 2 or, FP32, 4 chains per warp, b = 1, 2, 4 or 8 warps per
+ * block) and _ROWS (a = 1, 2, 4 or 8 blocks per chain).                      */
+enum {
+  HMC_PERSISTENT_WARPS = 0,
+  HMC_PERSISTENT_LANES = 1,
+  HMC_PERSISTENT_ROWS = 2
+};
+HMC_API int hmc_persistent_dense_shaped(
+    const hmc_chains* s, const void* GtG, const void* Gtd0, double dtd,
+    int prior, const void* prior_mean, const void* prior_w,
+    const hmc_schedule* schedule, int64_t proposals, int kernel, int a, int b,
+    int dry, void* stream);
 
 /* Several such targets of different dimensions and chain counts in one
  * launch (one group per target, up to 48 groups; every group has its own
