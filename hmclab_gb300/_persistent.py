@@ -25,38 +25,40 @@ def _smem(d, full, warps, esize):
     return ((3 if full else 1) * d * (d | 1) + warps * d) * esize
 
 
-def _lanes_smem(d, steps, chains_per_warp, warps, esize):
+def _lanes_groups(d, chains, esize):
+    """Groups of warps a block of csrc/persistent_lanes.cu may hold (up to 8
+    warps: one per 32 rows, or one per group for large FP32 batches)."""
+    warps = 1 if esize == 4 and d > 64 and chains >= 2048 else -(-d // 32)
+    return [g for g in (1, 2, 4, 8) if g * warps <= 8]
+
+
+def _lanes_smem(d, steps, chains, groups, esize):
     """Upper bound of one block's shared memory in csrc/persistent_lanes.cu:
-    the chains' vectors and step coefficients, and GtG."""
-    return ((d + 16 + 2 * steps) * warps * chains_per_warp + d * (d | 1)) * esize
+    the groups' vectors, step coefficients and sums, and GtG."""
+    vectors = groups * (2 * (d + 32) + 2 * steps) + 16
+    return vectors * chains * esize + groups * (64 * chains + 64) + d * (d | 1) * esize
 
 
-def _cluster(d, chains, esize):
-    """Blocks per chain of the rows kernel: one per 16 FP64 or 32 FP32 rows, as
-    long as every block has an SM of its own; FP64 products of more than 64
-    rows need two blocks of 512 threads.  Measured per proposal (10 steps,
-    FP64): d = 50, one chain 28.9 / 21.6 / 19.0 / 20.1 us on 1 / 2 / 4 / 8
-    blocks, 64 chains 28.9 / 21.7 / 25.8 / 42.5; d = 100, one chain 39.1 /
-    25.1 / 23.3 us on 2 / 4 / 8; FP32, d = 128, one chain 16.8 / 15.6 / 14.1 /
-    14.7 us on 1 / 2 / 4 / 8."""
-    rows = 16 if esize == 8 else 32
+def _cluster(d, chains):
+    """Blocks per chain of the rows kernel: one per 16 rows, as long as every
+    block has an SM of its own; products of more than 64 rows need two blocks
+    of 512 threads.  Measured per proposal of 10 steps: d = 50, one chain 28.1 /
+    20.2 / 17.9 / 18.3 us on 1 / 2 / 4 / 8 blocks, 64 chains 28.9 / 21.7 / 25.8 /
+    42.5; d = 100, one chain 37.9 / 24.6 / 22.1 us on 2 / 4 / 8."""
     r = 1
-    while r < 8 and r * rows < d and 2 * r * chains <= 152:
+    while r < 8 and r * 16 < d and 2 * r * chains <= 152:
         r *= 2
-    return max(r, 2) if esize == 8 and d > 64 else r
+    return max(r, 2) if d > 64 else r
 
 
 def _rows_kernel(d, chains, esize):
-    """Whether several lanes per row (one chain per cluster) beat one lane per
-    row.  FP64: while the chains leave SMs without one; a lone warp issues
-    FP64 at a quarter of its SM's rate (d = 50, one chain: 19 us per proposal
-    against 64 us; 304 chains 52 against 64, 1024 chains 177 against 90; d =
-    30, 304 chains 34 against 28).  FP32: beyond the 64 columns that the lanes
-    kernel holds in registers (d = 100, 152 chains 15 against 26 us, 304
-    chains 29 against 26; d = 50, one chain 11.4 against 6.4)."""
-    if esize == 8:
-        return chains <= (152 if d <= 32 else 304)
-    return d > 64 and chains <= 152
+    """Whether several lanes per row and a cluster per chain beat a thread per
+    row: FP64 chains that leave most SMs idle, as a lone warp issues FP64 at a
+    quarter of its SM's rate (d = 50, one chain 17.9 us per proposal against
+    36.3, 152 chains 28.7 against 37.3, 304 chains 56 against 37; d = 100, 64
+    chains 39 against 60, 152 chains 78 against 61).  FP32 chains never (d =
+    100, one chain 13.3 against 8.1)."""
+    return esize == 8 and chains <= (152 if d <= 64 else 76)
 
 
 def kernel_of(d, chains, esize, full, steps):
@@ -64,9 +66,9 @@ def kernel_of(d, chains, esize, full, steps):
     if full:
         return [(_lib.HMC_PERSISTENT_WARPS, w, 0) for w in _WARPS if _smem(d, full, w, esize) <= _SMEM]
     if _rows_kernel(d, chains, esize):
-        return [(_lib.HMC_PERSISTENT_ROWS, _cluster(d, chains, esize), 0)]
-    return [(_lib.HMC_PERSISTENT_LANES, ct, w) for ct in ((1, 2, 4) if esize == 4 else (1, 2)) for w in (1, 2, 4, 8)
-            if _lanes_smem(d, steps, ct, w, esize) <= _SMEM]
+        return [(_lib.HMC_PERSISTENT_ROWS, _cluster(d, chains), 0)]
+    return [(_lib.HMC_PERSISTENT_LANES, ct, g) for ct in ((1, 2, 4) if esize == 4 else (1, 2))
+            for g in _lanes_groups(d, chains, esize) if _lanes_smem(d, steps, ct, g, esize) <= _SMEM]
 
 
 # chosen launch shapes, per (dimension, chains, dtype, mass, prior, schedule length)

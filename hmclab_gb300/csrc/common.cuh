@@ -203,6 +203,21 @@ inline bool is_single(double coeff) { return (double)(float)coeff == coeff; }
 __device__ __forceinline__ float mass_root(float m) { return sqrtf(m); }
 __device__ __forceinline__ double mass_root(double m) { return sqrt(m); }
 
+// exp(dh) > u, the accept test, for dh = H0 - H1 (strict; NaN compares false).
+// An FP64 exponential is some forty FP64 instructions at 64 cycles each; the
+// FP32 one, within 1e-5 of the exact value for -80 < dh < 0 (its argument is
+// rounded by up to 5e-6 and its own error is 2 ulp), settles every test whose
+// sides differ by more than 1e-4.  The rest takes the FP64 test.
+__device__ __forceinline__ bool accept_test(double dh, double u) {
+  const float x = (float)dh, v = (float)u;
+  if (x > -80.f && x < 80.f && v > 1e-30f && v < 0.999f) {
+    const float a = expf(x);
+    if (a * 0.9999f > v) return true;
+    if (a * 1.0001f < v) return false;
+  }
+  return exp(dh) > u;
+}
+
 // ---------------------------------------------------------------------------
 // Per-chain reductions over the [d][C] layout: a block owns 32 consecutive
 // chains (threadIdx.x) and RY row lanes (threadIdx.y); rows are strided by RY

@@ -6,9 +6,9 @@
 // 128 costs a handful of microseconds per proposal instead of four launches
 // per leapfrog step.  Three kernels share the work:
 //
-//   persistent_lanes_kernel  (persistent_lanes.cu) many chains, unit or diagonal mass: a warp per
-//                            1, 2 or 4 chains, a lane per row
-//   persistent_rows_kernel   (persistent_rows.cu) few chains, unit or diagonal mass: a cluster of
+//   persistent_lanes_kernel  (persistent_lanes.cu) many chains, unit or diagonal mass: a group of
+//                            warps per 1, 2 or 4 chains, a thread per row
+//   persistent_rows_kernel   (persistent_rows.cu) few FP64 chains, unit or diagonal mass: a cluster of
 //                            blocks per chain, several lanes per row
 //   persistent_dense_kernel  full mass, and several targets in one launch: a
 //                            warp per chain
@@ -370,8 +370,8 @@ int check_common(const char* who, const hmc_schedule* sch, int64_t nprop, int wa
   return HMC_OK;
 }
 
-// kernel HMC_PERSISTENT_WARPS: a = warps per block; _LANES: a = chains per warp,
-// b = warps per block; _ROWS: a = blocks per chain.
+// kernel HMC_PERSISTENT_WARPS: a = warps per block; _LANES: a = chains per group,
+// b = groups per block; _ROWS: a = blocks per chain.
 template <typename T>
 int persistent_impl(const hmc_chains* s, const void* GtG, const void* Gtd0, double dtd, int prior,
                     const void* pmean, const void* pw, const hmc_schedule* sch, int64_t nprop, int kernel, int a, int b,
@@ -391,13 +391,11 @@ int persistent_impl(const hmc_chains* s, const void* GtG, const void* Gtd0, doub
     bool single = is_single(sch->first_drift);
     for (int k = 0; k < sch->steps; ++k) single = single && is_single(sch->kick[k]) && is_single(sch->drift[k]);
     if (kernel == HMC_PERSISTENT_LANES) {
-      HMC_REQUIRE(a == 1 || a == 2 || (a == 4 && sizeof(T) == 4), "%s: %d chains per warp", who, a);
-      HMC_REQUIRE(warps <= 8, "%s: at most 8 warps per block", who);
-      HMC_REQUIRE(lanes_smem<T>(tg.d, sch->steps, a, warps) <= 227 * 1024, "%s: d = %d does not fit in shared memory", who,
-                  tg.d);
+      HMC_REQUIRE(a == 1 || a == 2 || (a == 4 && sizeof(T) == 4), "%s: %d chains per group", who, a);
       rc = launch_lanes<T>(st, tg, *sch, nprop, dry, single, a, warps, stream);
     } else {
-      rc = launch_rows<T>(st, tg, *sch, nprop, dry, single, a, stream);
+      if constexpr (sizeof(T) == 4) return fail(HMC_ERR_INVALID_ARG, "%s: cluster per chain: FP64 only", who);
+      else rc = launch_rows<T>(st, tg, *sch, nprop, dry, single, a, stream);
     }
   } else {
     const int E = (tg.d + 31) / 32;

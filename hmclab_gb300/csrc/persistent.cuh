@@ -81,12 +81,9 @@ __device__ __forceinline__ void load_matrix(T* dst, const T* src, int d, int ld)
 // coefficient is an FP32 value (scaled_step).
 template <typename T>
 int launch_lanes(const State<T>& st, const Target<T>& tg, const hmc_schedule& sch, int64_t nprop, int dry, bool single,
-                 int chains_per_warp, int warps, cudaStream_t stream);
+                 int chains, int groups, cudaStream_t stream);
 template <typename T>
 int launch_rows(const State<T>& st, const Target<T>& tg, const hmc_schedule& sch, int64_t nprop, int dry, bool single,
                 int cluster, cudaStream_t stream);
-template <typename T>
-size_t lanes_smem(int d, int steps, int chains_per_warp, int warps);
-
 }  // namespace pers
 }  // namespace hmc

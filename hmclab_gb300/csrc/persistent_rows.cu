@@ -18,8 +18,8 @@ struct RowsShared {
   T z2[2][MAX_D / 4];
   T kick[HMC_SCHEDULE_MAX], drift[HMC_SCHEDULE_MAX], first;
   double u;
-  double part[ROWS_MAX_THREADS / 32][3];
-  double total[ROWS_MAX_CLUSTER][3];
+  double part[ROWS_MAX_THREADS / 32][2];
+  double total[ROWS_MAX_CLUSTER][2];  // misfit, K1 - K0
   int accept;
 };
 
@@ -38,8 +38,9 @@ __host__ __device__ constexpr int rows_stride(int d) {
 // row's lanes and the update, then the cluster barrier that publishes q; the
 // momenta (one warp per part of Box-Muller), the sums of the energies and the
 // exponential take the rest of a proposal.  One FP64 chain, 10 steps: d = 50
-// 19.0 us on four blocks against 69 us with the chain in one warp; d = 128
-// 24.8 against 271 us.
+// 17.9 us on four blocks against 69 us with the chain in one warp; d = 128
+// 24.1 against 271 us.  FP32 chains do better with a thread per row (d = 100:
+// 13.3 us here, 8.1 there).
 template <typename T, int KC>
 __global__ void __launch_bounds__(ROWS_MAX_THREADS) persistent_rows_kernel(State<T> s, Target<T> tg,
                                                                            const __grid_constant__ hmc_schedule sch,
@@ -91,15 +92,8 @@ __global__ void __launch_bounds__(ROWS_MAX_THREADS) persistent_rows_kernel(State
     const T* x = sh.q[buf];
     buf ^= 1;
     T v = (T)0;
-    if (sizeof(T) == 4) {  // columns modulo 4, the remainder in the first lane, as the other kernels
-      const int main = d & ~3;
-      for (int j = kc; j < main; j += KC) v = fma(a[j], x[j], v);
-      if (kc == 0)
-        for (int j = main; j < d; ++j) v = fma(a[j], x[j], v);
-    } else {
 #pragma unroll 4
-      for (int j = kc; j < d; j += KC) v = fma(a[j], x[j], v);
-    }
+    for (int j = kc; j < d; j += KC) v = fma(a[j], x[j], v);
 #pragma unroll
     for (int o = 1; o < KC; o *= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
@@ -136,7 +130,7 @@ __global__ void __launch_bounds__(ROWS_MAX_THREADS) persistent_rows_kernel(State
     }
     __syncthreads();
     T p = (T)0, q = qc;
-    double k0 = 0.0, k1 = 0.0, x = 0.0;
+    double dk = 0.0, x = 0.0;
     if (live) {
       T z;
       if (s.sz) {
@@ -148,7 +142,7 @@ __global__ void __launch_bounds__(ROWS_MAX_THREADS) persistent_rows_kernel(State
       }
       p = diag ? msq * z : z;
       const T mp = diag ? minv * p : p;
-      k0 = f64_of(p) * f64_of(mp);
+      dk = -(f64_of(p) * f64_of(mp));
       q = fma(sh.first, mp, qc);
     }
     for (int st = 0; st < sch.steps; ++st) {
@@ -169,22 +163,20 @@ __global__ void __launch_bounds__(ROWS_MAX_THREADS) persistent_rows_kernel(State
         x = fma(f64_of(dq), f64_of(pw * dq), x);
       }
       if (prior == PRIOR_LAPLACE) x = fma(2.0, f64_of((T)(fabs(q - pm) * pw)), x);
-      k1 = f64_of(p) * f64_of(diag ? minv * p : p);
+      dk = fma(f64_of(p), f64_of(diag ? minv * p : p), dk);
     }
     // sums over the rows: the lanes of a row hold the same value
 #pragma unroll
     for (int o = KC; o < 32; o *= 2) {
       x += __shfl_xor_sync(0xffffffffu, x, o);
-      k1 += __shfl_xor_sync(0xffffffffu, k1, o);
-      k0 += __shfl_xor_sync(0xffffffffu, k0, o);
+      dk += __shfl_xor_sync(0xffffffffu, dk, o);
     }
     if (lane == 0) {
       sh.part[warp][0] = x;
-      sh.part[warp][1] = k1;
-      sh.part[warp][2] = k0;
+      sh.part[warp][1] = dk;
     }
     __syncthreads();
-    if (tid < 3) {
+    if (tid < 2) {
       double v = 0.0;
       for (int k = 0; k < (int)blockDim.x / 32; ++k) v += sh.part[k][tid];
       for (int k = 0; k < cluster; ++k)
@@ -193,12 +185,12 @@ __global__ void __launch_bounds__(ROWS_MAX_THREADS) persistent_rows_kernel(State
     sync();
     if (warp == 0) {  // the same sums in every block: all take the same decision
       double v = 0.0;
-      if (lane < 3)
+      if (lane < 2)
         for (int k = 0; k < cluster; ++k) v += sh.total[k][lane];
       const double x1 = 0.5 * (__shfl_sync(0xffffffffu, v, 0) + tg.dtd);
-      const double e1 = 0.5 * __shfl_sync(0xffffffffu, v, 1), e0 = 0.5 * __shfl_sync(0xffffffffu, v, 2);
+      const double d1 = 0.5 * __shfl_sync(0xffffffffu, v, 1);
       if (lane == 0) {
-        sh.accept = exp((xc + e0) - (x1 + e1)) > sh.u ? 1 : 0;  // strict; NaN compares false
+        sh.accept = accept_test(xc - (x1 + d1), sh.u) ? 1 : 0;
         if (sh.accept) {
           xc = x1;
           ++n_acc;
@@ -227,7 +219,7 @@ __global__ void __launch_bounds__(ROWS_MAX_THREADS) persistent_rows_kernel(State
 template <typename T>
 int launch_rows(const State<T>& st, const Target<T>& tg, const hmc_schedule& sch, int64_t nprop, int dry, bool single,
                 int cluster, cudaStream_t stream) {
-  constexpr int KC = sizeof(T) == 8 ? 8 : 4;
+  constexpr int KC = 8;
   HMC_REQUIRE(cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8, "persistent rows: cluster of %d blocks",
               cluster);
   const int quads = (tg.d + 3) / 4, own_quads = (quads + cluster - 1) / cluster;
@@ -256,8 +248,6 @@ int launch_rows(const State<T>& st, const Target<T>& tg, const hmc_schedule& sch
   return check_launch("persistent_rows_kernel");
 }
 
-template int launch_rows<float>(const State<float>&, const Target<float>&, const hmc_schedule&, int64_t, int, bool, int,
-                                cudaStream_t);
 template int launch_rows<double>(const State<double>&, const Target<double>&, const hmc_schedule&, int64_t, int, bool,
                                  int, cudaStream_t);
 

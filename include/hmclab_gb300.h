@@ -727,8 +727,9 @@ HMC_API int hmc_persistent_dense(const hmc_chains* s, const void* GtG,
                                  int dry, void* stream);
 /* The same with the kernel and its launch shape named: _WARPS (a = warps per
  * block; the kernel of hmc_persistent_dense), and for unit and diagonal mass
- * _LANES (a = 1, 2 or, FP32, 4 chains per warp, b = 1, 2, 4 or 8 warps per
- * block) and _ROWS (a = 1, 2, 4 or 8 blocks per chain).                      */
+ * _LANES (a = 1, 2 or, FP32, 4 chains per group, b = 1,
+ * 2, 4 or 8 groups and at most 8 warps per block) and _ROWS (FP64; a = 1, 2, 4 or 8
+ * blocks per chain).                                                        */
 enum {
   HMC_PERSISTENT_WARPS = 0,
   HMC_PERSISTENT_LANES = 1,

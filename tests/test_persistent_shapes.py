@@ -40,19 +40,22 @@ def _run(smp, shape):
     (16, 9, "normal", "diag", "lf"), (19, 4, "none", "unit", "lf"), (20, 33, "normal", "unit", "4s"),
     (32, 6, "laplace", "diag", "lf"), (33, 2, "normal", "unit", "lf"), (50, 35, "normal", "diag", "3s"),
     (51, 3, "laplace", "unit", "lf"), (52, 5, "none", "diag", "lf"), (64, 17, "normal", "unit", "lf"),
-    (67, 2, "laplace", "diag", "lf"), (97, 7, "normal", "unit", "lf"), (128, 5, "normal", "diag", "4s")])
+    (67, 2, "laplace", "diag", "lf"), (97, 7, "normal", "unit", "lf"), (128, 5, "normal", "diag", "4s"),
+    (70, 2050, "normal", "unit", "lf"), (98, 2049, "laplace", "diag", "lf"), (128, 2051, "none", "unit", "lf")])
 @pytest.mark.parametrize("dtype", ["float32", "float64"])
 def test_kernels_agree(d, C, prior, mass, integrator, dtype):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from hmclab_gb300 import _lib
+    from hmclab_gb300._persistent import _lanes_groups
 
     def fresh():
         return _sampler(d, C, dtype, prior, mass, d + C, integrator)
 
     ref = _run(fresh(), (_lib.HMC_PERSISTENT_WARPS, 4, 0))
-    shapes = [(_lib.HMC_PERSISTENT_LANES, ct, w) for ct in ((1, 2, 4) if dtype == "float32" else (1, 2)) for w in (1, 4)]
-    shapes += [(_lib.HMC_PERSISTENT_ROWS, r, 0) for r in (1, 2, 4, 8) if dtype == "float32" or r > 1 or d <= 64]
+    shapes = [(_lib.HMC_PERSISTENT_LANES, ct, g) for ct in ((1, 2, 4) if dtype == "float32" else (1, 2))
+              for g in _lanes_groups(d, C, 4 if dtype == "float32" else 8)]
+    shapes += [(_lib.HMC_PERSISTENT_ROWS, r, 0) for r in (1, 2, 4, 8) if dtype == "float64" and (r > 1 or d <= 64)]
     assert 0 < ref[2].sum()
     for shape in shapes:
         got = _run(fresh(), shape)
@@ -76,7 +79,7 @@ def test_kernels_agree_on_injected_streams(dtype):
     rng = np.random.default_rng(0)
     streams = (rng.normal(size=(6, d, C)), rng.uniform(0.5, 1.5, size=(6, C)), rng.uniform(size=(6, C)))
     ref = _run(_sampler(d, C, dtype, "normal", "diag", 3, streams=streams), (_lib.HMC_PERSISTENT_WARPS, 2, 0))
-    for shape in ((_lib.HMC_PERSISTENT_LANES, 2, 2), (_lib.HMC_PERSISTENT_ROWS, 2, 0)):
+    for shape in ((_lib.HMC_PERSISTENT_LANES, 2, 2),) + (((_lib.HMC_PERSISTENT_ROWS, 2, 0),) if dtype == "float64" else ()):
         got = _run(_sampler(d, C, dtype, "normal", "diag", 3, streams=streams), shape)
         assert np.array_equal(got[2], ref[2])
         np.testing.assert_allclose(got[0], ref[0], rtol=0, atol=0 if dtype == "float32" else 1e-13)
