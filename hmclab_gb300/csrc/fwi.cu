@@ -30,7 +30,7 @@
 
 #include <mutex>
 
-#include "common.cuh"
+#include "fwi_cluster.cuh"
 
 namespace hmc {
 namespace fwi {
@@ -944,6 +944,83 @@ static StoreSlot store_slot(const hmc_fwi* s, int n) {
   return {base, base + 2 * cells, 4ll * (n / k) * s->nz};
 }
 
+static ShotForward forward_args(const hmc_fwi* s, int shot, int store) {
+  ShotForward a = {};
+  a.nx = s->nx;
+  a.nz = s->nz;
+  a.C = s->chains;
+  a.inv_h = 1.f / s->h;
+  a.dt = s->dt;
+  a.bx = s->bx;
+  a.bz = s->bz;
+  a.l2m = s->l2m;
+  a.lam = s->lam;
+  a.muxz = s->muxz;
+  a.taper = s->taper;
+  a.rec_map = s->rec_map;
+  a.vx = s->vx;
+  a.vz = s->vz;
+  a.sxx = s->sxx;
+  a.szz = s->szz;
+  a.sxz = s->sxz;
+  a.rec = s->rec + (int64_t)shot * s->nt * s->nrec * 2 * s->chains;
+  a.store = store ? s->store : nullptr;
+  a.planes = stored_planes(s);
+  a.snap = snapshot_interval(s);
+  a.nrec = s->nrec;
+  a.wait_ns = wait_limits().ns;
+  a.status = s->status;
+  return a;
+}
+static ShotAdjoint adjoint_args(const hmc_fwi* s) {
+  ShotAdjoint a = {};
+  a.nx = s->nx;
+  a.nz = s->nz;
+  a.C = s->chains;
+  a.inv_h = 1.f / s->h;
+  a.dt = s->dt;
+  a.w = (float)snapshot_interval(s);
+  a.bx = s->bx;
+  a.bz = s->bz;
+  a.l2m = s->l2m;
+  a.lam = s->lam;
+  a.muxz = s->muxz;
+  a.taper = s->taper;
+  a.rec_map = s->rec_map;
+  a.resid = s->resid;
+  a.store = s->store;
+  a.planes = stored_planes(s);
+  a.snap = snapshot_interval(s);
+  a.nrec = s->nrec;
+  a.nt = s->nt;
+  a.g_bx = s->g_bx;
+  a.g_bz = s->g_bz;
+  a.g_l2m = s->g_l2m;
+  a.g_lam = s->g_lam;
+  a.g_muxz = s->g_muxz;
+  a.wait_ns = wait_limits().ns;
+  a.status = s->status;
+  return a;
+}
+// Whether a shot runs with the wavefield on chip (fwi_cluster.cuh): grids of up
+// to 256 columns whose strips fit a cluster.  A stored wavefield has another
+// layout there ([chain][plane] instead of [plane][chain]), so the forward pass
+// that stores it and the adjoint that reads it decide together.  A null status
+// word keeps the direct-load kernels, and the wait-limit test hook the staged
+// ones, whose waits it shortens.  Per time step of 240 x 140 cells the staged
+// and direct-load kernels take 16.8 / 17.1 / 21.7 us (misfit) and 45 / 46 /
+// 82 us (misfit and gradient) for 1 / 16 / 64 chains, these 2.9 / 5.5 / 15.3 us
+// and 10 / 24 / 60 us; at 160 x 100 cells and 64 chains it is 11.8 and 37.9 us
+// against 7.8 and 38.0 us, the narrowest margin of the grids tried.
+static int on_chip(const hmc_fwi* s, int store, bool* yes) {
+  *yes = false;
+  if (!s->status || wait_limits().withhold) return HMC_OK;
+  static const Waves none = {};
+  HMC_TRY(cluster_forward(forward_args(s, 0, store), none, true, yes, nullptr));
+  if (*yes && store) HMC_TRY(cluster_adjoint(adjoint_args(s), true, yes, nullptr));
+  return HMC_OK;
+}
+
 extern "C" {
 
 HMC_API int hmc_fwi_prepare(const hmc_fwi* s, void* stream) {
@@ -975,9 +1052,9 @@ HMC_API int hmc_fwi_forward_shot_sources(const hmc_fwi* s, int shot, const hmc_f
               "hmc_fwi_forward_shot_sources: %d stress terms (a moment tensor with Mxz takes 4), at most %d", n_terms,
               MAX_SRC_TERMS);
   HMC_REQUIRE(!store || s->store, "hmc_fwi_forward_shot_sources: storing needs the store buffer");
+  const float src_scale = s->dt / (s->h * s->h);
   // the stress increments of step n; the wavelets are read on the host (a
   // handful of floats per step)
-  const float src_scale = s->dt / (s->h * s->h);
   auto source_step = [&](int n) {
     SourceStep ss{};
     ss.i0 = s->nx;
@@ -1008,6 +1085,48 @@ HMC_API int hmc_fwi_forward_shot_sources(const hmc_fwi* s, int shot, const hmc_f
     return ss;
   };
   cudaStream_t st = as_stream(stream);
+  bool chip = false;
+  if (n_src <= WAVE_SAMPLES) HMC_TRY(on_chip(s, store, &chip));
+  if (chip) {
+    ShotForward a = forward_args(s, shot, store);
+    Waves w = {};
+    auto term = [&](int q, int i, int j, float xx, float zz, float xz) {
+      w.i[w.n_terms] = (int16_t)i;
+      w.j[w.n_terms] = (int16_t)j;
+      w.first[w.n_terms] = q;
+      w.xx[w.n_terms] = xx;
+      w.zz[w.n_terms] = zz;
+      w.xz[w.n_terms] = xz;
+      ++w.n_terms;
+    };
+    for (int q = 0; q < n_src; ++q) {
+      const int i = src[q].x, j = src[q].z;
+      const float xz = 0.25f * src[q].mxz;
+      term(q, i, j, src[q].mxx, src[q].mzz, xz);
+      if (src[q].mxz != 0.f) {
+        term(q, i - 1, j - 1, 0.f, 0.f, xz);
+        term(q, i, j - 1, 0.f, 0.f, xz);
+        term(q, i - 1, j, 0.f, 0.f, xz);
+      }
+    }
+    // as many steps per launch as source samples fit its parameters
+    const int per = WAVE_SAMPLES / n_src;
+    const Waves sources = w;
+    for (int n0 = 0; n0 < s->nt; n0 += per) {
+      a.n0 = n0;
+      a.n1 = s->nt - n0 < per ? s->nt : n0 + per;
+      a.load = n0 > 0;
+      a.save = a.n1 < s->nt;
+      const int steps = a.n1 - n0;
+      for (int t = 0; t < w.n_terms; ++t) w.first[t] = sources.first[t] * steps;
+      for (int q = 0; q < n_src; ++q)
+        for (int n = 0; n < steps; ++n) w.s[q * steps + n] = src[q].stf_host[n0 + n] * src_scale;
+      bool ran = false;
+      HMC_TRY(cluster_forward(a, w, false, &ran, st));
+      HMC_REQUIRE(ran, "hmc_fwi_forward_shot_sources: no strip height fits");
+    }
+    return HMC_OK;
+  }
   const Grid g = grid_of(s);
   const int64_t cells = (int64_t)s->nx * s->nz * s->chains;
   const size_t fb = (size_t)cells * sizeof(float);
@@ -1080,6 +1199,14 @@ HMC_API int hmc_fwi_adjoint_shot(const hmc_fwi* s, int shot, void* stream) {
   HMC_REQUIRE(s->g_bx && s->g_bz && s->g_l2m && s->g_lam && s->g_muxz, "hmc_fwi_adjoint_shot: missing gradients");
   HMC_REQUIRE(s->t1 && s->t2 && s->t3 && s->t4 && s->t5, "hmc_fwi_adjoint_shot: missing adjoint temporaries");
   cudaStream_t st = as_stream(stream);
+  const int64_t rows = (int64_t)s->nt * s->nrec * 2;
+  const int64_t shot_off = (int64_t)shot * rows;
+  residual_kernel<<<grid_for(rows * s->chains), 256, 0, st>>>(rows, s->chains, s->rec + shot_off * s->chains,
+                                                              s->obs + shot_off, s->w, s->resid);
+  HMC_TRY(check_launch("residual_kernel"));
+  bool chip = false;
+  HMC_TRY(on_chip(s, 1, &chip));
+  if (chip) return cluster_adjoint(adjoint_args(s), false, &chip, st);
   const Grid g = grid_of(s);
   const int64_t cells = (int64_t)s->nx * s->nz * s->chains;
   const size_t fb = (size_t)cells * sizeof(float);
@@ -1087,11 +1214,6 @@ HMC_API int hmc_fwi_adjoint_shot(const hmc_fwi* s, int shot, void* stream) {
     cudaError_t e = cudaMemsetAsync(f, 0, fb, st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(fwi adjoint)");
   }
-  const int64_t rows = (int64_t)s->nt * s->nrec * 2;
-  const int64_t shot_off = (int64_t)shot * rows;
-  residual_kernel<<<grid_for(rows * s->chains), 256, 0, st>>>(rows, s->chains, s->rec + shot_off * s->chains,
-                                                              s->obs + shot_off, s->w, s->resid);
-  HMC_TRY(check_launch("residual_kernel"));
   Fields a{s->avx, s->avz, s->asxx, s->aszz, s->asxz};
   Params p{s->bx, s->bz, s->l2m, s->lam, s->muxz};
   Grads gr{s->g_bx, s->g_bz, s->g_l2m, s->g_lam, s->g_muxz};
