@@ -36,26 +36,29 @@ namespace hmc {
 namespace tc {
 
 constexpr int BM = 128;                   // chains per tile (UMMA M)
-constexpr int BN = 256;                   // matrix rows per tile (UMMA N)
+constexpr int BN = 256;                   // matrix rows per tile (UMMA N), many tiles
+constexpr int BN_FEW = 32;                // the same where 256 would leave most SMs idle
 constexpr int SWZ = 64;                   // swizzle span in bytes (64 or 128)
 constexpr int BK = SWZ / 2;               // k per stage = one swizzle row of bf16
 constexpr int UK = 16;                    // k per tcgen05.mma (kind::f16)
-constexpr int STAGES = SWZ == 64 ? 4 : 2;
 constexpr int A_BYTES = BM * BK * 2;      // per operand half (chains)
-constexpr int B_BYTES = BN * BK * 2;      // per operand half (rows)
-constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // hi/lo split (3 products)
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 // Stage layout for NPROD products: q_hi | q_lo | a_hi | a_lo (NPROD = 3) or
-// q | a (NPROD = 1, plain BF16 operands).
-template <int NPROD>
+// q | a (NPROD = 1, plain BF16 operands); ROWS matrix rows.  A short loop over
+// k is all latency, so narrow tiles hold as much of it as fits.
+template <int NPROD, int ROWS>
 struct Stage {
-  static constexpr int bytes = NPROD == 3 ? STAGE_BYTES : A_BYTES + B_BYTES;
+  static constexpr int b_bytes = ROWS * BK * 2;  // per operand half (rows)
+  static constexpr int bytes = (NPROD == 3 ? 2 : 1) * (A_BYTES + b_bytes);
   static constexpr int q_lo = A_BYTES;
   static constexpr int a_hi = NPROD == 3 ? 2 * A_BYTES : A_BYTES;
-  static constexpr int a_lo = a_hi + B_BYTES;
+  static constexpr int a_lo = a_hi + b_bytes;
+  static constexpr int count = ROWS == BN ? (SWZ == 64 ? 4 : 2) : (NPROD == 3 ? 10 : 20);
+  static constexpr int smem = count * bytes + 1024 + 512;
 };
+static_assert(Stage<3, BN>::smem <= 227 * 1024 && Stage<1, BN_FEW>::smem <= 227 * 1024 &&
+                  Stage<3, BN_FEW>::smem <= 227 * 1024,
+              "shared memory of a block");
 constexpr int THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
-constexpr uint32_t TMEM_COLS = 256;
 
 enum Epi { EPI_GRAD = 0, EPI_STEP = 1, EPI_MISFIT = 2, EPI_MLP_HIDDEN = 3, EPI_MLP_OUT = 4, EPI_MLP_BACK = 5 };
 enum Prior { PRIOR_NONE = 0, PRIOR_NORMAL = 1, PRIOR_LAPLACE = 2 };
@@ -209,13 +212,28 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
   for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
+// Store the first nr of 16 consecutive values of a row of pitch ld, in four
+// 16-byte stores where the row allows it.
+__device__ __forceinline__ void store_row16(float* dst, const float (&v)[16], int nr, int64_t ld) {
+  if (nr == 16 && (ld & 3) == 0 && ((uintptr_t)dst & 15) == 0) {
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) *(float4*)(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    if (j < nr) dst[j] = v[j];
+}
+
 // ---- the kernel -------------------------------------------------------------
-template <int EPI, int NPROD>
+template <int EPI, int NPROD, int ROWS>
 __global__ void __launch_bounds__(THREADS, 1)
     chain_gemm_kernel(const __grid_constant__ CUtensorMap tq_hi, const __grid_constant__ CUtensorMap tq_lo,
                       const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
                       int num_kb, EpiParams ep) {
-  using S = Stage<NPROD>;
+  using S = Stage<NPROD, ROWS>;
+  constexpr int STAGES = S::count;
+  constexpr uint32_t TMEM_COLS = ROWS;  // one FP32 column per matrix row (a power of two >= 32)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + STAGES * S::bytes);
@@ -226,7 +244,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int m0 = blockIdx.x * BM;  // first chain of the tile
-  const int n0 = blockIdx.y * BN;  // first matrix row of the tile
+  const int n0 = blockIdx.y * ROWS;  // first matrix row of the tile
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -251,7 +269,9 @@ __global__ void __launch_bounds__(THREADS, 1)
   int tma_issued_stage_uses = 0;  // producer bookkeeping for the abort drain
   if (warp == 0 && lane == 0) {
     // ---------------- TMA producer ----------------
-    const int kb_rot = (int)((blockIdx.x + 7u * blockIdx.y) % (unsigned)num_kb);
+    // (A rotation per 256 rows, whatever the tile: the sums' order, and so their
+    // rounding, does not depend on its width.)
+    const int kb_rot = (int)((blockIdx.x + 7u * (unsigned)(n0 / BN)) % (unsigned)num_kb);
     for (int kb = 0; kb < num_kb; ++kb) {
       const int s = kb % STAGES;
       if (kb >= STAGES) {
@@ -281,7 +301,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
   } else if (warp == 1 && lane == 0) {
     // ---------------- MMA issuer ----------------
-    constexpr uint32_t idesc = idesc_bf16(BM, BN);
+    constexpr uint32_t idesc = idesc_bf16(BM, ROWS);
     bool ok = true;
     for (int kb = 0; kb < num_kb; ++kb) {
       const int s = kb % STAGES;
@@ -347,7 +367,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     double misfit_part = 0.0;
     bool oob = false;
-    for (int cb = half; cb < BN / 16; cb += 2) {
+    for (int cb = half; cb < ROWS / 16; cb += 2) {
       float acc[16];
       if (ready) tmem_ld16(tbase + cb * 16, acc);  // warp-collective: every lane takes part
       if (!live_c) continue;
@@ -381,9 +401,8 @@ __global__ void __launch_bounds__(THREADS, 1)
           if (j < nr) {
             const int64_t r = r0 + j;
             if (EPI == EPI_MLP_HIDDEN) {
-              const float zv = acc[j] + ep.bias[r];
-              ep.z[c * ep.ldz + r] = zv;
-              v = gelu(zv);
+              acc[j] += ep.bias[r];
+              v = gelu(acc[j]);
             } else {
               v = acc[j] * gelu_grad(ep.z[c * ep.ldz + r]);
             }
@@ -391,6 +410,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           a16[j] = __float2bfloat16_rn(v);
           if (j < nr) ep.act_t[(r0 + j) * ep.ld_act_t + c] = a16[j];
         }
+        if (EPI == EPI_MLP_HIDDEN) store_row16(ep.z + c * ep.ldz + r0, acc, nr, ep.ldz);
         // only chunks holding valid rows: the columns past `rows` may belong
         // to another array stored in the same row (the output layer's skip input)
         if (nr > 0 && r0 + 16 <= ep.ld_act) {
@@ -403,11 +423,11 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int j = 0; j < 16; ++j) {
           if (j < nr) {
             const int64_t r = r0 + j;
-            const float yv = acc[j] + ep.bias[r];
-            if (ep.y) ep.y[c * ep.ldy + r] = yv;
-            if (ep.g_state) ep.g_state[r * C + c] = ep.out_scale[r] * yv + ep.out_shift[r];
+            acc[j] += ep.bias[r];
+            if (ep.g_state) ep.g_state[r * C + c] = ep.out_scale[r] * acc[j] + ep.out_shift[r];
           }
         }
+        if (ep.y) store_row16(ep.y + c * ep.ldy + r0, acc, nr, ep.ldy);
       } else {  // EPI_STEP
         // all loads of the chunk first (independent, in flight together)
         float qv[16], pv[16];
@@ -781,39 +801,54 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int
   return HMC_OK;
 }
 
+template <int EPI, int NPROD, int ROWS>
+int launch_tiles(int64_t C, int64_t rows, int64_t K, const void* q_hi, const void* q_lo, int64_t ldq, const void* a_hi,
+                 const void* a_lo, int64_t lda, const EpiParams& ep, cudaStream_t st) {
+  CUtensorMap mq_hi, mq_lo, ma_hi, ma_lo;
+  HMC_TRY(make_map(&mq_hi, q_hi, C, K, ldq, BM));
+  HMC_TRY(make_map(&ma_hi, a_hi, rows, K, lda, ROWS));
+  if (NPROD == 3) {
+    HMC_TRY(make_map(&mq_lo, q_lo, C, K, ldq, BM));
+    HMC_TRY(make_map(&ma_lo, a_lo, rows, K, lda, ROWS));
+  } else {
+    mq_lo = mq_hi;
+    ma_lo = ma_hi;
+  }
+  constexpr int smem = Stage<NPROD, ROWS>::smem;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(chain_gemm_kernel<EPI, NPROD, ROWS>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(chain_gemm_kernel)");
+    attr_set = true;
+  }
+  const int num_kb = (int)((K + BK - 1) / BK);
+  const dim3 grid((unsigned)((C + BM - 1) / BM), (unsigned)((rows + ROWS - 1) / ROWS));
+  EpiParams e = ep;
+  const WaitLimits wl = wait_limits();
+  e.wait_ns = wl.ns;
+  e.withhold = wl.withhold;
+  chain_gemm_kernel<EPI, NPROD, ROWS><<<grid, THREADS, smem, st>>>(mq_hi, mq_lo, ma_hi, ma_lo, num_kb, e);
+  return check_launch("chain_gemm_kernel");
+}
+
+// Tiles of 256 matrix rows read the operands least often; where they are so few
+// that most SMs would idle, eight times as many of 32 rows (512 x 256 outputs,
+// 512 products: 37 us with 4 wide tiles, 8.6 us with 32; the line is where the
+// narrow ones fill the SMs twice).
 template <int EPI, int NPROD = 3>
 int launch(int64_t C, int64_t rows, int64_t K, const void* q_hi, const void* q_lo, int64_t ldq, const void* a_hi,
            const void* a_lo, int64_t lda, const EpiParams& ep, cudaStream_t st) {
   HMC_REQUIRE(C > 0 && rows > 0 && K > 0, "tensor-core contraction: bad sizes");
   HMC_REQUIRE(C < (1ll << 31) && rows < (1ll << 31) && K < (1ll << 31), "tensor-core contraction: too large");
   HMC_REQUIRE(ep.status != nullptr, "tensor-core contraction: null status word");
-  CUtensorMap mq_hi, mq_lo, ma_hi, ma_lo;
-  HMC_TRY(make_map(&mq_hi, q_hi, C, K, ldq, BM));
-  HMC_TRY(make_map(&ma_hi, a_hi, rows, K, lda, BN));
-  if (NPROD == 3) {
-    HMC_TRY(make_map(&mq_lo, q_lo, C, K, ldq, BM));
-    HMC_TRY(make_map(&ma_lo, a_lo, rows, K, lda, BN));
-  } else {
-    mq_lo = mq_hi;
-    ma_lo = ma_hi;
+  const int64_t tiles = (C + BM - 1) / BM * ((rows + BN - 1) / BN);
+  HMC_REQUIRE((rows + BN - 1) / BN <= 65535, "tensor-core contraction: too many rows");
+  // (the fused step and the misfit, whose partial sums are per 256 rows, keep the wide tiles)
+  if constexpr (EPI != EPI_STEP && EPI != EPI_MISFIT) {
+    if (tiles <= 38) return launch_tiles<EPI, NPROD, BN_FEW>(C, rows, K, q_hi, q_lo, ldq, a_hi, a_lo, lda, ep, st);
   }
-  constexpr int smem = STAGES * Stage<NPROD>::bytes + 1024 + 256;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(chain_gemm_kernel<EPI, NPROD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(chain_gemm_kernel)");
-    attr_set = true;
-  }
-  const int num_kb = (int)((K + BK - 1) / BK);
-  const dim3 grid((unsigned)((C + BM - 1) / BM), (unsigned)((rows + BN - 1) / BN));
-  HMC_REQUIRE(grid.y <= 65535, "tensor-core contraction: too many rows");
-  EpiParams e = ep;
-  const WaitLimits wl = wait_limits();
-  e.wait_ns = wl.ns;
-  e.withhold = wl.withhold;
-  chain_gemm_kernel<EPI, NPROD><<<grid, THREADS, smem, st>>>(mq_hi, mq_lo, ma_hi, ma_lo, num_kb, e);
-  return check_launch("chain_gemm_kernel");
+  return launch_tiles<EPI, NPROD, BN>(C, rows, K, q_hi, q_lo, ldq, a_hi, a_lo, lda, ep, st);
 }
 
 }  // namespace tc

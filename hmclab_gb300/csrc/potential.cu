@@ -91,8 +91,21 @@ __global__ void w3_grad_kernel(int64_t B, int64_t n, const float* __restrict__ i
   __shared__ float part[16][33];
   const int64_t j = (int64_t)blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
-  if (j < n)
-    for (int64_t b = threadIdx.y; b < B; b += 16) s += in[b * ldi + j] * gelu_d1(z[b * ldz + j]);
+  if (j < n) {
+    // eight rows' loads in flight at a time; the sum's order is that of the rows
+    int64_t b = threadIdx.y;
+    for (; b + 7 * 16 < B; b += 8 * 16) {
+      float x[8], y[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        x[k] = in[(b + 16 * k) * ldi + j];
+        y[k] = z[(b + 16 * k) * ldz + j];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s = fmaf(x[k], gelu_d1(y[k]), s);
+    }
+    for (; b < B; b += 16) s = fmaf(in[b * ldi + j], gelu_d1(z[b * ldz + j]), s);
+  }
   part[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
   if (threadIdx.y == 0 && j < n) {
