@@ -102,6 +102,189 @@ __global__ void splitk_reduce_kernel(int64_t mn, int splits, T alpha, const T* _
   }
 }
 
+// The FP32 product.  A thread owns RPT rows x 4 columns of the output, CX
+// threads a block's columns and THREADS / CX groups its rows; k runs in chunks of
+// 16 that are loaded one chunk ahead, and a thread reads its rows and columns
+// with RPT + 4 16-byte loads per 16 RPT multiply-adds (the tile kernel above:
+// eight 4-byte loads per 16, and a block that waits for every chunk's loads).
+// Every output is one chain of fused multiply-adds in ascending k, as there, so
+// results do not change.  What bounds it is instruction issue; a block is four
+// warps, one per scheduler, and the rows per thread are those that leave the
+// matrix the least padding: 129 x 129 against 8192 columns, the full mass matrix
+// of a source location, took 26 us (192 padded rows) and takes 13.
+constexpr int KC = 16;
+template <int CX, int RPT, int THREADS, bool B16>
+__global__ void __launch_bounds__(THREADS, 3)
+    gemm_f32_kernel(int64_t M, int64_t N, int64_t K, float alpha, const float* __restrict__ A,
+                    const float* __restrict__ B, const float* __restrict__ bias, float bias_scale,
+                    const float* __restrict__ row_scale, float* out, int accumulate, int64_t k_chunk, float* partial) {
+  constexpr int CT = CX * 4;
+  constexpr int PITCH = KC + 4;  // the row groups of a warp read different banks
+  constexpr int ALOADS = KC * RPT / CX;                         // per thread
+  constexpr int BLOADS = (KC * (B16 ? CX : CT) + THREADS - 1) / THREADS;
+  constexpr int threads = THREADS, groups = threads / CX, rows = groups * RPT;
+  constexpr int buffer = rows * PITCH + KC * CT;  // floats: A chunk [row][k], then B chunk [k][column]
+  __shared__ __align__(16) float sm[2 * buffer];
+  const int tx = threadIdx.x % CX, ty = threadIdx.x / CX;
+  const int64_t row0 = (int64_t)blockIdx.y * rows, col0 = (int64_t)blockIdx.x * CT;
+  const int64_t kb = (int64_t)blockIdx.z * k_chunk;
+  const int64_t ke = kb + k_chunk < K ? kb + k_chunk : K;
+
+  // The next chunk travels in registers while this one is multiplied.  Rows and
+  // columns past the matrix repeat its last ones (their sums are not stored), so
+  // only the last chunk of k checks bounds.
+  float ar[ALOADS], br[B16 ? 4 * BLOADS : BLOADS];
+  constexpr int lstep = threads / KC;
+  const int lr = threadIdx.x / KC, lk = threadIdx.x % KC;
+  uint32_t aoff[ALOADS];  // (launches keep a block's rows of A below 2^31 elements)
+#pragma unroll
+  for (int i = 0; i < ALOADS; ++i) {
+    const int64_t r = lr + i * lstep, last = M - 1 - row0;
+    aoff[i] = (uint32_t)((r < last ? r : last) * K) + (uint32_t)lk;
+  }
+  const float* const abase = A + row0 * K;
+  auto fetch = [&](int64_t k0) {
+    const float* a = abase + k0;
+    if (k0 + KC <= ke) {
+#pragma unroll
+      for (int i = 0; i < ALOADS; ++i) ar[i] = a[aoff[i]];
+    } else {
+#pragma unroll
+      for (int i = 0; i < ALOADS; ++i) ar[i] = k0 + lk < ke ? a[aoff[i]] : 0.f;
+    }
+    const float* b = B + k0 * N + col0;
+    if constexpr (B16) {
+#pragma unroll
+      for (int i = 0; i < BLOADS; ++i) {
+        const int e = threadIdx.x + i * threads;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < KC * CX && k0 + e / CX < ke && col0 + e % CX * 4 < N) v = *(const float4*)(b + e / CX * N + e % CX * 4);
+        br[4 * i] = v.x, br[4 * i + 1] = v.y, br[4 * i + 2] = v.z, br[4 * i + 3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < BLOADS; ++i) {
+        const int e = threadIdx.x + i * threads;
+        br[i] = e < KC * CT && k0 + e / CT < ke && col0 + e % CT < N ? b[e / CT * N + e % CT] : 0.f;
+      }
+    }
+  };
+  auto put = [&](float* As) {
+    float* const Bs = As + rows * PITCH;
+#pragma unroll
+    for (int i = 0; i < ALOADS; ++i) As[(lr + i * lstep) * PITCH + lk] = ar[i];
+    if constexpr (B16) {
+#pragma unroll
+      for (int i = 0; i < BLOADS; ++i) {
+        const int e = threadIdx.x + i * threads;
+        if (e < KC * CX) *(float4*)(Bs + e * 4) = make_float4(br[4 * i], br[4 * i + 1], br[4 * i + 2], br[4 * i + 3]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < BLOADS; ++i) {
+        const int e = threadIdx.x + i * threads;
+        if (e < KC * CT) Bs[e] = br[i];
+      }
+    }
+  };
+
+  float acc[RPT][4];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  int now = 0;
+  if (kb < ke) {
+    fetch(kb);
+    put(sm);
+    __syncthreads();
+  }
+  for (int64_t k0 = kb; k0 < ke; k0 += KC) {
+    const bool more = k0 + KC < ke;
+    if (more) fetch(k0 + KC);
+    const float* As = sm + now * buffer;
+    const float* b = As + rows * PITCH + tx * 4;
+#pragma unroll
+    for (int kk = 0; kk < KC; kk += 4) {
+      float4 av[RPT];
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) av[i] = *(const float4*)(As + (ty + i * groups) * PITCH + kk);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 bv = *(const float4*)(b + (kk + q) * CT);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const float x = q == 0 ? av[i].x : q == 1 ? av[i].y : q == 2 ? av[i].z : av[i].w;
+          acc[i][0] = fmaf(x, bv.x, acc[i][0]);
+          acc[i][1] = fmaf(x, bv.y, acc[i][1]);
+          acc[i][2] = fmaf(x, bv.z, acc[i][2]);
+          acc[i][3] = fmaf(x, bv.w, acc[i][3]);
+        }
+      }
+    }
+    now ^= 1;
+    if (more) put(sm + now * buffer);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int64_t r = row0 + ty + i * groups;
+    if (r >= M) continue;
+    const float bv = bias && !partial ? bias_scale * bias[r] : 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t c = col0 + tx * 4 + j;
+      if (c >= N) continue;
+      if (partial) {
+        partial[((int64_t)blockIdx.z * M + r) * N + c] = acc[i][j];
+        continue;
+      }
+      float v = alpha * acc[i][j] + bv;
+      if (row_scale) v *= row_scale[r];
+      if (accumulate) v += out[r * N + c];
+      out[r * N + c] = v;
+    }
+  }
+}
+
+using F32Kernel = void (*)(int64_t, int64_t, int64_t, float, const float*, const float*, const float*, float, const float*,
+                           float*, int, int64_t, float*);
+template <int CX, int RPT, int THREADS>
+F32Kernel f32_kernel(bool b16) {
+  return b16 ? gemm_f32_kernel<CX, RPT, THREADS, true> : gemm_f32_kernel<CX, RPT, THREADS, false>;
+}
+int gemm_f32(unsigned splits, int64_t m, int64_t n, int64_t k, float alpha, const void* A, const void* B,
+             const void* bias, float bias_scale, const void* row_scale, void* out, int accumulate, int64_t k_chunk,
+             void* partial, cudaStream_t st) {
+  const bool b16 = n % 4 == 0 && ((uintptr_t)B & 15) == 0;
+  F32Kernel kern;
+  int rows, columns, threads;
+  if (n <= 4) {
+    // one model or a few chains: a thread per row, no columns of padding
+    // (14000 x 60, one column: 11.2 us with 64-column tiles, 3.3 us)
+    kern = f32_kernel<1, 1, 64>(b16);
+    rows = 64, columns = 4, threads = 64;
+  } else {
+    int rpt = 0;
+    int64_t least = 0;
+    for (int r : {9, 8, 6, 4, 2}) {
+      const int64_t padded = (m + 16 * r - 1) / (16 * r) * (16 * r);
+      if (rpt == 0 || padded < least) rpt = r, least = padded;
+    }
+    kern = rpt == 9   ? f32_kernel<8, 9, 128>(b16)
+           : rpt == 8 ? f32_kernel<8, 8, 128>(b16)
+           : rpt == 6 ? f32_kernel<8, 6, 128>(b16)
+           : rpt == 4 ? f32_kernel<8, 4, 128>(b16)
+                      : f32_kernel<8, 2, 128>(b16);
+    rows = 16 * rpt, columns = 32, threads = 128;
+  }
+  const dim3 grid((unsigned)((n + columns - 1) / columns), (unsigned)((m + rows - 1) / rows), splits);
+  HMC_REQUIRE(grid.y <= 65535, "hmc_gemm: matrix too large");
+  kern<<<grid, threads, 0, st>>>(m, n, k, alpha, (const float*)A, (const float*)B, (const float*)bias, bias_scale,
+                                 (const float*)row_scale, (float*)out, accumulate, k_chunk, (float*)partial);
+  return check_launch("gemm_f32_kernel");
+}
+
 // The same product for a handful of FP64 columns (one model, a few chains): a
 // warp per row of A and NC columns, its lanes striding over k, so every row
 // of A streams coalesced and 1000 rows occupy the chip, where the tile kernel
@@ -172,10 +355,9 @@ int gemm_ex(int dtype, int64_t m, int64_t n, int64_t k, double alpha, const void
     return gemv<double, 8>(m, n, k, alpha, A, B, bias, bias_scale, row_scale, out, accumulate, stream);
   }
   if (dtype == HMC_F32)
-    gemm_kernel<float><<<grid, 256, 0, stream>>>(m, n, k, (float)alpha, (const float*)A, (const float*)B,
-                                                  (const float*)bias, (float)bias_scale, (const float*)row_scale,
-                                                  (float*)out, accumulate, kc, nullptr);
-  else if (dtype == HMC_F64)
+    return gemm_f32(1, m, n, k, (float)alpha, A, B, bias, (float)bias_scale, row_scale, out, accumulate,
+                    kc, nullptr, stream);
+  if (dtype == HMC_F64)
     gemm_kernel<double><<<grid, 256, 0, stream>>>(m, n, k, alpha, (const double*)A, (const double*)B,
                                                    (const double*)bias, bias_scale, (const double*)row_scale,
                                                    (double*)out, accumulate, kc, nullptr);
@@ -207,9 +389,8 @@ int gemm_splitk(int dtype, int64_t m, int64_t n, int64_t k, double alpha, const 
   const dim3 grid((unsigned)((n + BN - 1) / BN), (unsigned)((m + BM - 1) / BM), (unsigned)splits);
   const unsigned rblocks = blocks_for(m * n, 256) < 152u * 8u ? blocks_for(m * n, 256) : 152u * 8u;
   if (dtype == HMC_F32) {
-    gemm_kernel<float><<<grid, 256, 0, stream>>>(m, n, k, 1.f, (const float*)A, (const float*)B, nullptr, 0.f,
-                                                  nullptr, nullptr, 0, chunk, (float*)work);
-    HMC_TRY(check_launch("gemm_kernel (split k)"));
+    HMC_TRY(gemm_f32((unsigned)splits, m, n, k, 1.f, A, B, nullptr, 0.f, nullptr, nullptr, 0, chunk, work,
+                     stream));
     splitk_reduce_kernel<float><<<rblocks, 256, 0, stream>>>(m * n, (int)splits, (float)alpha, (const float*)work,
                                                             (float*)out, accumulate);
   } else {
