@@ -42,6 +42,14 @@ def _column(coordinates, dimensions):
     return m.reshape(dimensions, 1)
 
 
+def _fills_output(method):
+    """Mark a `_device_misfit` / `_device_gradient` that writes every element of
+    `out` when it does not accumulate, so that callers need not clear it first.
+    An override in a subclass is a function of its own, without the mark."""
+    method.fills_output = True
+    return method
+
+
 class _AbstractDistribution:
     """Plugin base class (reference `base.py:21-374`).
 
@@ -107,12 +115,18 @@ class _AbstractDistribution:
             raise ValueError("the model batch must be contiguous (chains fastest)")
         return _dev.normalise_dtype(M.dtype)
 
+    def _fills(self, method):
+        return getattr(getattr(type(self), method), "fills_output", False)
+
+    def _new_output(self, method, accumulate):
+        return _dev.empty if not accumulate and self._fills(method) else _dev.zeros
+
     def misfit_batch(self, M, out=None, accumulate=False, stream=None):
         """chi for every column of M (device, (d, C)); returns float64 (C,).
         Bounds are not applied here (the sampler tracks them per chain)."""
         dtype = self._check_batch(M)
         if out is None:
-            out = _dev.zeros((M.shape[1],), "float64", M.device)
+            out = self._new_output("_device_misfit", accumulate)((M.shape[1],), "float64", M.device)
         self._device_misfit(M, out, bool(accumulate), dtype, _dev.stream_handle(stream))
         return out
 
@@ -120,7 +134,7 @@ class _AbstractDistribution:
         """d chi / d m for every column of M; returns a (d, C) tensor of M's dtype."""
         dtype = self._check_batch(M)
         if out is None:
-            out = _dev.zeros(tuple(M.shape), dtype, M.device)
+            out = self._new_output("_device_gradient", accumulate)(tuple(M.shape), dtype, M.device)
         self._device_gradient(M, out, bool(accumulate), dtype, _dev.stream_handle(stream))
         return out
 
@@ -268,6 +282,7 @@ class Normal(_AbstractDistribution):
             "icov": _dev.upload(_numpy.asarray(self.inverse_covariance), dtype),
         }
 
+    @_fills_output
     def _device_misfit(self, M, out, accumulate, dtype, stream):
         p = self._params(dtype)
         d, C = M.shape
@@ -279,6 +294,7 @@ class Normal(_AbstractDistribution):
             _lib.call("hmc_normal_full_misfit", _dev.dtype_code(dtype), d, C, M.data_ptr(), p["mean"].data_ptr(),
                       p["icov"].data_ptr(), work.data_ptr(), out.data_ptr(), int(accumulate), stream)
 
+    @_fills_output
     def _device_gradient(self, M, out, accumulate, dtype, stream):
         p = self._params(dtype)
         d, C = M.shape
@@ -335,11 +351,13 @@ class Laplace(_AbstractDistribution):
     def _make_params(self, dtype):
         return {"mean": _dev.upload(self.means[:, 0], dtype), "iw": _dev.upload(self.inverse_dispersions[:, 0], dtype)}
 
+    @_fills_output
     def _device_misfit(self, M, out, accumulate, dtype, stream):
         p = self._params(dtype)
         _lib.call("hmc_laplace_misfit", _dev.dtype_code(dtype), M.shape[0], M.shape[1], M.data_ptr(),
                   p["mean"].data_ptr(), p["iw"].data_ptr(), out.data_ptr(), int(accumulate), stream)
 
+    @_fills_output
     def _device_gradient(self, M, out, accumulate, dtype, stream):
         p = self._params(dtype)
         _lib.call("hmc_laplace_gradient", _dev.dtype_code(dtype), M.shape[0], M.shape[1], M.data_ptr(),
@@ -374,10 +392,12 @@ class Uniform(_AbstractDistribution):
         self.dimensions = int(lower.size)
         self.update_bounds(lower, upper)
 
+    @_fills_output
     def _device_misfit(self, M, out, accumulate, dtype, stream):
         if not accumulate:
             _lib.call("hmc_fill_zero", out.data_ptr(), out.numel() * out.element_size(), stream)
 
+    @_fills_output
     def _device_gradient(self, M, out, accumulate, dtype, stream):
         if not accumulate:
             _lib.call("hmc_fill_zero", out.data_ptr(), out.numel() * out.element_size(), stream)
@@ -422,13 +442,19 @@ class AdditiveDistribution(_AbstractDistribution):
         bounds = sum(d.misfit_bounds(m) for d in self.separate_distributions)
         return float(x.cpu()[0]) + const + bounds + self.misfit_bounds(m)
 
+    @_fills_output
     def _device_misfit(self, M, out, accumulate, dtype, stream):
         for k, dist in enumerate(self.separate_distributions):
             dist._device_misfit(M, out, accumulate or k > 0, dtype, stream)
 
+    @_fills_output
     def _device_gradient(self, M, out, accumulate, dtype, stream):
         for k, dist in enumerate(self.separate_distributions):
             dist._device_gradient(M, out, accumulate or k > 0, dtype, stream)
+
+    def _fills(self, method):
+        parts = self.separate_distributions
+        return super()._fills(method) and len(parts) > 0 and parts[0]._fills(method)
 
     def _device_misfit_after_gradient(self, M, out, accumulate, dtype, stream):
         for k, dist in enumerate(self.separate_distributions):
@@ -589,6 +615,7 @@ class LinearMatrix(_AbstractDistribution):
 
         return dtype == "float32" and _dense_tc.usable(self, C)
 
+    @_fills_output
     def _device_misfit(self, M, out, accumulate, dtype, stream):
         p = self._params(dtype)
         d, C = M.shape
@@ -612,6 +639,7 @@ class LinearMatrix(_AbstractDistribution):
                       p["val"].data_ptr(), p["data"].data_ptr(), p["iv"].data_ptr(), resid.data_ptr(), out.data_ptr(),
                       int(accumulate), stream)
 
+    @_fills_output
     def _device_gradient(self, M, out, accumulate, dtype, stream):
         p = self._params(dtype)
         d, C = M.shape
@@ -695,9 +723,11 @@ class SourceLocation3D(_AbstractDistribution):
                 p["rx"].data_ptr(), p["ry"].data_ptr(), p["rz"].data_ptr(), p["obs"].data_ptr(), p["iv"].data_ptr(),
                 int(self.infer_velocity), float(self.medium_velocity or 0.0))
 
+    @_fills_output
     def _device_misfit(self, M, out, accumulate, dtype, stream):
         _lib.call("hmc_srcloc3d_misfit", *self._args(M, dtype), out.data_ptr(), int(accumulate), stream)
 
+    @_fills_output
     def _device_gradient(self, M, out, accumulate, dtype, stream):
         _lib.call("hmc_srcloc3d_gradient", *self._args(M, dtype), out.data_ptr(), int(accumulate), stream)
 
@@ -991,6 +1021,7 @@ class ElasticFullWaveform2D(_AbstractDistribution):
                 st.zero_()
                 raise DeviceTimeoutError("elastic stencil tile load timed out (bounded wait expired)")
 
+    @_fills_output
     def _device_misfit(self, M, out, accumulate, dtype, stream):
         import ctypes
 
@@ -1010,6 +1041,7 @@ class ElasticFullWaveform2D(_AbstractDistribution):
             return self._device_misfit(M, out, accumulate, dtype, stream)
         _lib.call("hmc_fwi_misfit", ctypes.byref(d), self.config.n_shots, out.data_ptr(), int(accumulate), stream)
 
+    @_fills_output
     def _device_gradient(self, M, out, accumulate, dtype, stream):
         import ctypes
 

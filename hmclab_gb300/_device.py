@@ -12,11 +12,17 @@ except ImportError:  # pragma: no cover - torch is a hard requirement on GPU hos
 DTYPES = {"float32": _lib.HMC_F32, "float64": _lib.HMC_F64}
 
 
+_usable = False  # a device was found: asking again costs 5 us per call
+
+
 def require_cuda():
     """Load the library and check that a CUDA device is usable."""
-    if _torch is None or not _torch.cuda.is_available():
-        raise DeviceUnavailableError("hmclab_gb300 needs a CUDA device; none is available (no CPU fallback)")
-    _lib.load()
+    global _usable
+    if not _usable:
+        if _torch is None or not _torch.cuda.is_available():
+            raise DeviceUnavailableError("hmclab_gb300 needs a CUDA device; none is available (no CPU fallback)")
+        _lib.load()
+        _usable = True
     return _torch.device("cuda", _torch.cuda.current_device())
 
 
@@ -47,7 +53,8 @@ def upload(array, dtype, device=None):
     """Copy a numpy array (any float type) to a contiguous device tensor."""
     device = device or require_cuda()
     a = _np.array(array, dtype=_np.float64, order="C", copy=True)
-    return _torch.from_numpy(a).to(device=device, dtype=torch_dtype(dtype)).contiguous()
+    # rounded on the host, so that one copy is all the device does
+    return _torch.from_numpy(a).to(torch_dtype(dtype)).to(device)
 
 
 def upload_int32(array, device=None):
@@ -62,7 +69,8 @@ def ptr(t):
 
 def stream_handle(stream=None):
     if stream is None:
-        stream = _torch.cuda.current_stream()
+        # the handle alone, without a stream object around it (5 us)
+        return _torch._C._cuda_getCurrentRawStream(_torch.cuda.current_device())
     return stream.cuda_stream
 
 

@@ -338,8 +338,9 @@ def check(rc, name):
 
 
 def call(name, *args):
-    rc = getattr(load(), name)(*args)
-    check(rc, name)
+    rc = getattr(_lib or load(), name)(*args)
+    if rc:
+        check(rc, name)
 
 
 def launch_count():
