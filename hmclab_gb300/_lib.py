@@ -190,6 +190,36 @@ class HmcMlpOut(_ct.Structure):
     ]
 
 
+class HmcPotOut(_ct.Structure):
+    """Mirror of `hmc_pot_out` in include/hmclab_gb300.h."""
+
+    _fields_ = [
+        ("z", c_void_p),
+        ("ldz", c_int64),
+        ("act", c_void_p),
+        ("ld_act", c_int64),
+        ("act_t", c_void_p),
+        ("ld_act_t", c_int64),
+        ("out", c_void_p),
+        ("ld_out", c_int64),
+        ("out_t", c_void_p),
+        ("ld_out_t", c_int64),
+        ("y", c_void_p),
+        ("ldy", c_int64),
+        ("aux", c_void_p),
+        ("ld_aux", c_int64),
+        ("vec", c_void_p),
+        ("f", c_void_p),
+        ("ld_f", c_int64),
+    ]
+
+
+class HmcAdamArray(_ct.Structure):
+    """Mirror of `hmc_adam_array` in include/hmclab_gb300.h."""
+
+    _fields_ = [("n", c_int64), ("w", c_void_p), ("g", c_void_p), ("m", c_void_p), ("v", c_void_p)]
+
+
 HMC_MLP_HIDDEN, HMC_MLP_OUT, HMC_MLP_BACK, HMC_MLP_WGRAD = 0, 1, 2, 3
 HMC_POT_DELTA2, HMC_POT_DELTA1, HMC_POT_DBAR1, HMC_POT_DBAR2, HMC_POT_ZBAR1 = 0, 1, 2, 3, 4
 
@@ -244,6 +274,8 @@ SIGNATURES = {
     "hmc_tc_resid_misfit": [I64, I64, I64, P, P, I64, P, P, I64, P, P, P, P, I, P, S],
     "hmc_tc_partials_size": [I64, I64],
     "hmc_tc_mlp": [I, I64, I64, I64, P, I64, P, I64, P, P, P, S],
+    "hmc_tc_pot": [I, I64, I64, I64, P, I64, P, I64, P, P, P, S],
+    "hmc_mlp_adam_many": [I, P, _ct.c_float, _ct.c_float, _ct.c_float, _ct.c_float, I64, S],
     "hmc_mlp_input": [I64, I64, P, P, P, P, I64, S],
     "hmc_mlp_gather": [I64, I64, P, P, P, P, P, P, P, P, I64, P, I64, P, I64, S],
     "hmc_mlp_loss": [I64, I64, P, I64, P, I64, P, I64, P, I64, P, S],

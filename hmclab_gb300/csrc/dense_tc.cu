@@ -31,6 +31,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "gelu.cuh"
 
 namespace hmc {
 namespace tc {
@@ -60,7 +61,7 @@ static_assert(Stage<3, BN>::smem <= 227 * 1024 && Stage<1, BN_FEW>::smem <= 227 
               "shared memory of a block");
 constexpr int THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 
-enum Epi { EPI_GRAD = 0, EPI_STEP = 1, EPI_MISFIT = 2, EPI_MLP_HIDDEN = 3, EPI_MLP_OUT = 4, EPI_MLP_BACK = 5 };
+enum Epi { EPI_GRAD = 0, EPI_STEP = 1, EPI_MISFIT = 2, EPI_MLP_HIDDEN = 3, EPI_MLP_OUT = 4, EPI_MLP_BACK = 5, EPI_POT = 6 };
 enum Prior { PRIOR_NONE = 0, PRIOR_NORMAL = 1, PRIOR_LAPLACE = 2 };
 
 struct EpiParams {
@@ -101,6 +102,17 @@ struct EpiParams {
   float* g_state;          // [rows][C] scale * y + shift (OUT, may be null)
   const float* out_scale;
   const float* out_shift;
+  // EPI_POT: the element-wise step that follows the contraction (also z, act, act_t, y)
+  int pot_mode;
+  __nv_bfloat16* out;      // [C][ld_out] the step's result (BF16)
+  int64_t ld_out;
+  __nv_bfloat16* out_t;    // [rows][ld_out_t] the same, transposed (may be null)
+  int64_t ld_out_t;
+  const float* aux;        // [C][ld_aux]
+  int64_t ld_aux;
+  const float* vec;        // [rows]
+  float* f;                // [C][ld_f] second result (DBAR1)
+  int64_t ld_f;
   int* status;
   uint64_t wait_ns;  // bounded-wait limit (filled by the launcher)
   int withhold;      // test hook: block (0, 0) skips its first stage's copies
@@ -223,6 +235,38 @@ __device__ __forceinline__ void store_row16(float* dst, const float (&v)[16], in
 #pragma unroll
   for (int j = 0; j < 16; ++j)
     if (j < nr) dst[j] = v[j];
+}
+
+__device__ __forceinline__ void load_row16(float (&v)[16], const float* src, int nr, int64_t ld) {
+  if (nr == 16 && (ld & 3) == 0 && ((uintptr_t)src & 15) == 0) {
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) {
+      const float4 x = *(const float4*)(src + j);
+      v[j] = x.x, v[j + 1] = x.y, v[j + 2] = x.z, v[j + 3] = x.w;
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = j < nr ? src[j] : 0.f;
+}
+// The same in BF16, and transposed: element j of row c goes to dst_t[j][c].
+__device__ __forceinline__ void store_bf16(__nv_bfloat16* dst, int64_t ld, __nv_bfloat16* dst_t, int64_t ld_t,
+                                           const float (&v)[16], int nr) {
+  __align__(16) __nv_bfloat16 h[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16_rn(v[j]);
+  if (nr == 16 && (ld & 7) == 0 && ((uintptr_t)dst & 15) == 0) {
+    ((uint4*)dst)[0] = ((const uint4*)h)[0];
+    ((uint4*)dst)[1] = ((const uint4*)h)[1];
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < nr) dst[j] = h[j];
+  }
+  if (dst_t == nullptr) return;
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    if (j < nr) dst_t[j * ld_t] = h[j];
 }
 
 // ---- the kernel -------------------------------------------------------------
@@ -428,6 +472,44 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
         if (ep.y) store_row16(ep.y + c * ep.ldy + r0, acc, nr, ep.ldy);
+      } else if (EPI == EPI_POT) {
+        // The scalar potential's element-wise steps (potential.cu) on the fresh
+        // product, which then need no pass of their own.
+        if (nr <= 0) continue;
+        float zz[16], au[16], v[16];
+        float* zrow = ep.z + c * ep.ldz + r0;
+        if (ep.pot_mode == HMC_POT_DELTA2) {  // z = acc + b; a = GELU(z); out = vec GELU'(z)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) zz[j] = j < nr ? acc[j] + ep.bias[r0 + j] : 0.f;
+          store_row16(zrow, zz, nr, ep.ldz);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = gelu(zz[j]);
+          store_bf16(ep.act + c * ep.ld_act + r0, ep.ld_act, ep.act_t + r0 * ep.ld_act_t + c, ep.ld_act_t, v, nr);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = j < nr ? ep.vec[r0 + j] * pot::gelu_d1(zz[j]) : 0.f;
+        } else {
+          load_row16(zz, zrow, nr, ep.ldz);
+          if (ep.aux) load_row16(au, ep.aux + c * ep.ld_aux + r0, nr, ep.ld_aux);
+          if (ep.y) store_row16(ep.y + c * ep.ldy + r0, acc, nr, ep.ldy);
+          if (ep.pot_mode == HMC_POT_DBAR1) {
+            float f[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) f[j] = acc[j] * au[j] * pot::gelu_d2(zz[j]);
+            store_row16(ep.f + c * ep.ld_f + r0, f, nr, ep.ld_f);
+          }
+          if (ep.pot_mode == HMC_POT_DBAR2) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = j < nr ? acc[j] * ep.vec[r0 + j] * pot::gelu_d2(zz[j]) : 0.f;
+          } else if (ep.pot_mode == HMC_POT_ZBAR1) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = fmaf(acc[j], pot::gelu_d1(zz[j]), au[j]);
+          } else {  // DELTA1, DBAR1
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = acc[j] * pot::gelu_d1(zz[j]);
+          }
+        }
+        store_bf16(ep.out + c * ep.ld_out + r0, ep.ld_out, ep.out_t ? ep.out_t + r0 * ep.ld_out_t + c : nullptr,
+                   ep.ld_out_t, v, nr);
       } else {  // EPI_STEP
         // all loads of the chunk first (independent, in flight together)
         float qv[16], pv[16];
@@ -1044,6 +1126,49 @@ HMC_API int hmc_tc_mlp(int mode, int64_t M, int64_t N, int64_t K, const void* x,
     default:
       return fail(HMC_ERR_INVALID_ARG, "hmc_tc_mlp: unknown mode %d", mode);
   }
+}
+
+// A contraction and the element-wise step of the scalar potential that follows
+// it (out = that of hmc_pot_elementwise's mode on the product) in one launch.
+HMC_API int hmc_tc_pot(int mode, int64_t M, int64_t N, int64_t K, const void* x, int64_t ldx, const void* w,
+                       int64_t ldw, const float* bias, const hmc_pot_out* out, int* status, void* stream) {
+  HMC_REQUIRE(out != nullptr && x != nullptr && w != nullptr, "hmc_tc_pot: null argument");
+  HMC_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0, "hmc_tc_pot: pitches must be multiples of 8 elements");
+  HMC_REQUIRE(mode >= HMC_POT_DELTA2 && mode <= HMC_POT_ZBAR1, "hmc_tc_pot: unknown mode %d", mode);
+  HMC_REQUIRE(out->z && out->ldz >= N && out->out && out->ld_out >= N, "hmc_tc_pot: missing buffers");
+  HMC_REQUIRE(out->out_t == nullptr || out->ld_out_t >= M, "hmc_tc_pot: transposed pitch");
+  HMC_REQUIRE(out->y == nullptr || out->ldy >= N, "hmc_tc_pot: pitch of the product");
+  if (mode == HMC_POT_DELTA2)
+    HMC_REQUIRE(bias && out->vec && out->act && out->ld_act >= N && out->act_t && out->ld_act_t >= M && !out->y,
+                "hmc_tc_pot: DELTA2 buffers");
+  if (mode == HMC_POT_DBAR2) HMC_REQUIRE(out->vec != nullptr, "hmc_tc_pot: DBAR2 needs vec");
+  if (mode == HMC_POT_DBAR1) HMC_REQUIRE(out->f && out->ld_f >= N, "hmc_tc_pot: DBAR1 buffers");
+  const bool aux = mode == HMC_POT_DBAR1 || mode == HMC_POT_ZBAR1;
+  if (aux) HMC_REQUIRE(out->aux && out->ld_aux >= N, "hmc_tc_pot: missing aux");
+  EpiParams ep = {};
+  ep.C = M;
+  ep.rows = N;
+  ep.bias = bias;
+  ep.status = status;
+  ep.pot_mode = mode;
+  ep.z = out->z;
+  ep.ldz = out->ldz;
+  ep.act = (__nv_bfloat16*)out->act;
+  ep.ld_act = out->ld_act;
+  ep.act_t = (__nv_bfloat16*)out->act_t;
+  ep.ld_act_t = out->ld_act_t;
+  ep.y = out->y;
+  ep.ldy = out->ldy;
+  ep.out = (__nv_bfloat16*)out->out;
+  ep.ld_out = out->ld_out;
+  ep.out_t = (__nv_bfloat16*)out->out_t;
+  ep.ld_out_t = out->ld_out_t;
+  ep.aux = aux ? out->aux : nullptr;
+  ep.ld_aux = out->ld_aux;
+  ep.vec = out->vec;
+  ep.f = out->f;
+  ep.ld_f = out->ld_f;
+  return launch<EPI_POT, 1>(M, N, K, x, nullptr, ldx, w, nullptr, ldw, ep, as_stream(stream));
 }
 
 }  // extern "C"

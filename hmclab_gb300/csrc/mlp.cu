@@ -107,6 +107,23 @@ __global__ void adam_kernel(int64_t n, float* w, const float* __restrict__ g, fl
   }
 }
 
+// The same for several arrays in one launch: blockIdx.y picks the array.
+constexpr int ADAM_MAX = 8;
+struct AdamArrays {
+  hmc_adam_array a[ADAM_MAX];
+};
+__global__ void adam_many_kernel(AdamArrays arrays, float lr, float b1, float b2, float eps, float c1, float c2) {
+  const hmc_adam_array& t = arrays.a[blockIdx.y];
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < t.n; k += (int64_t)gridDim.x * blockDim.x) {
+    const float gk = t.g[k];
+    const float mk = b1 * t.m[k] + (1.f - b1) * gk;
+    const float vk = b2 * t.v[k] + (1.f - b2) * gk * gk;
+    t.m[k] = mk;
+    t.v[k] = vk;
+    t.w[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+  }
+}
+
 __global__ void cast_kernel(int64_t rows, int64_t cols, const float* __restrict__ w, __nv_bfloat16* w16, int64_t ld,
                             __nv_bfloat16* w16t, int64_t ldt) {
   const int64_t total = rows * cols;
@@ -188,6 +205,22 @@ HMC_API int hmc_mlp_adam(int64_t n, float* w, const float* g, float* m, float* v
   const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
   adam_kernel<<<grid_for(n), 256, 0, as_stream(stream)>>>(n, w, g, m, v, lr, beta1, beta2, eps, c1, c2);
   return check_launch("mlp adam_kernel");
+}
+
+HMC_API int hmc_mlp_adam_many(int count, const hmc_adam_array* arrays, float lr, float beta1, float beta2, float eps,
+                              int64_t step, void* stream) {
+  HMC_REQUIRE(count > 0 && count <= ADAM_MAX && arrays && step > 0, "hmc_mlp_adam_many: bad arguments (1 to %d arrays)",
+              ADAM_MAX);
+  AdamArrays a = {};
+  int64_t most = 0;
+  for (int k = 0; k < count; ++k) {
+    a.a[k] = arrays[k];
+    HMC_REQUIRE(a.a[k].n > 0 && a.a[k].w && a.a[k].g && a.a[k].m && a.a[k].v, "hmc_mlp_adam_many: array %d", k);
+    most = a.a[k].n > most ? a.a[k].n : most;
+  }
+  const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
+  adam_many_kernel<<<dim3(grid_for(most), (unsigned)count), 256, 0, as_stream(stream)>>>(a, lr, beta1, beta2, eps, c1, c2);
+  return check_launch("mlp adam_many_kernel");
 }
 
 HMC_API int hmc_mlp_cast(int64_t rows, int64_t cols, const float* w, void* w16, int64_t ld, void* w16_t, int64_t ldt,

@@ -22,18 +22,10 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "gelu.cuh"
 
 namespace hmc {
 namespace pot {
-
-// GELU(z) = z Phi(z): first and second derivatives Phi(z) + z phi(z) and
-// phi(z) (2 - z^2), with Phi(z) = erfc(-z / sqrt 2) / 2 as in the forward
-// epilogue of the contraction kernel.
-__device__ __forceinline__ float normal_pdf(float z) { return 0.39894228040143268f * __expf(-0.5f * z * z); }
-__device__ __forceinline__ float gelu_d1(float z) {
-  return 0.5f * erfcf(-z * 0.70710678118654752f) + z * normal_pdf(z);
-}
-__device__ __forceinline__ float gelu_d2(float z) { return normal_pdf(z) * (2.f - z * z); }
 
 // One 32 x 32 tile of a [B][n] result per block (block 32 x 8): the value of
 // element (b, j) for the selected mode goes to out_bf [B][ld_bf] (BF16), to

@@ -484,6 +484,9 @@ class MLPSurrogate(_Surrogate):
 
 
 
+_POT_PITCH = {"act": "ld_act", "act_t": "ld_act_t", "y": "ldy", "aux": "ld_aux", "f": "ld_f"}
+
+
 def quadratic_fit(x, y, ridge=1e-3):
     """Gradient of the quadratic x^T A x / 2 + beta . x closest to the pairs
     (x_k, y_k) (rows of x, y): the ridge least-squares affine map
@@ -550,8 +553,6 @@ class PotentialSurrogate(_Surrogate):
         self.inv_g = torch.ones(d, **f32)
         self.scale = torch.ones(d, **f32)  # 1 / (s_q sigma_g): grad_x f -> normalised gradient
         self.bias_out = torch.zeros(d, **f32)  # scale * beta - mu_g / sigma_g
-        self.zero_h1 = torch.zeros(h1, **f32)
-        self.zero_h2 = torch.zeros(h2, **f32)
         self.W1_16 = torch.zeros((h1, _pad(d)), **bf)
         self.W1t_16 = torch.zeros((d, _pad(h1)), **bf)
         self.W2_16 = torch.zeros((h2, _pad(h1)), **bf)
@@ -594,10 +595,10 @@ class PotentialSurrogate(_Surrogate):
                 "idx": z((B,), torch.int32), "Xt": z((d, pB), bf), "T": z((B, d), f32), "Y": z((B, d), f32),
                 "D2t": z((h2, pB), bf), "D1t": z((h1, pB), bf),
                 "E": z((B, _pad(d)), bf), "Et": z((d, pB), bf),
-                "DB1": z((B, h1), f32), "UB1": z((B, _pad(h1)), bf), "UB1t": z((h1, pB), bf),
+                "UB1": z((B, _pad(h1)), bf), "UB1t": z((h1, pB), bf),
                 "ZB1p": z((B, h1), f32), "DB2": z((B, h2), f32),
                 "ZB2": z((B, _pad(h2)), bf), "ZB2t": z((h2, pB), bf),
-                "AB1": z((B, h1), f32), "ZB1": z((B, _pad(h1)), bf), "ZB1t": z((h1, pB), bf),
+                "ZB1": z((B, _pad(h1)), bf), "ZB1t": z((h1, pB), bf),
                 "dv": z((B,), f32), "S2t": z((h2, pB), bf), "S1t": z((h1, pB), bf),
             })
         self._bufs[key] = b
@@ -630,11 +631,20 @@ class PotentialSurrogate(_Surrogate):
         _lib.call("hmc_tc_mlp", mode, M, N, K, x.data_ptr(), ldx, w.data_ptr(), w.shape[1],
                   bias.data_ptr() if bias is not None else None, ctypes.byref(out), self.status.data_ptr(), stream)
 
-    def _ew(self, mode, B, n, stream, z, out_bf, out_t=None, inp=None, aux=None, vec=None, out_f=None):
-        _lib.call("hmc_pot_elementwise", mode, B, n, _dev.ptr(inp), inp.shape[1] if inp is not None else 0,
-                  z.data_ptr(), z.shape[1], _dev.ptr(aux), aux.shape[1] if aux is not None else 0, _dev.ptr(vec),
-                  out_bf.data_ptr(), out_bf.stride(0), _dev.ptr(out_t), out_t.shape[1] if out_t is not None else 0,
-                  _dev.ptr(out_f), out_f.shape[1] if out_f is not None else 0, stream)
+    def _pot(self, mode, M, N, K, x, ldx, w, z, out, out_t, stream, bias=None, **arrays):
+        """A contraction with an element-wise step of the potential in its
+        epilogue; `arrays` are further row-major arrays of hmc_pot_out."""
+        import ctypes
+
+        o = _lib.HmcPotOut(z=z.data_ptr(), ldz=z.shape[1], out=out.data_ptr(), ld_out=out.shape[1])
+        if out_t is not None:
+            o.out_t, o.ld_out_t = out_t.data_ptr(), out_t.shape[1]
+        for k, v in arrays.items():
+            setattr(o, k, v.data_ptr())
+            if v.dim() == 2:
+                setattr(o, _POT_PITCH[k], v.shape[1])
+        _lib.call("hmc_tc_pot", mode, M, N, K, x.data_ptr(), ldx, w.data_ptr(), w.shape[1], _dev.ptr(bias),
+                  ctypes.byref(o), self.status.data_ptr(), stream)
 
     def _gradient_pass(self, b, B, stream, training, g_state=None):
         """grad_x f of the rows of b["X"], normalised (y = scale grad_x f +
@@ -645,14 +655,10 @@ class PotentialSurrogate(_Surrogate):
         ldg = b["Ag"].shape[1]
         o = self._out(z=b["Z1"], ldz=h1, act=b["A1"], ld_act=_pad(h1), act_t=b["A1t"], ld_act_t=pB)
         self._mm(_lib.HMC_MLP_HIDDEN, B, h1, d, b["X"], ldg, self.W1_16, P["b1"], o, stream)
-        o = self._out(z=b["Z2"], ldz=h2, act=b["A2"], ld_act=_pad(h2), act_t=b["A2t"], ld_act_t=pB)
-        self._mm(_lib.HMC_MLP_HIDDEN, B, h2, h1, b["A1"], _pad(h1), self.W2_16, P["b2"], o, stream)
-        self._ew(_lib.HMC_POT_DELTA2, B, h2, stream, b["Z2"], b["D2"], b.get("D2t") if training else None,
-                 vec=P["w3"])
-        self._mm(_lib.HMC_MLP_OUT, B, h1, h2, b["D2"], _pad(h2), self.W2t_16, self.zero_h1,
-                 self._out(y=b["U1"], ldy=h1), stream)
-        self._ew(_lib.HMC_POT_DELTA1, B, h1, stream, b["Z1"], b["Ag"], b.get("D1t") if training else None,
-                 inp=b["U1"])
+        self._pot(_lib.HMC_POT_DELTA2, B, h2, h1, b["A1"], _pad(h1), self.W2_16, b["Z2"], b["D2"], b.get("D2t"), stream,
+                  bias=P["b2"], act=b["A2"], act_t=b["A2t"], vec=P["w3"])
+        self._pot(_lib.HMC_POT_DELTA1, B, h1, h2, b["D2"], _pad(h2), self.W2t_16, b["Z1"], b["Ag"], b.get("D1t"), stream,
+                  y=b["U1"])
         if g_state is None:
             o = self._out(y=b["Y"], ldy=d)
         else:
@@ -778,20 +784,16 @@ class PotentialSurrogate(_Surrogate):
                   b["E"].data_ptr(), _pad(d), b["Et"].data_ptr(), pB, self.loss_buf.data_ptr(), h)
         # dW1 = delta1^T e; dbar1 = e W1^T -> ubar1, zbar1 (partial)
         self._wgrad(d, h1, B, b["Et"], b["D1t"], G["W1"], 0, h)
-        self._mm(_lib.HMC_MLP_OUT, B, h1, d, b["E"], _pad(d), self.W1_16, self.zero_h1,
-                 self._out(y=b["DB1"], ldy=h1), h)
-        self._ew(_lib.HMC_POT_DBAR1, B, h1, h, b["Z1"], b["UB1"], b["UB1t"], inp=b["DB1"], aux=b["U1"],
-                 out_f=b["ZB1p"])
+        self._pot(_lib.HMC_POT_DBAR1, B, h1, d, b["E"], _pad(d), self.W1_16, b["Z1"], b["UB1"], b["UB1t"], h,
+                  aux=b["U1"], f=b["ZB1p"])
         # dW2 = delta2^T ubar1; dbar2 = ubar1 W2^T -> dw3, zbar2
         self._wgrad(h1, h2, B, b["UB1t"], b["D2t"], G["W2"], 0, h)
-        self._mm(_lib.HMC_MLP_OUT, B, h2, h1, b["UB1"], _pad(h1), self.W2_16, self.zero_h2,
-                 self._out(y=b["DB2"], ldy=h2), h)
+        self._pot(_lib.HMC_POT_DBAR2, B, h2, h1, b["UB1"], _pad(h1), self.W2_16, b["Z2"], b["ZB2"], b["ZB2t"], h,
+                  y=b["DB2"], vec=P["w3"])
         _lib.call("hmc_pot_w3_grad", B, h2, b["DB2"].data_ptr(), h2, b["Z2"].data_ptr(), h2, G["w3"].data_ptr(), h)
-        self._ew(_lib.HMC_POT_DBAR2, B, h2, h, b["Z2"], b["ZB2"], b["ZB2t"], inp=b["DB2"], vec=P["w3"])
         # abar1 = zbar2 W2 -> zbar1; the forward pass's weight and bias gradients
-        self._mm(_lib.HMC_MLP_OUT, B, h1, h2, b["ZB2"], _pad(h2), self.W2t_16, self.zero_h1,
-                 self._out(y=b["AB1"], ldy=h1), h)
-        self._ew(_lib.HMC_POT_ZBAR1, B, h1, h, b["Z1"], b["ZB1"], b["ZB1t"], inp=b["AB1"], aux=b["ZB1p"])
+        self._pot(_lib.HMC_POT_ZBAR1, B, h1, h2, b["ZB2"], _pad(h2), self.W2t_16, b["Z1"], b["ZB1"], b["ZB1t"], h,
+                  aux=b["ZB1p"])
         self._wgrad(h1, h2, B, b["A1t"], b["ZB2t"], G["W2"], 1, h)
         _lib.call("hmc_mlp_bias_grad", h2, B, b["ZB2t"].data_ptr(), pB, G["b2"].data_ptr(), h)
         self._wgrad(d, h1, B, b["Xt"], b["ZB1t"], G["W1"], 1, h)
@@ -799,9 +801,9 @@ class PotentialSurrogate(_Surrogate):
         if self._vt is not None and self._vt_w > 0:
             self._value_step(b, B, h)
         self.steps += 1
-        for k in P:
-            _lib.call("hmc_mlp_adam", P[k].numel(), P[k].data_ptr(), G[k].data_ptr(), self.m1[k].data_ptr(),
-                      self.m2[k].data_ptr(), lr, beta1, beta2, eps, self.steps, h)
+        arrays = (_lib.HmcAdamArray * len(P))(*(
+            (P[k].numel(), P[k].data_ptr(), G[k].data_ptr(), self.m1[k].data_ptr(), self.m2[k].data_ptr()) for k in P))
+        _lib.call("hmc_mlp_adam_many", len(P), arrays, lr, beta1, beta2, eps, self.steps, h)
         self._cast(h)
         return self.loss_buf
 

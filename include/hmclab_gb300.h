@@ -473,6 +473,17 @@ HMC_API int hmc_mlp_bias_grad(int64_t n, int64_t B, const void* delta_t,
 HMC_API int hmc_mlp_adam(int64_t n, float* w, const float* g, float* m,
                          float* v, float lr, float beta1, float beta2,
                          float eps, int64_t step, void* stream);
+/* The same step for up to 8 arrays of parameters in one launch.             */
+typedef struct hmc_adam_array {
+  int64_t n;
+  float* w;
+  const float* g;
+  float* m;
+  float* v;
+} hmc_adam_array;
+HMC_API int hmc_mlp_adam_many(int count, const hmc_adam_array* arrays, float lr,
+                              float beta1, float beta2, float eps, int64_t step,
+                              void* stream);
 /* FP32 weights w [rows][cols] -> BF16 w16 [rows][ld] and w16_t [cols][ldt]. */
 HMC_API int hmc_mlp_cast(int64_t rows, int64_t cols, const float* w,
                          void* w16, int64_t ld, void* w16_t, int64_t ldt,
@@ -485,8 +496,9 @@ HMC_API int hmc_mlp_record(int64_t d, int64_t C, const float* src, float* dst,
  * MLP surrogate it stands in for distribution.gradient in the leapfrog,
  * Samplers.py:1562,1573).  f(x) = w3 . GELU(W2 GELU(W1 x + b1) + b2)
  * + x^T A x / 2 + beta . x; the leapfrog uses grad_q f, a conservative field.
- * Its contractions run through hmc_tc_mlp; these are the element-wise steps
- * of the gradient pass and of the double backpropagation that trains it.
+ * Its contractions run through hmc_tc_mlp and hmc_tc_pot; these are the
+ * element-wise steps of the gradient pass and of the double backpropagation
+ * that trains it.
  * hmc_pot_elementwise: for every (b < B, j < n), with z [B][ldz]:
  *   HMC_POT_DELTA2  v = vec[j] GELU'(z)
  *   HMC_POT_DELTA1  v = in GELU'(z)
@@ -505,6 +517,34 @@ HMC_API int hmc_pot_elementwise(int mode, int64_t B, int64_t n, const float* in,
                                 const float* vec, void* out_bf, int64_t ld_bf,
                                 void* out_t, int64_t ld_t, float* out_f,
                                 int64_t ldf, void* stream);
+/* hmc_tc_pot: a contraction (operands as for hmc_tc_mlp) with one of these
+ * steps in its epilogue: `in` is the product, which also goes to y [M][ldy]
+ * (nullable); v -> out [M][ld_out] and out_t [N][ld_out_t] (nullable), DBAR1's
+ * second result -> f [M][ld_f].  DELTA2 belongs to a hidden layer: z = product
+ * + bias is written, with GELU(z) -> act, act_t (BF16); the other modes read z. */
+typedef struct hmc_pot_out {
+  float* z;
+  int64_t ldz;
+  void* act; /* BF16 */
+  int64_t ld_act;
+  void* act_t; /* BF16 */
+  int64_t ld_act_t;
+  void* out; /* BF16 */
+  int64_t ld_out;
+  void* out_t; /* BF16 */
+  int64_t ld_out_t;
+  float* y;
+  int64_t ldy;
+  const float* aux;
+  int64_t ld_aux;
+  const float* vec;
+  float* f;
+  int64_t ld_f;
+} hmc_pot_out;
+HMC_API int hmc_tc_pot(int mode, int64_t M, int64_t N, int64_t K,
+                       const void* x, int64_t ldx, const void* w, int64_t ldw,
+                       const float* bias, const hmc_pot_out* out, int* status,
+                       void* stream);
 /* g[j] = sum_b in[b][j] GELU'(z[b][j]) (the gradient of w3).                 */
 HMC_API int hmc_pot_w3_grad(int64_t B, int64_t n, const float* in, int64_t ldi,
                             const float* z, int64_t ldz, float* g,

@@ -91,3 +91,75 @@ def test_few_tiles_split_products(rows, C, K):
     ops = [_operand(big_r, K, 1), _operand(big_r, K, 2) / 256, _operand(big_c, K, 3), _operand(big_c, K, 4) / 256]
     bias = torch.randn(big_r, device="cuda")
     assert torch.equal(product(rows, C, ops), product(big_r, big_c, ops)[:rows, :C])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(256, 512, 512), (1, 16, 30), (130, 48, 65), (100, 37, 40), (2560, 512, 24)])
+def test_potential_steps_in_the_epilogue(M, N, K):
+    """Product and element-wise step in one launch against the product and
+    hmc_pot_elementwise, which evaluate the same expressions.  The product is
+    equal bit for bit; the step may be contracted differently, so its FP32
+    results agree to a few ulp and its BF16 ones to one (2^-7 relative)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    g = torch.Generator(device="cuda").manual_seed(9)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    x, w = _operand(M, K, 1), _operand(N, K, 2)
+    bias, vec, aux, z = rnd(N), rnd(N), rnd(M, N), rnd(M, N)
+    pM, pN = _pad(M), _pad(N) + 16
+    stream = torch.cuda.current_stream().cuda_stream
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    mm = (M, N, K, x.data_ptr(), x.shape[1], w.data_ptr(), w.shape[1])
+    bf = lambda *s: torch.full(s, 7.0, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+
+    for mode in range(5):
+        hidden = mode == _lib.HMC_POT_DELTA2
+        y, zr = torch.zeros((M, N), device="cuda"), z.clone()
+        a1, a1t, want, want_t, wf = bf(M, _pad(N)), bf(N, pM), bf(M, pN), bf(N, pM), torch.zeros((M, N), device="cuda")
+        if hidden:
+            o = _lib.HmcMlpOut(z=zr.data_ptr(), ldz=N, act=a1.data_ptr(), ld_act=_pad(N), act_t=a1t.data_ptr(), ld_act_t=pM)
+            _lib.call("hmc_tc_mlp", _lib.HMC_MLP_HIDDEN, *mm, bias.data_ptr(), ctypes.byref(o), status.data_ptr(), stream)
+        else:
+            zero = torch.zeros(N, device="cuda")
+            o = _lib.HmcMlpOut(y=y.data_ptr(), ldy=N)
+            _lib.call("hmc_tc_mlp", _lib.HMC_MLP_OUT, *mm, zero.data_ptr(), ctypes.byref(o), status.data_ptr(), stream)
+        _lib.call("hmc_pot_elementwise", mode, M, N, y.data_ptr(), N, zr.data_ptr(), N, aux.data_ptr(), N, vec.data_ptr(),
+                  want.data_ptr(), pN, want_t.data_ptr(), pM, wf.data_ptr(), N, stream)
+
+        for transposed in (True, False):
+            y2, z2, f2 = torch.zeros((M, N), device="cuda"), z.clone(), torch.zeros((M, N), device="cuda")
+            a2, a2t, got, got_t = bf(M, _pad(N)), bf(N, pM), bf(M, pN), bf(N, pM)
+            o = _lib.HmcPotOut(z=z2.data_ptr(), ldz=N, act=a2.data_ptr(), ld_act=_pad(N), act_t=a2t.data_ptr(), ld_act_t=pM,
+                               out=got.data_ptr(), ld_out=pN, aux=aux.data_ptr(), ld_aux=N, vec=vec.data_ptr(),
+                               f=f2.data_ptr(), ld_f=N)
+            if transposed:
+                o.out_t, o.ld_out_t = got_t.data_ptr(), pM
+            if not hidden:
+                o.y, o.ldy = y2.data_ptr(), N
+            _lib.call("hmc_tc_pot", mode, *mm, bias.data_ptr(), ctypes.byref(o), status.data_ptr(), stream)
+            torch.cuda.synchronize()
+            assert int(status) == 0
+            assert torch.equal(y, y2) and torch.equal(zr, z2)
+            if hidden:
+                assert torch.equal(a1[:, :N], a2[:, :N]) and torch.equal(a1t[:, :M], a2t[:, :M])
+            close = lambda p, q, ulp: bool(((p.float() - q.float()).abs() <= ulp * q.float().abs() + 1e-6).all())  # noqa: E731
+            assert close(got[:, :N], want[:, :N], 2.0**-7) and torch.all(got[:, N:] == 7.0)
+            assert torch.all(got_t == 7.0) if not transposed else torch.equal(got_t[:, :M], got[:, :N].t())
+            assert close(f2, wf, 2.0**-21) if mode == _lib.HMC_POT_DBAR1 else not bool(f2.any())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [(1,), (300, 7, 70000, 1, 513), (5,) * 8])
+def test_adam_of_several_arrays(sizes):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    stream = torch.cuda.current_stream().cuda_stream
+    one = [[torch.rand(n, device="cuda") for _ in range(4)] for n in sizes]
+    many = [[t.clone() for t in a] for a in one]
+    for step in (1, 2):
+        for w, g, m, v in one:
+            _lib.call("hmc_mlp_adam", w.numel(), w.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), 1e-3, 0.9, 0.999, 1e-8,
+                      step, stream)
+        arrays = (_lib.HmcAdamArray * len(sizes))(*((a[0].numel(), *(t.data_ptr() for t in a)) for a in many))
+        _lib.call("hmc_mlp_adam_many", len(sizes), arrays, 1e-3, 0.9, 0.999, 1e-8, step, stream)
+    assert all(torch.equal(p, q) for a, b in zip(one, many) for p, q in zip(a, b))
