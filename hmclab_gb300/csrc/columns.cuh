@@ -25,8 +25,11 @@ struct ColumnShape {
 
 // Tile width: 32 chains (one 128-byte FP32 row segment per warp), or the next
 // power of two for fewer chains, whose idle lanes then take rows instead.
-// Cluster: doubled while the grid stays within about two resident waves and
-// every lane keeps four rows; fewer than 32 chains always spread over eight
+// Cluster: doubled while the grid stays within one resident wave (two blocks on
+// an SM) and every lane keeps four rows: a block sums, waits for the cluster and
+// then moves rows, and a second wave pays these latencies again (a pass of two
+// proposals of 20 steps, d = 1000, 4096 chains: 2052 us at up to 256 blocks, 2063
+// at 512, 2113 at 1024, 2116 at 128); fewer than 32 chains always spread over eight
 // SMs, because a warp alone on its scheduler issues FP64 at half the SM's rate
 // (d = 1000, one chain: momenta in 13 us on eight SMs,
 // 418 us in one lane of one block's warps).
@@ -38,7 +41,7 @@ inline ColumnShape column_shape(int64_t C, int64_t rows) {
   if (s.log_x < 5) {
     while (s.cluster < 8 && rows >= 16 * s.cluster) s.cluster *= 2;
   } else {
-    while (s.cluster < 8 && 2 * s.cluster * tiles <= 1024 && rows >= 4 * lanes * 2 * s.cluster) s.cluster *= 2;
+    while (s.cluster < 8 && 2 * s.cluster * tiles <= 256 && rows >= 4 * lanes * 2 * s.cluster) s.cluster *= 2;
   }
   return s;
 }

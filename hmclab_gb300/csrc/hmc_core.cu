@@ -341,29 +341,43 @@ __global__ void __launch_bounds__(COL_THREADS) kinetic_kernel(ChainView<T> s, co
 
 // K1, the accept test (FP64, one thread per chain), and the accepted or kept
 // position into q_cur and the sample ring.  Bound by memory latency; d = 4096,
-// 1024 chains, cold cache: 37 us against 565 us.
+// 1024 chains, cold cache: 37 us against 565 us.  The test's operands are loaded
+// while the rows are summed, and without step-size adaptation it needs alpha only
+// to the side of u it falls on (accept_test).
 template <typename T, int MASS>
 __global__ void __launch_bounds__(COL_THREADS) end_kernel(ChainView<T> s, ColumnShape shape) {
   __shared__ ColumnShared sh;
   const ColumnTile t = column_tile(shape, s.C);
   const int64_t c = t.c;
   const int64_t n = s.control[0];
+  // what the accept test needs besides K1, loaded while the rows are summed
+  double x0 = 0.0, x1 = 0.0, k0 = 0.0, b = 1.0, u = 0.0;
+  if (t.first && t.live) {
+    x0 = s.x_cur[c];
+    x1 = s.x_prop[c];
+    k0 = s.k_cur[c];
+    if (s.beta) b = s.beta[c];
+    if (s.flags[c] & HMC_FLAG_OUT_OF_BOUNDS) {
+      x1 = INFINITY;
+      s.x_prop[c] = x1;
+    }
+    if (s.su) {
+      u = s.su[(n % s.slen) * s.C + c];
+    } else {
+      double ue;
+      philox_scalars(s.seed, (uint32_t)c, (uint64_t)n, &ue, &u);
+    }
+  }
   const double ks = column_total(shape, t.live ? kinetic_partial<T, MASS>(s, s.p, s.v, t) : 0.0, sh);
   if (t.first) {
     int accept = 0;
     if (t.live) {
       const double k1 = 0.5 * ks;
       s.k_prop[c] = k1;
-      double x1 = s.x_prop[c];
-      if (s.flags[c] & HMC_FLAG_OUT_OF_BOUNDS) {
-        x1 = INFINITY;
-        s.x_prop[c] = x1;
-      }
-      const double b = s.beta ? s.beta[c] : 1.0;
-      const double h0 = (s.beta ? b * s.x_cur[c] : s.x_cur[c]) + s.k_cur[c];
+      const double h0 = (s.beta ? b * x0 : x0) + k0;
       const double h1 = (s.beta ? b * x1 : x1) + k1;
-      const double alpha = exp(h0 - h1);
       if (s.autotune) {
+        const double alpha = exp(h0 - h1);
         const T eps_now = s.eps[c];
         if (s.rec_eps && n < s.rec_len) {
           s.rec_eps[n * s.C + c] = (double)eps_now;
@@ -374,15 +388,10 @@ __global__ void __launch_bounds__(COL_THREADS) end_kernel(ChainView<T> s, Column
         double e = (double)eps_now - w * (s.target - fmin(a, 1.0));
         if (e <= 0.0) e = fmax(e, s.min_eps);
         s.eps[c] = (T)e;
-      }
-      double u;
-      if (s.su) {
-        u = s.su[(n % s.slen) * s.C + c];
+        accept = alpha > u ? 1 : 0;  // strict; NaN compares false
       } else {
-        double ue;
-        philox_scalars(s.seed, (uint32_t)c, (uint64_t)n, &ue, &u);
+        accept = accept_test(h0 - h1, u) ? 1 : 0;
       }
-      accept = alpha > u ? 1 : 0;  // strict; NaN compares false
       if (accept) {
         s.x_cur[c] = x1;
         s.accepted[c] += 1;
