@@ -676,7 +676,7 @@ __global__ void srcloc_kernel(int64_t E, int64_t S, int64_t C, const T* __restri
 // matters (the kernel above is issue-bound, so instructions are the lever),
 // two stations per instruction on Blackwell's packed FP32 pipe:
 //   - stations staged in pairs, (x_a, x_b, y_a, y_b) and (z_a, z_b), and the
-//     pair data of 16 events x a chunk of stations as (w_a, w_b, o_a, o_b),
+//     pair data of 8 events x a chunk of stations as (w_a, w_b, o_a, o_b),
 //     (w, o) = (1 / std^2, observed time), in shared memory; a NaN
 //     observation or weight, and the padding of an odd chunk, is staged as
 //     (0, 0), which makes every term of that pair zero — the nansum of the
@@ -730,25 +730,33 @@ __device__ __forceinline__ float x2_sum(f32x2 v) {
   return a + b;
 }
 
+// Blocks of 32 chains and 8 events; the blocks of a cluster share a tile's
+// events and add their FP64 parts in block 0.  FP32 arithmetic bounds it (57 % of
+// the pipe over the chip with 16 events per block and a loop over events: 256
+// blocks on 152 SMs left a sixth of it waiting).  32 events, 200 stations,
+// 8192 chains, four proposals of five steps: 1706 us, now 1582.
+constexpr int SL_BY = 8;  // event lanes per block
 template <bool GRAD>
-__global__ void srcloc_f32_kernel(int64_t E, int64_t S, int64_t C, const float* __restrict__ M,
-                                  const float* __restrict__ rx, const float* __restrict__ ry,
-                                  const float* __restrict__ rz, const float* __restrict__ obs,
-                                  const float* __restrict__ iv, int infer_v, float v_fixed, double* out_x,
-                                  float* out_g, int accumulate) {
+__global__ void __launch_bounds__(RED_X * SL_BY, 4)
+    srcloc_f32_kernel(int64_t E, int64_t S, int64_t C, const float* __restrict__ M, const float* __restrict__ rx,
+                      const float* __restrict__ ry, const float* __restrict__ rz, const float* __restrict__ obs,
+                      const float* __restrict__ iv, int infer_v, float v_fixed, double* out_x, float* out_g,
+                      int accumulate, int pairs, int blocks) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ulonglong2* sxy = (ulonglong2*)smem_raw;             // [SL_PAIRS] (x_a, x_b), (y_a, y_b)
-  f32x2* sz = (f32x2*)(sxy + SL_PAIRS);                // [SL_PAIRS] (z_a, z_b)
-  ulonglong2* swo = (ulonglong2*)(sz + SL_PAIRS);      // [SL_EY][SL_PAIRS] (w_a, w_b), (o_a, o_b)
-  __shared__ double red[SL_EY][RED_X + 1];
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
-  const int64_t c = blockIdx.x * (int64_t)RED_X + threadIdx.x;
+  ulonglong2* sxy = (ulonglong2*)smem_raw;  // [pairs] (x_a, x_b), (y_a, y_b)
+  ulonglong2* swo = sxy + pairs;            // [SL_BY][pairs] (w_a, w_b), (o_a, o_b)
+  f32x2* sz = (f32x2*)(swo + SL_BY * pairs);  // [pairs] (z_a, z_b)
+  __shared__ double red[SL_BY][RED_X + 1];
+  __shared__ double part[RED_X];
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = RED_X * SL_BY;
+  const int rank = (int)(blockIdx.x % (unsigned)blocks);
+  const int64_t c = blockIdx.x / (unsigned)blocks * (int64_t)RED_X + threadIdx.x;
   const bool live = c < C;
   const float v = live ? (infer_v ? M[(4 * E) * C + c] : v_fixed) : 1.f;
   const float inv_v = 1.f / v;
   const f32x2 IV = x2_pack(inv_v, inv_v), EPS = x2_pack(1e-30f, 1e-30f);
   double mis = 0.0, gvd_total = 0.0;
-  for (int64_t e0 = 0; e0 < E; e0 += SL_EY) {
+  for (int64_t e0 = rank * SL_BY; e0 < E; e0 += blocks * SL_BY) {
     const int64_t e = e0 + threadIdx.y;
     const bool ev = live && e < E;
     float x = 0.f, y = 0.f, z = 0.f, t0 = 0.f;
@@ -772,9 +780,8 @@ __global__ void srcloc_f32_kernel(int64_t E, int64_t S, int64_t C, const float* 
                                  x2_pack(ry[s0 + a], hb ? ry[s0 + b] : 0.f));
         sz[k] = x2_pack(rz[s0 + a], hb ? rz[s0 + b] : 0.f);
       }
-      for (int k = tid; k < SL_EY * np; k += nthr) {
-        const int ye = k / np, kp = k - ye * np;
-        const int64_t ee = e0 + ye;
+      for (int kp = threadIdx.x; kp < np; kp += RED_X) {
+        const int64_t ee = e;
         float w[2] = {0.f, 0.f}, o[2] = {0.f, 0.f};
         for (int h = 0; h < 2; ++h) {
           const int ks = 2 * kp + h;
@@ -784,11 +791,11 @@ __global__ void srcloc_f32_kernel(int64_t E, int64_t S, int64_t C, const float* 
             if (isnan(w[h]) || isnan(o[h])) w[h] = o[h] = 0.f;
           }
         }
-        swo[ye * SL_PAIRS + kp] = make_ulonglong2(x2_pack(w[0], w[1]), x2_pack(o[0], o[1]));
+        swo[threadIdx.y * pairs + kp] = make_ulonglong2(x2_pack(w[0], w[1]), x2_pack(o[0], o[1]));
       }
       __syncthreads();
       if (!ev) continue;
-      const ulonglong2* my = swo + threadIdx.y * SL_PAIRS;
+      const ulonglong2* my = swo + threadIdx.y * pairs;
       f32x2 ms = zero;
 #pragma unroll 4
       for (int k = 0; k < np; ++k) {
@@ -832,12 +839,22 @@ __global__ void srcloc_f32_kernel(int64_t E, int64_t S, int64_t C, const float* 
       gvd_total += (double)x2_sum(gvd);
     }
   }
-  // Reduce the velocity partial (or the misfit) over the event lanes.
+  // Reduce the velocity partial (or the misfit) over the event lanes and blocks.
   red[threadIdx.y][threadIdx.x] = GRAD ? gvd_total : mis;
   __syncthreads();
-  if (threadIdx.y == 0 && live) {
-    double sum = 0.0;
-    for (int yy = 0; yy < SL_EY; ++yy) sum += red[yy][threadIdx.x];
+  double sum = 0.0;
+  if (threadIdx.y == 0) {
+    for (int yy = 0; yy < SL_BY; ++yy) sum += red[yy][threadIdx.x];
+    part[threadIdx.x] = sum;
+  }
+  if (blocks > 1) {
+    auto tile = cooperative_groups::this_cluster();
+    tile.sync();
+    if (rank == 0 && threadIdx.y == 0)
+      for (int r = 1; r < blocks; ++r) sum += *tile.map_shared_rank(&part[threadIdx.x], r);
+    tile.sync();  // no block leaves while its part is read
+  }
+  if (rank == 0 && threadIdx.y == 0 && live) {
     if (GRAD) {
       if (infer_v) {
         const int64_t o = (4 * E) * C + c;
@@ -861,21 +878,27 @@ int srcloc(bool grad, int64_t E, int64_t S, int64_t C, const void* M, const void
   HMC_REQUIRE(M && rx && ry && rz && obs && iv, "%s: null argument", who);
   HMC_REQUIRE(grad ? out_g != nullptr : out_x != nullptr, "%s: null output", who);
   if (sizeof(T) == 4) {
-    const size_t smem = SL_PAIRS * (sizeof(ulonglong2) + sizeof(f32x2)) + (size_t)SL_EY * SL_PAIRS * sizeof(ulonglong2);
-    auto k32 = grad ? srcloc_f32_kernel<true> : srcloc_f32_kernel<false>;
-    static bool attr_set = false;
-    if (!attr_set) {
-      cudaError_t e1 = cudaFuncSetAttribute(srcloc_f32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem);
-      cudaError_t e2 = cudaFuncSetAttribute(srcloc_f32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem);
-      if (e1 != cudaSuccess || e2 != cudaSuccess)
-        return cuda_fail(e1 != cudaSuccess ? e1 : e2, "cudaFuncSetAttribute(srcloc_f32)");
-      attr_set = true;
-    }
-    k32<<<red_grid(C), dim3(RED_X, SL_EY), smem, st>>>(E, S, C, (const float*)M, (const float*)rx, (const float*)ry,
-                                                        (const float*)rz, (const float*)obs, (const float*)iv, infer_v,
-                                                        (float)v_fixed, out_x, (float*)out_g, accumulate);
+    // stations staged at a time, and blocks that share a tile's events
+    const int pairs = S < SL_CHUNK ? (int)(S + 1) / 2 : SL_PAIRS;
+    const int64_t groups = (E + SL_BY - 1) / SL_BY;
+    const int blocks = groups < 8 ? (int)groups : 8;
+    const int64_t tiles = (C + RED_X - 1) / RED_X;
+    HMC_REQUIRE(tiles * blocks <= 0x7FFFFFFF, "%s: too many chains", who);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * blocks));
+    cfg.blockDim = dim3(RED_X, SL_BY);
+    cfg.dynamicSmemBytes = (size_t)pairs * ((1 + SL_BY) * sizeof(ulonglong2) + sizeof(f32x2));
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {(unsigned)blocks, 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, grad ? srcloc_f32_kernel<true> : srcloc_f32_kernel<false>, E, S, C,
+                                       (const float*)M, (const float*)rx, (const float*)ry, (const float*)rz,
+                                       (const float*)obs, (const float*)iv, infer_v, (float)v_fixed, out_x,
+                                       (float*)out_g, accumulate, pairs, blocks);
+    if (e != cudaSuccess) return cuda_fail(e, who);
     return check_launch(who);
   }
   const size_t smem = 3 * (size_t)S * sizeof(T);
