@@ -944,6 +944,20 @@ static StoreSlot store_slot(const hmc_fwi* s, int n) {
   return {base, base + 2 * cells, 4ll * (n / k) * s->nz};
 }
 
+static int cluster_forward(const ShotForward& a, const Waves& w, bool dry, bool* ran, cudaStream_t st) {
+  *ran = false;
+  if (a.nx > CLUSTER_COLUMNS || a.C > 0x7FFFFFFF / CLUSTER_MAX) return HMC_OK;
+  return a.nx <= 128   ? cluster_forward_at<128>(a, w, dry, ran, st)
+         : a.nx <= 192 ? cluster_forward_at<192>(a, w, dry, ran, st)
+                       : cluster_forward_at<256>(a, w, dry, ran, st);
+}
+static int cluster_adjoint(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st) {
+  *ran = false;
+  if (a.nx > CLUSTER_COLUMNS || a.C > 0x7FFFFFFF / CLUSTER_MAX) return HMC_OK;
+  return a.nx <= 128   ? cluster_adjoint_at<128>(a, dry, ran, st)
+         : a.nx <= 192 ? cluster_adjoint_at<192>(a, dry, ran, st)
+                       : cluster_adjoint_at<256>(a, dry, ran, st);
+}
 static ShotForward forward_args(const hmc_fwi* s, int shot, int store) {
   ShotForward a = {};
   a.nx = s->nx;
@@ -1011,7 +1025,7 @@ static ShotAdjoint adjoint_args(const hmc_fwi* s) {
 // and direct-load kernels take 16.8 / 17.1 / 21.7 us (misfit) and 45 / 46 /
 // 82 us (misfit and gradient) for 1 / 16 / 64 chains, these 2.9 / 5.5 / 15.3 us
 // and 10 / 24 / 60 us; at 160 x 100 cells and 64 chains it is 11.8 and 37.9 us
-// against 7.8 and 38.0 us, the narrowest margin of the grids tried.
+// against 8.1 and 34.7 us, the narrowest margin of the grids tried.
 static int on_chip(const hmc_fwi* s, int store, bool* yes) {
   *yes = false;
   if (!s->status || wait_limits().withhold) return HMC_OK;

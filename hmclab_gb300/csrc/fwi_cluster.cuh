@@ -1,6 +1,6 @@
 // Elastic time loops with the wavefield on chip: one thread-block cluster per
-// chain advances a whole shot in one launch (fwi_cluster_forward.cu,
-// fwi_cluster_adjoint.cu; fwi.cu holds the scheme and the per-step kernels).
+// chain advances a whole shot in one launch (fwi_cluster_forward.cuh,
+// fwi_cluster_adjoint.cuh; fwi.cu holds the scheme and the per-step kernels).
 //
 // A block of the cluster owns RZ consecutive rows of the grid, a thread one
 // column of them; the fields it owns stay in its registers for all time steps.
@@ -35,7 +35,6 @@ constexpr float CC2 = -1.0f / 24.0f;
 
 constexpr int CLUSTER_MAX = 16;      // blocks per cluster (16 needs the non-portable opt-in)
 constexpr int CLUSTER_COLUMNS = 256; // columns of the grid: one thread each, up to 255 registers
-constexpr int PITCH = CLUSTER_COLUMNS;  // row pitch in shared memory, constant so that offsets are immediates
 constexpr int WAVE_SAMPLES = 6000;   // source samples passed by value with a launch
 constexpr int WAVE_TERMS = 32;       // stress terms (a moment tensor with Mxz takes four)
 
@@ -139,7 +138,7 @@ __device__ __forceinline__ void halo_wait(const HaloBarriers& h, int k, uint32_t
   }
 }
 
-// Rows of PITCH floats of shared memory a block needs.
+// Rows of shared memory (one float per column) of shared memory a block needs.
 constexpr int forward_rows(int rz) { return 10 * rz + 12; }
 constexpr int adjoint_rows(int rz) { return 14 * rz + 24; }
 
@@ -148,9 +147,16 @@ constexpr int adjoint_rows(int rz) { return 14 * rz + 24; }
 #define HMC_ADJOINT_STRIPS(X) X(4) X(5) X(7) X(9) X(11) X(14)
 
 // Launch one shot; false when no strip height fits (the caller then runs the
-// per-step kernels).  dry: only tell whether it would run.
-int cluster_forward(const ShotForward& a, const Waves& w, bool dry, bool* ran, cudaStream_t st);
-int cluster_adjoint(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st);
+// per-step kernels).  dry: only tell whether it would run.  The pitch of a row
+// in shared memory is a constant, so that offsets are immediates; a narrow grid
+// takes a narrow one, which lets several blocks share an SM: 64 chains of 100 x
+// 70 cells take 21.4 us per step of misfit and gradient with 256 columns and 15.0
+// with 128 (compiled in fwi_cluster_128.cu, fwi_cluster_192.cu and
+// fwi_cluster_256.cu).
+template <int PITCH>
+int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, bool* ran, cudaStream_t st);
+template <int PITCH>
+int cluster_adjoint_at(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st);
 
 // The strip height for C chains: the cheapest number of waves of resident
 // clusters, a step of a wave costing its rows' instructions (those of all
@@ -160,9 +166,9 @@ struct ClusterChoice {
   double cost = 0.0;
 };
 template <typename Kernel>
-void consider_strip(ClusterChoice& best, Kernel kern, int rz, int rows, int nx, int nz, int64_t C, double row_instr) {
+void consider_strip(ClusterChoice& best, Kernel kern, int rz, int floats, int nx, int nz, int64_t C, double row_instr) {
   const int R = (nz + rz - 1) / rz;
-  const size_t smem = (size_t)rows * PITCH * sizeof(float);
+  const size_t smem = (size_t)floats * sizeof(float);
   if (R > CLUSTER_MAX || smem > 227 * 1024 - 64) return;
   const int threads = (nx + 31) / 32 * 32;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
@@ -194,9 +200,9 @@ void consider_strip(ClusterChoice& best, Kernel kern, int rz, int rows, int nx, 
 }
 
 template <typename Kernel, typename... A>
-int launch_cluster(const char* who, Kernel kern, int rows, int nx, int R, int64_t C, cudaStream_t st, const A&... args) {
+int launch_cluster(const char* who, Kernel kern, int floats, int nx, int R, int64_t C, cudaStream_t st, const A&... args) {
   HMC_REQUIRE(C * R <= 0x7FFFFFFF, "%s: too many chains", who);
-  const size_t smem = (size_t)rows * PITCH * sizeof(float);
+  const size_t smem = (size_t)floats * sizeof(float);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(C * R));
   cfg.blockDim = dim3((unsigned)((nx + 31) / 32 * 32));

@@ -1,5 +1,7 @@
 // Adjoint elastic simulation and gradients of one shot, a cluster per chain
 // (fwi_cluster.cuh).
+#pragma once
+
 #include "fwi_cluster.cuh"
 #include "quotient.cuh"
 
@@ -19,8 +21,9 @@ __device__ __forceinline__ void stage4(float* dst, const float* src) {
 // stored planes of the forward velocities and the parameters sit in shared
 // memory.  A plane's copy starts when the buffer's last reader is done (after
 // the velocity pass) and is waited for before the barrier of the stress pass.
-template <int RZ>
-__global__ void __launch_bounds__(CLUSTER_COLUMNS, 1) cluster_adjoint_kernel(const __grid_constant__ ShotAdjoint g) {
+template <int RZ, int PITCH>
+__global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 7) ? 2 : 1)
+    cluster_adjoint_kernel(const __grid_constant__ ShotAdjoint g) {
   extern __shared__ __align__(16) float smem[];
   __shared__ HaloBarriers bars;
   const int nx = g.nx, nz = g.nz;
@@ -332,11 +335,12 @@ __global__ void __launch_bounds__(CLUSTER_COLUMNS, 1) cluster_adjoint_kernel(con
 }
 #undef HMC_DP
 
-int cluster_adjoint(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st) {
+template <int PITCH>
+int cluster_adjoint_at(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st) {
   *ran = false;
-  if (a.nx > CLUSTER_COLUMNS || a.C > 0x7FFFFFFF / CLUSTER_MAX) return HMC_OK;
   ClusterChoice best;
-#define HMC_STRIP(RZ) consider_strip(best, cluster_adjoint_kernel<RZ>, RZ, adjoint_rows(RZ), a.nx, a.nz, a.C, 210.0);
+#define HMC_STRIP(RZ) \
+  consider_strip(best, cluster_adjoint_kernel<RZ, PITCH>, RZ, adjoint_rows(RZ) * PITCH, a.nx, a.nz, a.C, 210.0);
   HMC_ADJOINT_STRIPS(HMC_STRIP)
 #undef HMC_STRIP
   if (best.rz == 0) return HMC_OK;
@@ -347,8 +351,8 @@ int cluster_adjoint(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st) 
   switch (best.rz) {
 #define HMC_STRIP(RZ) \
   case RZ: \
-    return launch_cluster("cluster_adjoint_kernel", cluster_adjoint_kernel<RZ>, adjoint_rows(RZ), a.nx, best.R, a.C, st, \
-                          g);
+    return launch_cluster("cluster_adjoint_kernel", cluster_adjoint_kernel<RZ, PITCH>, adjoint_rows(RZ) * PITCH, a.nx, \
+                          best.R, a.C, st, g);
     HMC_ADJOINT_STRIPS(HMC_STRIP)
 #undef HMC_STRIP
   }

@@ -1,4 +1,6 @@
 // Forward elastic simulation of one shot, a cluster per chain (fwi_cluster.cuh).
+#pragma once
+
 #include "fwi_cluster.cuh"
 
 namespace hmc {
@@ -7,8 +9,8 @@ namespace fwi {
 #define HMC_DP(a, b, c, d) ((CC1 * ((a) - (b)) + CC2 * ((c) - (d))) * g.inv_h)
 
 // The same expressions as velocity_kernel and stress_kernel, in the same order.
-template <int RZ>
-__global__ void __launch_bounds__(CLUSTER_COLUMNS, RZ <= 10 ? 2 : 1)
+template <int RZ, int PITCH>
+__global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
     cluster_forward_kernel(const __grid_constant__ ShotForward g, const __grid_constant__ Waves src) {
   extern __shared__ __align__(16) float smem[];
   __shared__ HaloBarriers bars;
@@ -257,11 +259,12 @@ __global__ void __launch_bounds__(CLUSTER_COLUMNS, RZ <= 10 ? 2 : 1)
 }
 #undef HMC_DP
 
-int cluster_forward(const ShotForward& a, const Waves& w, bool dry, bool* ran, cudaStream_t st) {
+template <int PITCH>
+int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, bool* ran, cudaStream_t st) {
   *ran = false;
-  if (a.nx > CLUSTER_COLUMNS || a.C > 0x7FFFFFFF / CLUSTER_MAX) return HMC_OK;
   ClusterChoice best;
-#define HMC_STRIP(RZ) consider_strip(best, cluster_forward_kernel<RZ>, RZ, forward_rows(RZ), a.nx, a.nz, a.C, 75.0);
+#define HMC_STRIP(RZ) \
+  consider_strip(best, cluster_forward_kernel<RZ, PITCH>, RZ, forward_rows(RZ) * PITCH, a.nx, a.nz, a.C, 75.0);
   HMC_FORWARD_STRIPS(HMC_STRIP)
 #undef HMC_STRIP
   if (best.rz == 0) return HMC_OK;
@@ -272,8 +275,8 @@ int cluster_forward(const ShotForward& a, const Waves& w, bool dry, bool* ran, c
   switch (best.rz) {
 #define HMC_STRIP(RZ) \
   case RZ: \
-    return launch_cluster("cluster_forward_kernel", cluster_forward_kernel<RZ>, forward_rows(RZ), a.nx, best.R, a.C, st, \
-                          g, w);
+    return launch_cluster("cluster_forward_kernel", cluster_forward_kernel<RZ, PITCH>, forward_rows(RZ) * PITCH, a.nx, \
+                          best.R, a.C, st, g, w);
     HMC_FORWARD_STRIPS(HMC_STRIP)
 #undef HMC_STRIP
   }

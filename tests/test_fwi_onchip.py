@@ -47,7 +47,7 @@ def _config(nx, nz, nt=60, pad=8, **kw):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nx,nz", [(15, 12), (16, 21), (47, 39), (48, 40), (49, 41), (84, 64), (112, 65), (124, 66), (61, 96),
-                                   (240, 97), (239, 138), (100, 208)])
+                                   (240, 97), (239, 138), (100, 208), (113, 50), (176, 45), (177, 30)])
 @pytest.mark.parametrize("C", [1, 3])
 def test_strips_and_columns(nx, nz, C):
     _check(_config(nx, nz), C)
