@@ -290,6 +290,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int m0 = blockIdx.x * BM;  // first chain of the tile
   const int n0 = blockIdx.y * ROWS;  // first matrix row of the tile
 
+  // Narrow tiles come in chains of short launches: the next one may be set up
+  // while this one runs (programmatic dependent launch).  It touches memory
+  // only after its wait below.
+  if (ROWS == BN_FEW) asm volatile("griddepcontrol.launch_dependents;" :::);
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
@@ -309,6 +313,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (ROWS == BN_FEW) asm volatile("griddepcontrol.wait;" ::: "memory");  // earlier launches are complete
 
   int tma_issued_stage_uses = 0;  // producer bookkeeping for the abort drain
   if (warp == 0 && lane == 0) {
@@ -910,7 +915,19 @@ int launch_tiles(int64_t C, int64_t rows, int64_t K, const void* q_hi, const voi
   const WaitLimits wl = wait_limits();
   e.wait_ns = wl.ns;
   e.withhold = wl.withhold;
-  chain_gemm_kernel<EPI, NPROD, ROWS><<<grid, THREADS, smem, st>>>(mq_hi, mq_lo, ma_hi, ma_lo, num_kb, e);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ROWS == BN_FEW ? 1 : 0;
+  cudaError_t le =
+      cudaLaunchKernelEx(&cfg, chain_gemm_kernel<EPI, NPROD, ROWS>, mq_hi, mq_lo, ma_hi, ma_lo, num_kb, e);
+  if (le != cudaSuccess) return cuda_fail(le, "chain_gemm_kernel");
   return check_launch("chain_gemm_kernel");
 }
 
