@@ -198,6 +198,30 @@ __device__ __forceinline__ T scaled_step(double coeff, bool single, T e) {
 }
 inline bool is_single(double coeff) { return (double)(float)coeff == coeff; }
 
+// Short kernels that follow one another on a stream (the surrogates' training
+// steps) overlap their launch latencies: each is launched with programmatic
+// stream serialisation, lets its successor be set up at once, and touches memory
+// only after its predecessors have completed.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" :::);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+int launch_chained(const char* who, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) return cuda_fail(e, who);
+  return check_launch(who);
+}
+
 // sqrt of a mass: FP32 through the correctly rounded single-precision root,
 // which equals the FP64 root rounded to FP32.
 __device__ __forceinline__ float mass_root(float m) { return sqrtf(m); }

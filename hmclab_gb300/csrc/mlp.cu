@@ -22,6 +22,7 @@ inline unsigned grid_for(int64_t n) {
 // exactly K = d columns, and the rest of a row may hold other data.
 __global__ void input_kernel(int64_t d, int64_t C, const float* __restrict__ q, const float* __restrict__ mu,
                              const float* __restrict__ inv_s, __nv_bfloat16* x, int64_t ldx) {
+  chain_begin();
   __shared__ float tile[32][33];
   const int64_t i0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
   for (int y = threadIdx.y; y < 32; y += blockDim.y) {
@@ -40,6 +41,7 @@ __global__ void gather_kernel(int64_t B, int64_t d, const int32_t* __restrict__ 
                               const float* __restrict__ inv_s, const float* __restrict__ gmu,
                               const float* __restrict__ ginv, __nv_bfloat16* x, int64_t ldx, __nv_bfloat16* xt,
                               int64_t ldxt, float* t, int64_t ldt) {
+  chain_begin();
   const int64_t total = B * d;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = e / d, i = e % d;
@@ -86,6 +88,7 @@ __global__ void sum_partials_kernel(int n, const double* __restrict__ p, double 
 
 // One warp per row: db[r] = sum_c delta_t[r][c].
 __global__ void bias_grad_kernel(int64_t n, int64_t B, const __nv_bfloat16* __restrict__ dt, int64_t ld, float* db) {
+  chain_begin();
   const int64_t r = blockIdx.x * (int64_t)(blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
   if (r >= n) return;
@@ -113,6 +116,7 @@ struct AdamArrays {
   hmc_adam_array a[ADAM_MAX];
 };
 __global__ void adam_many_kernel(AdamArrays arrays, float lr, float b1, float b2, float eps, float c1, float c2) {
+  chain_begin();
   const hmc_adam_array& t = arrays.a[blockIdx.y];
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < t.n; k += (int64_t)gridDim.x * blockDim.x) {
     const float gk = t.g[k];
@@ -126,6 +130,7 @@ __global__ void adam_many_kernel(AdamArrays arrays, float lr, float b1, float b2
 
 __global__ void cast_kernel(int64_t rows, int64_t cols, const float* __restrict__ w, __nv_bfloat16* w16, int64_t ld,
                             __nv_bfloat16* w16t, int64_t ldt) {
+  chain_begin();
   const int64_t total = rows * cols;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / cols, c = e % cols;
@@ -164,8 +169,8 @@ HMC_API int hmc_mlp_input(int64_t d, int64_t C, const float* q, const float* mu,
   HMC_REQUIRE(q && mu && inv_sigma && x, "hmc_mlp_input: null argument");
   HMC_REQUIRE((d + 31) / 32 <= 65535, "hmc_mlp_input: too many features");
   const dim3 grid((unsigned)((C + 31) / 32), (unsigned)((d + 31) / 32));
-  input_kernel<<<grid, dim3(32, 8), 0, as_stream(stream)>>>(d, C, q, mu, inv_sigma, (__nv_bfloat16*)x, ldx);
-  return check_launch("mlp input_kernel");
+  return launch_chained("mlp input_kernel", input_kernel, grid, dim3(32, 8), as_stream(stream), d, C, q, mu, inv_sigma,
+                        (__nv_bfloat16*)x, ldx);
 }
 
 HMC_API int hmc_mlp_gather(int64_t B, int64_t d, const int32_t* idx, const float* q_store, const float* g_store,
@@ -174,10 +179,9 @@ HMC_API int hmc_mlp_gather(int64_t B, int64_t d, const int32_t* idx, const float
   HMC_REQUIRE(B > 0 && d > 0 && ldx >= d && ldxt >= B && ldt >= d, "hmc_mlp_gather: bad sizes");
   HMC_REQUIRE(idx && q_store && g_store && mu && inv_sigma && g_mu && g_inv_sigma && x && x_t && t,
               "hmc_mlp_gather: null argument");
-  gather_kernel<<<grid_for(B * d), 256, 0, as_stream(stream)>>>(B, d, idx, q_store, g_store, mu, inv_sigma, g_mu,
-                                                               g_inv_sigma, (__nv_bfloat16*)x, ldx,
-                                                               (__nv_bfloat16*)x_t, ldxt, t, ldt);
-  return check_launch("mlp gather_kernel");
+  return launch_chained("mlp gather_kernel", gather_kernel, grid_for(B * d), 256, as_stream(stream), B, d, idx,
+                        q_store, g_store, mu, inv_sigma, g_mu, g_inv_sigma, (__nv_bfloat16*)x, ldx,
+                        (__nv_bfloat16*)x_t, ldxt, t, ldt);
 }
 
 HMC_API int hmc_mlp_loss(int64_t B, int64_t n, const float* y, int64_t ldy, const float* t, int64_t ldt, void* dy,
@@ -195,8 +199,8 @@ HMC_API int hmc_mlp_loss(int64_t B, int64_t n, const float* y, int64_t ldy, cons
 
 HMC_API int hmc_mlp_bias_grad(int64_t n, int64_t B, const void* delta_t, int64_t ld, float* db, void* stream) {
   HMC_REQUIRE(n > 0 && B > 0 && ld >= B && delta_t && db, "hmc_mlp_bias_grad: bad arguments");
-  bias_grad_kernel<<<blocks_for(n, 8), 256, 0, as_stream(stream)>>>(n, B, (const __nv_bfloat16*)delta_t, ld, db);
-  return check_launch("mlp bias_grad_kernel");
+  return launch_chained("mlp bias_grad_kernel", bias_grad_kernel, blocks_for(n, 8), 256, as_stream(stream), n, B,
+                        (const __nv_bfloat16*)delta_t, ld, db);
 }
 
 HMC_API int hmc_mlp_adam(int64_t n, float* w, const float* g, float* m, float* v, float lr, float beta1, float beta2,
@@ -219,16 +223,15 @@ HMC_API int hmc_mlp_adam_many(int count, const hmc_adam_array* arrays, float lr,
     most = a.a[k].n > most ? a.a[k].n : most;
   }
   const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-  adam_many_kernel<<<dim3(grid_for(most), (unsigned)count), 256, 0, as_stream(stream)>>>(a, lr, beta1, beta2, eps, c1, c2);
-  return check_launch("mlp adam_many_kernel");
+  return launch_chained("mlp adam_many_kernel", adam_many_kernel, dim3(grid_for(most), (unsigned)count), 256,
+                        as_stream(stream), a, lr, beta1, beta2, eps, c1, c2);
 }
 
 HMC_API int hmc_mlp_cast(int64_t rows, int64_t cols, const float* w, void* w16, int64_t ld, void* w16_t, int64_t ldt,
                          void* stream) {
   HMC_REQUIRE(rows > 0 && cols > 0 && ld >= cols && ldt >= rows && w && w16 && w16_t, "hmc_mlp_cast: bad arguments");
-  cast_kernel<<<grid_for(rows * cols), 256, 0, as_stream(stream)>>>(rows, cols, w, (__nv_bfloat16*)w16, ld,
-                                                                    (__nv_bfloat16*)w16_t, ldt);
-  return check_launch("mlp cast_kernel");
+  return launch_chained("mlp cast_kernel", cast_kernel, grid_for(rows * cols), 256, as_stream(stream), rows, cols, w,
+                        (__nv_bfloat16*)w16, ld, (__nv_bfloat16*)w16_t, ldt);
 }
 
 HMC_API int hmc_mlp_record(int64_t d, int64_t C, const float* src, float* dst, int64_t base, void* stream) {

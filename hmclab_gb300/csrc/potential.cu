@@ -1,5 +1,6 @@
 // Element-wise kernels of the scalar-potential surrogate; its contractions run
-// in dense_tc.cu (hmc_tc_mlp, OUT and WGRAD modes).
+// in dense_tc.cu (hmc_tc_mlp and hmc_tc_pot, whose epilogues evaluate the steps
+// of elementwise_kernel on the fresh product).
 //
 // The surrogate is a potential f(x) = w3 . GELU(W2 GELU(W1 x + b1) + b2)
 // + x^T A x / 2 + beta . x of the normalised position x = (q - mu) / s; the
@@ -80,6 +81,7 @@ __global__ void elementwise_kernel(int mode, int64_t B, int64_t n, const float* 
 // column are added in a fixed order (deterministic).
 __global__ void w3_grad_kernel(int64_t B, int64_t n, const float* __restrict__ in, int64_t ldi,
                                const float* __restrict__ z, int64_t ldz, float* g) {
+  chain_begin();
   __shared__ float part[16][33];
   const int64_t j = (int64_t)blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
@@ -112,6 +114,7 @@ __global__ void w3_grad_kernel(int64_t B, int64_t n, const float* __restrict__ i
 __global__ void loss_kernel(int64_t B, int64_t n, const float* __restrict__ y, int64_t ldy,
                             const float* __restrict__ t, int64_t ldt, const float* __restrict__ scale,
                             __nv_bfloat16* e, int64_t lde, __nv_bfloat16* et, int64_t ldet, double* partial) {
+  chain_begin();
   __shared__ double sh[256];
   double acc = 0.0;
   const int64_t total = B * n;
@@ -135,6 +138,7 @@ __global__ void loss_kernel(int64_t B, int64_t n, const float* __restrict__ y, i
 // One warp: lane l adds partials l, l + 32, ...; the lanes' sums are combined
 // by a fixed shuffle tree (deterministic).
 __global__ void sum_kernel(int n, const double* __restrict__ p, double scale, double* out) {
+  chain_begin();
   double s = 0.0;
   for (int k = threadIdx.x; k < n; k += 32) s += p[k];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -216,6 +220,7 @@ __global__ void scale_columns_kernel(int64_t rows, int64_t B, const __nv_bfloat1
 __global__ void scaled_cast_kernel(int64_t rows, int64_t cols, const float* __restrict__ src, int64_t lds,
                                    int transposed, const float* __restrict__ scale, __nv_bfloat16* dst, int64_t ldd,
                                    int64_t k0) {
+  chain_begin();
   __shared__ float tile[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
   if (transposed) {
@@ -280,8 +285,8 @@ HMC_API int hmc_pot_elementwise(int mode, int64_t B, int64_t n, const float* in,
 HMC_API int hmc_pot_w3_grad(int64_t B, int64_t n, const float* in, int64_t ldi, const float* z, int64_t ldz,
                             float* g, void* stream) {
   HMC_REQUIRE(B > 0 && n > 0 && in && z && g && ldi >= n && ldz >= n, "hmc_pot_w3_grad: bad arguments");
-  w3_grad_kernel<<<(unsigned)((n + 31) / 32), dim3(32, 16), 0, as_stream(stream)>>>(B, n, in, ldi, z, ldz, g);
-  return check_launch("pot w3_grad_kernel");
+  return launch_chained("pot w3_grad_kernel", w3_grad_kernel, (unsigned)((n + 31) / 32), dim3(32, 16),
+                        as_stream(stream), B, n, in, ldi, z, ldz, g);
 }
 
 HMC_API int hmc_pot_loss(int64_t B, int64_t n, const float* y, int64_t ldy, const float* t, int64_t ldt,
@@ -291,11 +296,10 @@ HMC_API int hmc_pot_loss(int64_t B, int64_t n, const float* y, int64_t ldy, cons
   HMC_REQUIRE(y && t && scale && e && e_t && loss, "hmc_pot_loss: null argument");
   const unsigned b = blocks_for(B * n, 256);
   const unsigned grid = b > 1024u ? 1024u : b;
-  loss_kernel<<<grid, 256, 0, as_stream(stream)>>>(B, n, y, ldy, t, ldt, scale, (__nv_bfloat16*)e, lde,
-                                                   (__nv_bfloat16*)e_t, ldet, loss + 1);
-  HMC_TRY(check_launch("pot loss_kernel"));
-  sum_kernel<<<1, 32, 0, as_stream(stream)>>>((int)grid, loss + 1, 1.0 / (double)B, loss);
-  return check_launch("pot sum_kernel");
+  HMC_TRY(launch_chained("pot loss_kernel", loss_kernel, grid, 256, as_stream(stream), B, n, y, ldy, t, ldt, scale,
+                         (__nv_bfloat16*)e, lde, (__nv_bfloat16*)e_t, ldet, loss + 1));
+  return launch_chained("pot sum_kernel", sum_kernel, 1, 32, as_stream(stream), (int)grid, loss + 1, 1.0 / (double)B,
+                        loss);
 }
 
 HMC_API int hmc_pot_value_residual(int64_t B, int64_t h, const void* a2, int64_t lda, const float* w3,
@@ -332,9 +336,8 @@ HMC_API int hmc_pot_scaled_cast(int64_t rows, int64_t cols, const float* src, in
   HMC_REQUIRE(lds >= (transposed ? rows : cols), "hmc_pot_scaled_cast: source pitch");
   HMC_REQUIRE((rows + 31) / 32 <= 65535, "hmc_pot_scaled_cast: too many rows");
   const dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32));
-  scaled_cast_kernel<<<grid, dim3(32, 8), 0, as_stream(stream)>>>(rows, cols, src, lds, transposed, scale,
-                                                                  (__nv_bfloat16*)dst, ldd, k0);
-  return check_launch("pot scaled_cast_kernel");
+  return launch_chained("pot scaled_cast_kernel", scaled_cast_kernel, grid, dim3(32, 8), as_stream(stream), rows, cols,
+                        src, lds, transposed, scale, (__nv_bfloat16*)dst, ldd, k0);
 }
 
 }  // extern "C"
