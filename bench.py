@@ -61,27 +61,6 @@ def peaks():
         return 6800.0, 1900.0, 1700.0, "fallback"
 
 
-def l2_copy_rate(mbytes=40, reps=50):
-    """Read + write bandwidth (GB/s) of a device copy whose source and
-    destination (2 x `mbytes` MB) stay resident in the 129 MB L2: the roof of
-    kernels whose working set lives in L2 (the elastic stencils of one shot),
-    measured in the same process with CUDA events, after warm-up."""
-    import torch
-
-    n = mbytes * 1024 * 1024 // 4
-    src = torch.ones(n, dtype=torch.float32, device="cuda")
-    dst = torch.empty_like(src)
-    for _ in range(5):
-        dst.copy_(src)
-    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    e0.record()
-    for _ in range(reps):
-        dst.copy_(src)
-    e1.record()
-    e1.synchronize()
-    return 2.0 * 4 * n * reps / (e0.elapsed_time(e1) / 1e3) / 1e9
-
-
 # ---------------------------------------------------------------------------
 # Workload: dense linear, 4096 chains
 # ---------------------------------------------------------------------------
@@ -204,7 +183,7 @@ class Cfg1Workload:
     # gradients and one misfit, each a 50 x 50 product
     def roofline_spec(self, smp):
         work = float(self.proposals_per_step) * (self.L + 1) * 2 * self.n_model**2
-        return {"kernel": "persistent_dense_kernel (whole proposals, one warp per chain, GtG in shared memory)",
+        return {"kernel": "persistent_rows_kernel (whole proposals, the chain's rows spread over a cluster of blocks)",
                 "bound": "fp64", "unit": "TFLOP/s", "work": work, "work_name": "algorithmic_flop_per_launch",
                 "extra": {"proposals_per_launch": self.proposals_per_step, "persistent": smp._persistent is not None}}
 
@@ -395,15 +374,6 @@ FWI_REFERENCE = os.path.join(ROOT, "tests", "golden", "fwi_reference.npz")
 # Monte Carlo error (|z| at most this, over all 600 parameters)
 FWI_MIN_TRUNCATED = 0.95
 FWI_MAX_Z = 4.5
-# DRAM bytes (read + write) of one forward time step at C = 64 from one ncu
-# capture of velocity_tma_kernel (60.5 + 0.4 MB) and stress_tma_kernel
-# (69.0 + 1.2 MB) on a cold cache; in the time loop the fields stay in L2 and
-# DRAM moves less
-FWI_STEP_DRAM_BYTES = 131.0e6
-# DRAM bytes of one time step of an exact gradient at C = 64 (ncu, cold cache):
-# forward with the velocity store 131 MB + adjoint velocity pass 195.6 MB +
-# adjoint stress pass 70.7 MB
-FWI_GRADIENT_STEP_DRAM_BYTES = 397.3e6
 
 
 class FwiWorkload:
@@ -462,14 +432,24 @@ class FwiWorkload:
         return dict(stepsize=self.stepsize, amount_of_steps=self.L, mass_matrix=self.mass(), chains=self.chains,
                     dtype="float32")
 
-    # algorithmic HBM bytes of one forward time step (velocity + stress
-    # kernels) for all chains: velocity phase reads vx, vz, sxx, szz, sxz, bx,
+    # bytes one forward time step would move if the fields lived in memory, for
+    # all chains: velocity phase reads vx, vz, sxx, szz, sxz, bx,
     # bz and writes vx, vz; stress phase reads vx, vz, sxx, szz, sxz, l2m, lam,
     # muxz and writes sxx, szz, sxz: 20 FP32 words per cell and chain
     def stencil_bytes_per_step(self):
         return 80.0 * self.cells * self.chains
 
-    # algorithmic HBM bytes of one time step of an exact gradient: the forward
+    # FP32 operations of one forward time step (a stencil difference is 6, its
+    # use in an update 3 to 4, the taper 1 per field) and of one time step of
+    # an exact gradient: that plus the adjoint velocity pass (30), its scaled
+    # operands (4), the five correlations (48) and the adjoint stress pass (40)
+    def stencil_flops_per_step(self):
+        return 72.0 * self.cells * self.chains
+
+    def gradient_flops_per_step(self):
+        return 194.0 * self.cells * self.chains
+
+    # the same for one time step of an exact gradient: the forward
     # step with the velocity store (80 + 8 B) plus the adjoint velocity pass
     # (112 B: adjoint fields, temporaries, stored velocities of two steps,
     # read-modify-write of five gradient accumulators) and stress pass (56 B)
@@ -1159,34 +1139,26 @@ def run_fwi_arm(args, wl):
                  f"{B} plain HMC proposals of every chain (the fallback the screen chose)")
 
     hbm, bf16, bf16s, src = peaks()
-    achieved = wl.stencil_bytes_per_step() / t_step / 1e9
-    l2 = l2_copy_rate()
+    # the fields of a shot stay in registers and shared memory, so FP32 issue is
+    # what bounds a step; memory sees the stored wavefield only
+    fp32 = 152 * 128 * 2 * 2.07e9 / 1e12
+    achieved = wl.stencil_flops_per_step() / t_step / 1e12
+    on_chip = ("a cluster of blocks holds each chain's fields in registers and shared memory for a whole shot; the "
+               "same step through memory would move `bytes_through_memory`")
     forward_roof = {
-        "kernel": "fwi forward time step: velocity_tma_kernel + stress_tma_kernel (the exact misfit)",
-        "bound": "l2", "achieved": achieved, "peak": l2, "unit": "GB/s", "frac": achieved / l2,
-        "peak_source": "measured in this run: read + write rate of a copy over a 2 x 40 MB L2-resident buffer",
-        "hbm_peak": hbm, "hbm_peak_source": src, "frac_of_hbm": achieved / hbm,
-        "traffic": FWI_STEP_DRAM_BYTES, "traffic_source": "ncu capture of one velocity + one stress launch at "
-                                                          "C = 64, default (cold) cache control",
-        "step_s": t_step, "algorithmic_bytes_per_step": wl.stencil_bytes_per_step(),
-        "note": "one shot's fields and parameters (86 MB at 64 chains) stay in the 129 MB L2 over the time loop, so "
-                "the binding roof is the L2 rate, not HBM; DRAM traffic per step (`traffic`, cold cache) is 0.76 "
-                "of the algorithmic bytes"}
+        "kernel": "fwi forward time step: cluster_forward_kernel (the exact misfit)",
+        "bound": "fp32", "achieved": achieved, "peak": fp32, "unit": "TFLOP/s", "frac": achieved / fp32,
+        "peak_source": "nominal", "step_s": t_step, "algorithmic_flop_per_step": wl.stencil_flops_per_step(),
+        "bytes_through_memory": wl.stencil_bytes_per_step(), "hbm_peak": hbm, "hbm_peak_source": src, "note": on_chip}
     if t_gstep is not None:
         # plain HMC spends its time in exact gradients: forward with store and
-        # the adjoint passes, whose fields, temporaries and accumulators
-        # (20 fields, 172 MB at 64 chains) exceed the L2
-        g_ach = wl.gradient_bytes_per_step() / t_gstep / 1e9
-        roof = {"kernel": "fwi exact-gradient time step: velocity_tma_kernel + stress_tma_kernel (with store), then "
-                          "adj_velocity_tma_kernel<1, true> + adj_stress_tma_kernel<4>",
-                "bound": "hbm", "achieved": g_ach, "peak": hbm, "unit": "GB/s", "frac": g_ach / hbm,
-                "peak_source": src, "traffic": FWI_GRADIENT_STEP_DRAM_BYTES,
-                "traffic_source": "ncu captures of the forward, adjoint velocity and adjoint stress launches at "
-                                  "C = 64, default (cold) cache control",
-                "step_s": t_gstep, "algorithmic_bytes_per_step": wl.gradient_bytes_per_step(),
-                "l2_peak": l2, "frac_of_l2": g_ach / l2,
-                "note": "part of the working set stays in L2, so the algorithmic rate can exceed the HBM copy rate; "
-                        "DRAM traffic per step (cold cache) is 0.72 of the algorithmic bytes",
+        # the adjoint passes
+        g_ach = wl.gradient_flops_per_step() / t_gstep / 1e12
+        roof = {"kernel": "fwi exact-gradient time step: cluster_forward_kernel (with store), cluster_adjoint_kernel",
+                "bound": "fp32", "achieved": g_ach, "peak": fp32, "unit": "TFLOP/s", "frac": g_ach / fp32,
+                "peak_source": "nominal", "step_s": t_gstep,
+                "algorithmic_flop_per_step": wl.gradient_flops_per_step(),
+                "bytes_through_memory": wl.gradient_bytes_per_step(), "note": on_chip,
                 "forward_stencil": forward_roof}
     else:
         roof = forward_roof

@@ -778,10 +778,11 @@ class ElasticFullWaveform2D(_AbstractDistribution):
     single_dtype = "float32"
     # each shot is a CUDA graph of its own, replayed from the host
     graph_safe = False
-    # forward stencils read their neighbourhoods from shared-memory tiles
-    # staged by the tensor memory accelerator (chain counts that are a
-    # multiple of 32); False selects the direct-load kernels, which give the
-    # same records.  Set before the first evaluation.
+    # shots run with the wavefield on chip (a cluster of blocks per chain), or,
+    # on grids too wide or tall for that, with stencil neighbourhoods staged
+    # by the tensor memory accelerator (chain counts that are a multiple of
+    # 32); False selects the direct-load kernels, which give the same records.
+    # Set before the first evaluation.
     staged_tiles: bool = True
 
     def __init__(self, _input, ux_obs=None, uz_obs=None, temperature=None, omp_threads_override=None,
@@ -1011,8 +1012,8 @@ class ElasticFullWaveform2D(_AbstractDistribution):
             raise NotImplementedError("the elastic finite-difference kernels run in FP32 (float32 chains)")
 
     def check_device_status(self):
-        """The forward stencils stage their tiles through bounded barrier
-        waits; a wait that ran out sets the workspace's status word."""
+        """The stencils wait for tiles or for neighbouring blocks at bounded
+        barriers; a wait that ran out sets the workspace's status word."""
         from hmclab_gb300.Helpers.CustomExceptions import DeviceTimeoutError
 
         for key, ws in self.__dict__.get("_scratch_cache", {}).items():

@@ -31,8 +31,7 @@ optional Robbins-Monro step adaptation (`:1494-1522`), thinned samples
                 exp(-misfit / T_c) (the tempered posteriors that the
                 reference runs as separate distributions in parallel tempering)
   persistent    None (default): small dense linear-Gaussian targets (d <= 128)
-                run whole blocks of proposals in one persistent launch, one
-                warp per chain; False forces one launch per leapfrog step
+                run whole blocks of proposals in one persistent launch; False forces one launch per leapfrog step
   exchange_interval
                 after every proposal whose index is a multiple of this (the
                 first one included, as in the reference), the chains are

@@ -6,6 +6,10 @@
 // map_kernels_to_velocity), restated from Virieux (1986) / Levander (1988)
 // with a Cerjan et al. (1985) sponge.
 //
+// A shot runs with the wavefield on chip (fwi_cluster.cuh) wherever the grid
+// fits; the kernels of this file, one launch per half step, serve the others,
+// and everything around the time loops.
+//
 // Layout: every field is [nz][nx][C] (chain fastest), so each warp reads 32
 // chains of one cell in one 128-byte transaction and the stencil neighbours
 // of a block stay in L1/L2; one shot is simulated at a time so that the

@@ -1,9 +1,11 @@
 // General row-major matrix product on the CUDA cores:
 //   out[m][n] = alpha * A[m][k] B[k][n] + bias[m] + (accumulate ? out : 0).
 // Used for the FP64 verification path (dense LinearMatrix at d = 50, full mass
-// matrices, full-covariance Normal priors) and for small FP32 products.  The
-// FP32 production contraction of the dense LinearMatrix runs on the tensor
-// cores (dense_tc.cu).
+// matrices, full-covariance Normal priors) and for FP32 products (full mass
+// matrices, the elastic model's blob projections).  The FP32 production
+// contraction of the dense LinearMatrix runs on the tensor cores (dense_tc.cu).
+// gemm_kernel: FP64, any shape; gemv_kernel: FP64, few columns;
+// gemm_f32_kernel: FP32.
 #include "common.cuh"
 
 namespace hmc {

@@ -58,7 +58,8 @@ HMC_API const char* hmc_last_error(void);
 /* Number of kernels this library has launched since load (host-side counter). */
 HMC_API int64_t hmc_launch_count(void);
 /* Limits of the bounded waits of the kernels that stage operands through
- * tensor-copy barriers (tensor-core contractions, elastic stencils).  The
+ * tensor-copy barriers (tensor-core contractions, staged elastic stencils;
+ * withholding selects the latter over the on-chip shots).  The
  * default is 2 s with nothing withheld.  A test hook: with withhold = 1,
  * block 0 of every such launch skips its first barrier arrival, so its wait
  * runs out after wait_ns (1 us .. 2 s); the kernel then sets its status word
@@ -629,8 +630,11 @@ typedef struct hmc_fwi {
   float* t4;
   float* t5;
   double* partial;          /* [64][C] misfit partial sums (work)           */
-  int* status;              /* set to 1 when a tile load timed out (nullable:
-                               then the stencils read without staged tiles) */
+  int* status;              /* set to 1 when a tile load or a halo exchange
+                               timed out (nullable: then the per-step
+                               direct-load kernels run). The layout of
+                               `store` depends on the path: forward and
+                               adjoint of a shot need the same struct       */
   int32_t snapshot_interval; /* k: the adjoint correlates the forward and
                                adjoint fields at steps n = 0, k, 2k, ...
                                only, weighted by k (psvWave's
@@ -736,8 +740,7 @@ HMC_API int hmc_moments(int dtype, int64_t N, int64_t d, int64_t C,
  * One launch runs `proposals` whole HMC proposals (Samplers.py:1463-1584:
  * momentum draw, first drift, every kick and drift of the integrator, the
  * misfit at the end point, the FP64 accept test of :1471-1492 and the
- * thinned sample record) for every chain, one warp per chain, for the
- * posterior  [prior +] premultiplied dense LinearMatrix
+ * thinned sample record) for every chain, for the posterior  [prior +] premultiplied dense LinearMatrix
  * (LinearMatrix.py:164-208: gradient GtG m - Gtd0, misfit
  * 0.5 (m^T (GtG m - 2 Gtd0) + dtd)) with d <= 128, GtG held in shared
  * memory.  prior: 0 none, 1 Normal with diagonal inverse variances prior_w
