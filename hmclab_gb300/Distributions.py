@@ -151,6 +151,16 @@ class _AbstractDistribution:
     def _device_gradient(self, M, out, accumulate, dtype, stream):
         raise _AbstractMethodError()
 
+    def _row_prior(self, dtype):
+        """(kind, mean, weights) of a prior whose gradient is a function of each
+        element alone (kind 1 Normal, 2 Laplace), None for other targets."""
+        return None
+
+    def _gradient_with_prior(self, prior, M, out, dtype, stream):
+        """Write the sum of this target's gradient and a row prior's in one go;
+        False (and nothing written) where there is no such path."""
+        return False
+
     def _device_misfit_after_gradient(self, M, out, accumulate, dtype, stream):
         """The misfit at M, called right after _device_gradient at the same
         M (targets whose gradient runs a forward simulation reuse it)."""
@@ -306,6 +316,12 @@ class Normal(_AbstractDistribution):
             _lib.call("hmc_normal_full_gradient", _dev.dtype_code(dtype), d, C, M.data_ptr(), p["mean"].data_ptr(),
                       p["icov"].data_ptr(), work.data_ptr(), out.data_ptr(), int(accumulate), stream)
 
+    def _row_prior(self, dtype):
+        if not self.diagonal or type(self)._device_gradient is not Normal._device_gradient:
+            return None
+        p = self._params(dtype)
+        return 1, p["mean"], p["iv"]
+
     def normalize(self):
         cov = self.covariance
         if isinstance(cov, (float, int, _numpy.floating)):
@@ -362,6 +378,12 @@ class Laplace(_AbstractDistribution):
         p = self._params(dtype)
         _lib.call("hmc_laplace_gradient", _dev.dtype_code(dtype), M.shape[0], M.shape[1], M.data_ptr(),
                   p["mean"].data_ptr(), p["iw"].data_ptr(), out.data_ptr(), int(accumulate), stream)
+
+    def _row_prior(self, dtype):
+        if type(self)._device_gradient is not Laplace._device_gradient:
+            return None
+        p = self._params(dtype)
+        return 2, p["mean"], p["iw"]
 
     def normalize(self):
         self.normalization_constant = _numpy.log(
@@ -449,7 +471,15 @@ class AdditiveDistribution(_AbstractDistribution):
 
     @_fills_output
     def _device_gradient(self, M, out, accumulate, dtype, stream):
-        for k, dist in enumerate(self.separate_distributions):
+        parts = self.separate_distributions
+        done = 0
+        if not accumulate and len(parts) >= 2:
+            # a prior and a target that adds it in its own last pass, in either order
+            for prior, target in ((parts[0], parts[1]), (parts[1], parts[0])):
+                if target._gradient_with_prior(prior, M, out, dtype, stream):
+                    done = 2
+                    break
+        for k, dist in enumerate(parts[done:], done):
             dist._device_gradient(M, out, accumulate or k > 0, dtype, stream)
 
     def _fills(self, method):
@@ -663,6 +693,19 @@ class LinearMatrix(_AbstractDistribution):
                       p["col"].data_ptr(), p["val"].data_ptr(), p["trp"].data_ptr(), p["tcol"].data_ptr(),
                       p["tval"].data_ptr(), p["data"].data_ptr(), p["iv"].data_ptr(), resid.data_ptr(),
                       out.data_ptr(), int(accumulate), stream)
+
+    def _gradient_with_prior(self, prior, M, out, dtype, stream):
+        # (an unaligned M keeps the two passes: the four-chain product reads it in 16 bytes)
+        if (self.dense or self.premultiplication or dtype != "float32" or M.data_ptr() % 16
+                or type(self)._device_gradient is not LinearMatrix._device_gradient):
+            return False
+        row = prior._row_prior(dtype)
+        if row is None:
+            return False
+        C = M.shape[1]
+        resid = self._scratch("resid", (self.n_data, C), dtype, M.device)
+        self._csr_plan(C, M.device, stream).gradient_with_prior(M, resid, out, row, stream)
+        return True
 
     @staticmethod
     def create_default(dimensions: int, dtype=_numpy.dtype("float64")) -> "LinearMatrix":

@@ -153,6 +153,13 @@ class CsrSlabPlan:
                   self.data_c.data_ptr(), self.p["iv"].data_ptr(), resid.data_ptr(), out.data_ptr(), int(accumulate),
                   stream)
 
+    def gradient_with_prior(self, M, resid, out, prior, stream):
+        """out = the gradient of `prior` (kind, mean, weights) plus this one's."""
+        kind, mean, w = prior
+        _lib.call("hmc_csr_slab_gradient_prior", self._ref_g, self._ref_gt, self.C, M.data_ptr(), self.center.data_ptr(),
+                  self.data_c.data_ptr(), self.p["iv"].data_ptr(), kind, mean.data_ptr(), w.data_ptr(), resid.data_ptr(),
+                  out.data_ptr(), stream)
+
     def gradient(self, M, resid, out, accumulate, stream):
         _lib.call("hmc_csr_slab_gradient", self._ref_g, self._ref_gt, self.C, M.data_ptr(), self.center.data_ptr(),
                   self.data_c.data_ptr(), self.p["iv"].data_ptr(), resid.data_ptr(), out.data_ptr(), int(accumulate),

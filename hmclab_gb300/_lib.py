@@ -238,6 +238,7 @@ SIGNATURES = {
     "hmc_stream_capturing": [S, P],
     "hmc_csr_slab_misfit": [P, I64, P, P, P, P, P, P, I, S],
     "hmc_csr_slab_gradient": [P, P, I64, P, P, P, P, P, P, I, S],
+    "hmc_csr_slab_gradient_prior": [P, P, I64, P, P, P, P, I, P, P, P, P, S],
     "hmc_philox_normal": [I, I64, I64, c_uint64, c_uint64, c_uint32, P, S],
     "hmc_philox_raw": [I64, c_uint32, c_uint32, c_uint32, c_uint32, c_uint32, c_uint32, P, S],
     "hmc_begin_trajectory": [P, D, S],

@@ -353,12 +353,25 @@ __device__ __forceinline__ void csr_slab_centre(float* buf, const float* __restr
   }
 }
 
+// A prior's gradient that the product is added to, in place of what `out` holds:
+// the pass that writes it (prior_gradient_kernel, the same expressions) and the
+// read of it here were 9 of the 106 us of a tomography leapfrog step (4096 cells,
+// 1024 chains).  The product of weight and distance is rounded before it is
+// added, as it is there.
+struct CsrPrior {
+  int kind;  // PRIOR_NORMAL_DIAG + 1, PRIOR_LAPLACE + 1, or 0: none
+  const float *q, *mean, *w;
+  __device__ __forceinline__ float gradient(float x, int row) const {
+    return kind == PRIOR_NORMAL_DIAG + 1 ? -__fmul_rn(w[row], mean[row] - x) : sgn(x - mean[row]) * w[row];
+  }
+};
+
 template <int RPW, bool VEC4>
 __global__ void __launch_bounds__(CSR_THREADS, 2)
     csr_slab_kernel(int rows, int cols, int C, const int32_t* __restrict__ col, const float* __restrict__ val,
                     const int32_t* __restrict__ slab_ptr, int n_slabs, int slab, const float* __restrict__ X,
                     const float* __restrict__ center, const float* __restrict__ bias, const float* __restrict__ rs,
-                    float* out, int accumulate) {
+                    float* out, int accumulate, CsrPrior prior) {
   extern __shared__ __align__(16) float sx[];  // two buffers of [slab][32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = blockIdx.x * 32, c = c0 + lane;
@@ -411,7 +424,10 @@ __global__ void __launch_bounds__(CSR_THREADS, 2)
     if (bias) v -= bias[r];
     if (rs) v *= rs[r];
     const int64_t o = (int64_t)r * C + c;
-    out[o] = accumulate ? out[o] + v : v;
+    if (prior.kind)
+      out[o] = prior.gradient(prior.q[o], r) + v;
+    else
+      out[o] = accumulate ? out[o] + v : v;
   }
 }
 
@@ -429,7 +445,7 @@ template <int VEC>
 __global__ void csr_gather_kernel(int rows, int C, const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
                                   const float* __restrict__ val, const float* __restrict__ X,
                                   const float* __restrict__ center, const float* __restrict__ bias,
-                                  const float* __restrict__ rs, float* out, int accumulate) {
+                                  const float* __restrict__ rs, float* out, int accumulate, CsrPrior prior) {
   using V = typename std::conditional<VEC == 4, float4, float>::type;
   const int r = blockIdx.y;
   const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
@@ -472,33 +488,39 @@ __global__ void csr_gather_kernel(int rows, int C, const int32_t* __restrict__ r
   float* o = out + (int64_t)r * C + c;
   V ov;
   float* os = (float*)&ov;
-  if (accumulate) ov = *(const V*)o;
+  if (prior.kind) {
+    ov = *(const V*)(prior.q + (int64_t)r * C + c);
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) os[v] = prior.gradient(os[v], r);
+  } else if (accumulate) {
+    ov = *(const V*)o;
+  }
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
     float y = a[v];
     if (bias) y -= bb;
     if (rs) y *= ss;
-    os[v] = accumulate ? os[v] + y : y;
+    os[v] = accumulate || prior.kind ? os[v] + y : y;
   }
   *(V*)o = ov;
 }
 
 int csr_gather(const hmc_csr_slabs* A, int64_t C, const float* X, const float* center, const float* bias,
-               const float* rs, float* out, int accumulate, cudaStream_t st) {
+               const float* rs, float* out, int accumulate, const CsrPrior& prior, cudaStream_t st) {
   HMC_REQUIRE(A->rows <= 65535, "csr gather product: at most 65535 rows per launch");
   if (A->kernel == HMC_CSR_GATHER4) {
-    HMC_REQUIRE(C % 4 == 0 && ((uintptr_t)X & 15) == 0 && ((uintptr_t)out & 15) == 0,
+    HMC_REQUIRE(C % 4 == 0 && ((uintptr_t)X & 15) == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)prior.q & 15) == 0,
                 "csr gather product: four chains per thread need C % 4 == 0 and 16-byte aligned operands");
     const int64_t q = C / 4;
     const int threads = q >= 256 ? 256 : (q >= 128 ? 128 : (q >= 64 ? 64 : 32));
     const dim3 grid((unsigned)((q + threads - 1) / threads), (unsigned)A->rows);
     csr_gather_kernel<4><<<grid, threads, 0, st>>>((int)A->rows, (int)C, A->row_ptr, A->col, A->val, X, center, bias,
-                                                   rs, out, accumulate);
+                                                   rs, out, accumulate, prior);
   } else {
     const int threads = C >= 256 ? 256 : (C >= 128 ? 128 : (C >= 64 ? 64 : 32));
     const dim3 grid((unsigned)((C + threads - 1) / threads), (unsigned)A->rows);
     csr_gather_kernel<1><<<grid, threads, 0, st>>>((int)A->rows, (int)C, A->row_ptr, A->col, A->val, X, center, bias,
-                                                   rs, out, accumulate);
+                                                   rs, out, accumulate, prior);
   }
   return check_launch("csr_gather_kernel");
 }
@@ -524,7 +546,7 @@ int csr_slab_check(const hmc_csr_slabs* A, const char* who) {
 
 template <int RPW, bool VEC4>
 int csr_slab_launch(const hmc_csr_slabs* A, int64_t C, const float* X, const float* center, const float* bias,
-                    const float* rs, float* out, int accumulate, cudaStream_t st) {
+                    const float* rs, float* out, int accumulate, const CsrPrior& prior, cudaStream_t st) {
   const int smem = 2 * A->slab * 32 * (int)sizeof(float);  // double buffer
   static int attr_bytes = 0;  // per instantiation: the largest size enabled so far
   if (smem > 48 * 1024 && smem > attr_bytes) {
@@ -539,29 +561,29 @@ int csr_slab_launch(const hmc_csr_slabs* A, int64_t C, const float* X, const flo
   const dim3 grid((unsigned)((C + 31) / 32), (unsigned)groups);
   csr_slab_kernel<RPW, VEC4><<<grid, CSR_THREADS, smem, st>>>((int)A->rows, (int)A->cols, (int)C, A->col, A->val,
                                                               A->slab_ptr, n_slabs, A->slab, X, center, bias, rs,
-                                                              out, accumulate);
+                                                              out, accumulate, prior);
   return check_launch("csr_slab_kernel");
 }
 
 template <int RPW>
 int csr_slab_launch(const hmc_csr_slabs* A, int64_t C, const float* X, const float* center, const float* bias,
-                    const float* rs, float* out, int accumulate, cudaStream_t st) {
+                    const float* rs, float* out, int accumulate, const CsrPrior& prior, cudaStream_t st) {
   const bool vec4 = C % 4 == 0 && ((uintptr_t)X & 15) == 0;
-  return vec4 ? csr_slab_launch<RPW, true>(A, C, X, center, bias, rs, out, accumulate, st)
-              : csr_slab_launch<RPW, false>(A, C, X, center, bias, rs, out, accumulate, st);
+  return vec4 ? csr_slab_launch<RPW, true>(A, C, X, center, bias, rs, out, accumulate, prior, st)
+              : csr_slab_launch<RPW, false>(A, C, X, center, bias, rs, out, accumulate, prior, st);
 }
 
 int csr_slab(const hmc_csr_slabs* A, int64_t C, const float* X, const float* center, const float* bias,
-             const float* rs, float* out, int accumulate, cudaStream_t st) {
+             const float* rs, float* out, int accumulate, cudaStream_t st, const CsrPrior& prior = CsrPrior{}) {
   HMC_REQUIRE(C < (1ll << 31) && (C + 31) / 32 <= 0x7fffffff, "csr slab product: too many chains");
-  if (A->kernel != HMC_CSR_SLAB) return csr_gather(A, C, X, center, bias, rs, out, accumulate, st);
+  if (A->kernel != HMC_CSR_SLAB) return csr_gather(A, C, X, center, bias, rs, out, accumulate, prior, st);
   switch (A->rows_per_warp) {
     case 4:
-      return csr_slab_launch<4>(A, C, X, center, bias, rs, out, accumulate, st);
+      return csr_slab_launch<4>(A, C, X, center, bias, rs, out, accumulate, prior, st);
     case 8:
-      return csr_slab_launch<8>(A, C, X, center, bias, rs, out, accumulate, st);
+      return csr_slab_launch<8>(A, C, X, center, bias, rs, out, accumulate, prior, st);
     default:
-      return csr_slab_launch<16>(A, C, X, center, bias, rs, out, accumulate, st);
+      return csr_slab_launch<16>(A, C, X, center, bias, rs, out, accumulate, prior, st);
   }
 }
 
@@ -1081,6 +1103,24 @@ int hmc_csr_slab_gradient(const hmc_csr_slabs* G, const hmc_csr_slabs* Gt, int64
   cudaStream_t st = as_stream(stream);
   HMC_TRY(csr_slab(G, C, M, center, data, inv_var, resid, 0, st));
   return csr_slab(Gt, C, resid, nullptr, nullptr, nullptr, out_g, accumulate, st);
+}
+
+int hmc_csr_slab_gradient_prior(const hmc_csr_slabs* G, const hmc_csr_slabs* Gt, int64_t C, const float* M,
+                                const float* center, const float* data, const float* inv_var, int prior,
+                                const float* prior_mean, const float* prior_w, float* resid, float* out_g,
+                                void* stream) {
+  HMC_TRY(csr_slab_check(G, "hmc_csr_slab_gradient_prior"));
+  HMC_TRY(csr_slab_check(Gt, "hmc_csr_slab_gradient_prior"));
+  HMC_REQUIRE(Gt->rows == G->cols && Gt->cols == G->rows, "hmc_csr_slab_gradient_prior: G^T shape does not match G");
+  HMC_REQUIRE(C >= 0, "hmc_csr_slab_gradient_prior: bad sizes");
+  HMC_REQUIRE(prior == 1 || prior == 2, "hmc_csr_slab_gradient_prior: unknown prior kind %d", prior);
+  if (C == 0) return HMC_OK;
+  HMC_REQUIRE(M && data && inv_var && resid && out_g && prior_mean && prior_w && M != out_g,
+              "hmc_csr_slab_gradient_prior: null or aliased argument");
+  const CsrPrior p{prior == 1 ? PRIOR_NORMAL_DIAG + 1 : PRIOR_LAPLACE + 1, M, prior_mean, prior_w};
+  cudaStream_t st = as_stream(stream);
+  HMC_TRY(csr_slab(G, C, M, center, data, inv_var, resid, 0, st));
+  return csr_slab(Gt, C, resid, nullptr, nullptr, nullptr, out_g, 0, st, p);
 }
 
 int hmc_srcloc3d_misfit(int dtype, int64_t E, int64_t S, int64_t C, const void* M, const void* rx, const void* ry,

@@ -333,6 +333,15 @@ HMC_API int hmc_csr_slab_gradient(const hmc_csr_slabs* G, const hmc_csr_slabs* G
                                   const float* data, const float* inv_var,
                                   float* resid, float* out_g, int accumulate,
                                   void* stream);
+/* The gradient plus that of a prior at M (prior 1: Normal with inverse variances
+ * prior_w, 2: Laplace with inverse dispersions), written to out_g in the last
+ * pass: the sum of hmc_normal_diag_gradient or hmc_laplace_gradient and an
+ * accumulating hmc_csr_slab_gradient, bit for bit.                          */
+HMC_API int hmc_csr_slab_gradient_prior(
+    const hmc_csr_slabs* G, const hmc_csr_slabs* Gt, int64_t C, const float* M,
+    const float* center, const float* data, const float* inv_var, int prior,
+    const float* prior_mean, const float* prior_w, float* resid, float* out_g,
+    void* stream);
 
 /* SourceLocation.py:482-540 (SourceLocation3D, homogeneous velocity).
  * Parameters are interleaved [x,y,z,T] per event followed by v when
