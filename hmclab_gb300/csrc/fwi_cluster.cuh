@@ -61,6 +61,7 @@ struct ShotForward {
   int snap;                          // snapshot interval
   int nrec, n0, n1, load, save;
   uint64_t wait_ns;  // limit of a halo wait
+  int withhold;      // test hook: one thread of block 0 sends no halos
   int* status;
 };
 
@@ -76,6 +77,7 @@ struct ShotAdjoint {
   int snap, nrec, nt;
   float *g_bx, *g_bz, *g_l2m, *g_lam, *g_muxz;  // [cells][C], accumulated
   uint64_t wait_ns;
+  int withhold;
   int* status;
 };
 
@@ -120,9 +122,12 @@ __device__ __forceinline__ bool halo_try(const HaloBarriers& h, int k, uint32_t 
       : "memory");
   return ok != 0;
 }
-// Wait for the halos, at most limit_ns (2 s in production); on expiry the
-// status word is set and no later wait of this thread spins, so every block
-// still reaches the end of its loop and the final cluster barrier.
+// Wait for the halos, at most limit_ns (2 s in production) or until another
+// block has given up, which its neighbours' neighbours would otherwise notice
+// one limit after the other; on expiry the
+// status word is set, and from then on this thread neither waits, sends nor arms
+// a barrier (whose phase never completed), so every block still reaches the end of
+// its loop and the final cluster barrier.
 __device__ __forceinline__ void halo_wait(const HaloBarriers& h, int k, uint32_t parity, uint64_t limit_ns, int* status,
                                           bool& dead) {
   if (dead || halo_try(h, k, parity)) return;
@@ -130,12 +135,22 @@ __device__ __forceinline__ void halo_wait(const HaloBarriers& h, int k, uint32_t
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
   while (!halo_try(h, k, parity)) {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    if (t - t0 > limit_ns) {
+    if (t - t0 > limit_ns || *(volatile int*)status != 0) {
       atomicExch(status, 1);
       dead = true;
       return;
     }
   }
+}
+
+// After a wait that ran out, edge rows may still be on their way when their sender
+// reaches the end: 20 us, long past their arrival, before the last barrier.
+__device__ __forceinline__ void halo_drain(bool dead) {
+  if (!dead) return;
+  uint64_t t0, t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  do asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  while (t - t0 < 20000);
 }
 
 // Rows of shared memory (one float per column) of shared memory a block needs.

@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
   // then row 0 of t1 and t4, of t2, t3 and t5 (halos: t2 and t4 rows -1, RZ and
   // RZ + 1, t3 and t5 rows -2, -1 and RZ), then two buffers of stored vx (rows
   // -1 .. RZ + 1) and vz (rows -2 .. RZ).  t4 takes the rows of t1, which has
-  // no halo, once all threads have read it.
+  // no halo, once all threads have read it, and t1 those of t4 likewise.
   constexpr int TP = 5 * RZ;
   constexpr int T1 = 6 * RZ + 1, T4 = T1, T2 = T1 + RZ + 3, T3 = T2 + RZ + 4, T5 = T3 + RZ + 3, P0 = T5 + RZ + 1,
                 BUF = 2 * (RZ + 3);
@@ -124,10 +124,11 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
                  down_bar = remote_of(smem_of(&bars), has_down ? rank + 1 : rank);
   uint32_t parity = 0;
   bool dead = false;
+  const bool sends = column && !(g.withhold && blockIdx.x == 0 && i == 0);
   // edge rows of the operands a (rows -1, RZ, RZ + 1) and b (rows -2, -1, RZ) to
   // the neighbours; k numbers the barrier
 #define PUSH(k, a, b)                                                             \
-  if (column) {                                                                   \
+  if (sends && !dead) {                                                           \
     if (has_down) {                                                               \
       halo_push(down + ((a)-1) * PITCH * 4, ROW((a) + RZ - 1), down_bar + 8 * k); \
       halo_push(down + ((b)-2) * PITCH * 4, ROW((b) + RZ - 2), down_bar + 8 * k); \
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
   __syncthreads();                                         \
   if (bytes) { /* some neighbour */                        \
     halo_wait(bars, k, parity, g.wait_ns, g.status, dead); \
-    if (i == 0) halo_arm(bars, k, bytes);                  \
+    if (i == 0 && !dead) halo_arm(bars, k, bytes);         \
   }
 
   auto stresses = [&]() {
@@ -175,7 +176,6 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
     for (int z = 0; z < RZ; ++z)
       if (valid >> z & 1u) {
         const float l2m = ROW(2 * RZ + z), lam = ROW(3 * RZ + z);
-        ROW(T1 + z) = g.dt * (l2m * asxx[z] + lam * aszz[z]);
         ROW(T2 + z) = g.dt * (lam * asxx[z] + l2m * aszz[z]);
         ROW(T3 + z) = ROW(4 * RZ + z) * asxz[z];
       }
@@ -311,6 +311,12 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
     // ---- adjoint stresses
     stresses();
     PUSH(1, T2, T3)
+    __syncthreads();  // t4 has been read: its rows take t1
+    if (xin) {
+#pragma unroll
+      for (int z = 0; z < RZ; ++z)
+        if (valid >> z & 1u) ROW(T1 + z) = g.dt * (ROW(2 * RZ + z) * asxx[z] + ROW(3 * RZ + z) * aszz[z]);
+    }
     asm volatile("cp.async.wait_all;" ::: "memory");
     SETTLE(1)
     parity ^= 1;
@@ -328,6 +334,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
       g.g_bz[k] = gbz[z];
     }
   }
+  halo_drain(dead);
   cluster_barrier();  // no block leaves while a neighbour may push to it
 #undef SETTLE
 #undef PUSH

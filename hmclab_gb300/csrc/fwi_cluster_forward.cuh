@@ -83,11 +83,12 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
                  down_bar = remote_of(smem_of(&bars), has_down ? rank + 1 : rank);
   uint32_t parity = 0;
   bool dead = false;
+  const bool sends = column && !(g.withhold && blockIdx.x == 0 && i == 0);
 
   // Edge rows to the neighbours: fa is differentiated downwards (rows -2, -1,
   // RZ) and fb upwards (rows -1, RZ, RZ + 1); k numbers the barrier.
 #define PUSH(k, fa, fb, ha, hb)                                             \
-  if (column) {                                                             \
+  if (sends && !dead) {                                                     \
     if (has_down) {                                                         \
       halo_push(down + (ha) * PITCH * 4, fa[RZ - 2], down_bar + 8 * k);     \
       halo_push(down + (ha + 1) * PITCH * 4, fa[RZ - 1], down_bar + 8 * k); \
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
   __syncthreads();                                           \
   if (bytes) { /* some neighbour */                          \
     halo_wait(bars, k, parity, g.wait_ns, g.status, dead);   \
-    if (i == 0) halo_arm(bars, k, bytes);                    \
+    if (i == 0 && !dead) halo_arm(bars, k, bytes);           \
   }
 
   const int64_t cells = (int64_t)nx * nz;
@@ -252,6 +253,7 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
         g.sxz[k] = sxz[z];
       }
   }
+  halo_drain(dead);
   cluster_barrier();  // no block leaves while a neighbour may push to it
 #undef PUSH
 #undef PUBLISH

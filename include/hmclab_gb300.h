@@ -58,8 +58,9 @@ HMC_API const char* hmc_last_error(void);
 /* Number of kernels this library has launched since load (host-side counter). */
 HMC_API int64_t hmc_launch_count(void);
 /* Limits of the bounded waits of the kernels that stage operands through
- * tensor-copy barriers (tensor-core contractions, staged elastic stencils;
- * withholding selects the latter over the on-chip shots).  The
+ * tensor-copy barriers (tensor-core contractions, staged elastic stencils) and
+ * of the on-chip elastic shots, whose first block then sends no halos
+ * (withholding selects the staged stencils for multiples of 32 chains).  The
  * default is 2 s with nothing withheld.  A test hook: with withhold = 1,
  * block 0 of every such launch skips its first barrier arrival, so its wait
  * runs out after wait_ns (1 us .. 2 s); the kernel then sets its status word

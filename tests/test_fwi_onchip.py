@@ -82,6 +82,41 @@ def test_grids_that_do_not_fit_keep_the_stencil_kernels():
     _check(_config(40, 230, nt=20), 2)  # 246 rows
 
 
+@pytest.mark.gpu
+def test_repeated_gradients_are_equal():
+    """Blocks and warps drift against each other differently from run to run; what
+    they hand over in shared memory must not depend on it."""
+    cfg = _config(112, 60)
+    (chip, direct), M = _pair(cfg, 64)
+    g = direct.gradient_batch(M)
+    for _ in range(40):
+        assert bool((chip.gradient_batch(M) == g).all())
+    chip.check_device_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("C", [1, 5])
+def test_a_wait_that_runs_out_is_reported_and_the_context_survives(C):
+    """Under the wait-limit hook one thread of the first block sends no halos, so
+    its neighbours' waits run out after 1 ms; every block still ends."""
+    from hmclab_gb300 import _lib
+    from hmclab_gb300.Helpers.CustomExceptions import DeviceTimeoutError
+
+    cfg = _config(60, 50)
+    (chip, direct), M = _pair(cfg, C)
+    x, g = direct.misfit_batch(M), direct.gradient_batch(M)
+    for call in ("misfit_batch", "gradient_batch"):
+        hooked = H.Distributions.ElasticFullWaveform2D(chip)  # a copy captures its shots' graphs under the hook
+        with _lib.wait_limits(1_000_000, withhold=True):
+            getattr(hooked, call)(M)
+            x.cpu()
+        with pytest.raises(DeviceTimeoutError):
+            hooked.check_device_status()
+        del hooked
+    assert bool((chip.misfit_batch(M) == x).all()) and bool((chip.gradient_batch(M) == g).all())
+    chip.check_device_status()
+
+
 _QUOTIENT = r"""
 #include "quotient.cuh"
 #include <cstdint>
