@@ -1031,7 +1031,7 @@ static ShotAdjoint adjoint_args(const hmc_fwi* s) {
 // time step of 240 x 140 cells the staged
 // and direct-load kernels take 16.8 / 17.1 / 21.7 us (misfit) and 45 / 46 /
 // 82 us (misfit and gradient) for 1 / 16 / 64 chains, these 2.9 / 5.5 / 15.3 us
-// and 10 / 24 / 60 us; at 160 x 100 cells and 64 chains it is 11.8 and 37.9 us
+// and 10 / 24 / 62 us; at 160 x 100 cells and 64 chains it is 11.8 and 37.9 us
 // against 8.1 and 34.7 us, the narrowest margin of the grids tried.
 static int on_chip(const hmc_fwi* s, int store, bool* yes) {
   *yes = false;

@@ -155,7 +155,10 @@ __device__ __forceinline__ void halo_drain(bool dead) {
 
 // Rows of shared memory (one float per column) of shared memory a block needs.
 constexpr int forward_rows(int rz) { return 10 * rz + 12; }
-constexpr int adjoint_rows(int rz) { return 14 * rz + 24; }
+// (strips above 11 rows fit only if t4 shares the rows of t1, which takes two
+// more barriers of the block: 1.8 % of a single model's pass)
+constexpr bool adjoint_shares(int rz) { return rz > 11; }
+constexpr int adjoint_rows(int rz) { return adjoint_shares(rz) ? 14 * rz + 24 : 15 * rz + 25; }
 
 // Strip heights compiled.
 #define HMC_FORWARD_STRIPS(X) X(4) X(5) X(7) X(9) X(10) X(14)

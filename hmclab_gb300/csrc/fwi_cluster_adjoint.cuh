@@ -35,11 +35,13 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
   // shared memory, in rows of PITCH: thread-private parameters and the taper,
   // then row 0 of t1 and t4, of t2, t3 and t5 (halos: t2 and t4 rows -1, RZ and
   // RZ + 1, t3 and t5 rows -2, -1 and RZ), then two buffers of stored vx (rows
-  // -1 .. RZ + 1) and vz (rows -2 .. RZ).  t4 takes the rows of t1, which has
-  // no halo, once all threads have read it, and t1 those of t4 likewise.
+  // -1 .. RZ + 1) and vz (rows -2 .. RZ).  In the tallest strips t4 takes the
+  // rows of t1, which has no halo, once all threads have read it, and t1 those
+  // of t4 likewise.
+  constexpr bool SHARE = adjoint_shares(RZ);
   constexpr int TP = 5 * RZ;
-  constexpr int T1 = 6 * RZ + 1, T4 = T1, T2 = T1 + RZ + 3, T3 = T2 + RZ + 4, T5 = T3 + RZ + 3, P0 = T5 + RZ + 1,
-                BUF = 2 * (RZ + 3);
+  constexpr int T1 = 6 * RZ + 1, T4 = SHARE ? T1 : T1 + RZ + 1, T2 = T4 + RZ + 3, T3 = T2 + RZ + 4,
+                T5 = T3 + RZ + 3, P0 = T5 + RZ + 1, BUF = 2 * (RZ + 3);
   static_assert(P0 + 2 * BUF == adjoint_rows(RZ), "shared-memory rows");
   float* const my = smem + i;
 #define ROW(r) my[(r) * PITCH]
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
           }
       }
     }
-    __syncthreads();
+    if (SHARE) __syncthreads();  // t1 has been read: its rows take t4
     if (xin) {
 #pragma unroll
       for (int z = 0; z < RZ; ++z)
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
     // ---- adjoint stresses
     stresses();
     PUSH(1, T2, T3)
-    __syncthreads();  // t4 has been read: its rows take t1
+    if (SHARE) __syncthreads();  // t4 has been read: its rows take t1
     if (xin) {
 #pragma unroll
       for (int z = 0; z < RZ; ++z)
