@@ -4,9 +4,10 @@
 // matrices, full-covariance Normal priors) and for FP32 products (full mass
 // matrices, the elastic model's blob projections).  The FP32 production
 // contraction of the dense LinearMatrix runs on the tensor cores (dense_tc.cu).
-// gemm_kernel: FP64, any shape; gemv_kernel: FP64, few columns;
-// gemm_f32_kernel: FP32.
+// gemm_kernel: FP64, any shape, and FP32 rows too long for 32-bit offsets;
+// gemv_kernel: FP64, few columns; gemm_f32_kernel: FP32.
 #include "common.cuh"
+#include "gemm_shape.cuh"
 
 namespace hmc {
 namespace {
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(THREADS, 3)
   float ar[ALOADS], br[B16 ? 4 * BLOADS : BLOADS];
   constexpr int lstep = threads / KC;
   const int lr = threadIdx.x / KC, lk = threadIdx.x % KC;
-  uint32_t aoff[ALOADS];  // (launches keep a block's rows of A below 2^31 elements)
+  uint32_t aoff[ALOADS];  // (f32_offsets_fit)
 #pragma unroll
   for (int i = 0; i < ALOADS; ++i) {
     const int64_t r = lr + i * lstep, last = M - 1 - row0;
@@ -259,20 +260,23 @@ int gemm_f32(unsigned splits, int64_t m, int64_t n, int64_t k, float alpha, cons
              const void* bias, float bias_scale, const void* row_scale, void* out, int accumulate, int64_t k_chunk,
              void* partial, cudaStream_t st) {
   const bool b16 = n % 4 == 0 && ((uintptr_t)B & 15) == 0;
+  const bool few = n <= F32_FEW_COLUMNS;
+  const int rpt = few ? f32_offsets_fit(F32_FEW_ROWS, k) : f32_rows_per_thread(m, k);
+  if (rpt == 0) {
+    const dim3 tiles((unsigned)((n + BN - 1) / BN), (unsigned)((m + BM - 1) / BM), splits);
+    gemm_kernel<float><<<tiles, 256, 0, st>>>(m, n, k, alpha, (const float*)A, (const float*)B, (const float*)bias,
+                                              bias_scale, (const float*)row_scale, (float*)out, accumulate, k_chunk,
+                                              (float*)partial);
+    return check_launch("gemm_kernel");
+  }
   F32Kernel kern;
   int rows, columns, threads;
-  if (n <= 4) {
+  if (few) {
     // one model or a few chains: a thread per row, no columns of padding
     // (14000 x 60, one column: 11.2 us with 64-column tiles, 3.3 us)
     kern = f32_kernel<1, 1, 64>(b16);
-    rows = 64, columns = 4, threads = 64;
+    rows = F32_FEW_ROWS, columns = F32_FEW_COLUMNS, threads = 64;
   } else {
-    int rpt = 0;
-    int64_t least = 0;
-    for (int r : {9, 8, 6, 4, 2}) {
-      const int64_t padded = (m + 16 * r - 1) / (16 * r) * (16 * r);
-      if (rpt == 0 || padded < least) rpt = r, least = padded;
-    }
     kern = rpt == 9   ? f32_kernel<8, 9, 128>(b16)
            : rpt == 8 ? f32_kernel<8, 8, 128>(b16)
            : rpt == 6 ? f32_kernel<8, 6, 128>(b16)

@@ -1,0 +1,69 @@
+"""The rules that choose a product's kernel and blocks (csrc/gemm_shape.cuh),
+compiled for the host, and products at the sizes where they change."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import hmclab_gb300 as H
+from hmclab_gb300 import _lib
+
+_SOURCE = r"""
+#include "gemm_shape.cuh"
+extern "C" {
+int rows_per_thread(int64_t m, int64_t k) { return hmc::f32_rows_per_thread(m, k); }
+int few_columns_fit(int64_t k) { return hmc::f32_offsets_fit(hmc::F32_FEW_ROWS, k); }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("gemm_shape")
+    (d / "r.cpp").write_text(_SOURCE)
+    csrc = os.path.join(os.path.dirname(H.__file__), "csrc")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", csrc, str(d / "r.cpp"), "-o", str(d / "r.so")],
+                   check=True)
+    lib = ctypes.CDLL(str(d / "r.so"))
+    for f in (lib.rows_per_thread, lib.few_columns_fit):
+        f.argtypes = [ctypes.c_int64] * (2 if f is lib.rows_per_thread else 1)
+    return lib
+
+
+def _cuda():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch
+
+
+def test_offsets_of_a_block_stay_within_32_bits(rules):
+    """A block's offsets reach its rows times k; rows too long for that go to
+    the kernel with 64-bit offsets (0)."""
+    for k in (1, 600, 29_800_000, 29_826_162, 30_200_000, 33_600_000, 40_000_000, 134_000_000, 135_000_000, 2**33):
+        for m in (1, 33, 129, 144, 1000):
+            r = rules.rows_per_thread(m, k)
+            assert r in (0, 2, 4, 6, 8, 9) and 16 * r * k < 2**32, (m, k, r)
+            assert r > 0 or 32 * k >= 2**32 - 32
+        assert rules.few_columns_fit(k) == (64 * k < 2**32 - 64)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(144, 8, 30_200_000), (64, 2, 68_000_000), (31, 8, 139_000_000)])
+def test_long_rows(m, n, k):
+    """Rows whose offsets pass 2^32 (17 GB): one entry per row, so every product is
+    exact and an entry read from elsewhere shows."""
+    torch = _cuda()
+    A = torch.zeros((m, k), device="cuda")
+    B = torch.zeros((k, n), device="cuda")
+    rng = np.random.default_rng(k)
+    at = np.sort(rng.choice(k, size=m, replace=False))
+    A[torch.arange(m), torch.from_numpy(at)] = torch.arange(1.0, m + 1, device="cuda")
+    b = rng.integers(1, 100, size=(m, n)).astype(np.float32)
+    B[torch.from_numpy(at).cuda()] = torch.from_numpy(b).cuda()
+    out, work = torch.empty((m, n), device="cuda"), torch.empty(256 * m * n, device="cuda")
+    _lib.call("hmc_gemm_splitk", _lib.HMC_F32, m, n, k, 1.0, A.data_ptr(), B.data_ptr(), out.data_ptr(), 0, work.data_ptr(),
+              work.numel(), torch.cuda.current_stream().cuda_stream)
+    assert np.array_equal(out.cpu().numpy(), np.arange(1.0, m + 1)[:, None] * b)
