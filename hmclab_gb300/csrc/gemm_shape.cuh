@@ -10,15 +10,17 @@ namespace hmc {
 // Rows per thread of gemm_f32_kernel for more than four columns (a block owns
 // sixteen times as many), the choice with the least padding; 0: gemm_kernel, whose
 // offsets have 64 bits.  A block of gemm_f32_kernel keeps 32-bit offsets from its
-// first row of A, so its rows times k have to stay below 2^32.
+// first row of A, so its rows times k have to stay below 2^32; a grid has at most
+// 65535 blocks of rows.
 constexpr int F32_FEW_COLUMNS = 4, F32_FEW_ROWS = 64;  // up to four columns: 64 rows, a thread each
+constexpr int64_t GRID_ROWS = 65535;
 inline bool f32_offsets_fit(int64_t rows, int64_t k) { return k < (int64_t)0xffffffff / rows; }
 inline int f32_rows_per_thread(int64_t m, int64_t k) {
   int rpt = 0;
   int64_t least = 0;
   for (int r : {9, 8, 6, 4, 2}) {
-    if (!f32_offsets_fit(16 * r, k)) continue;
-    const int64_t padded = (m + 16 * r - 1) / (16 * r) * (16 * r);
+    const int64_t blocks = (m + 16 * r - 1) / (16 * r), padded = blocks * (16 * r);
+    if (!f32_offsets_fit(16 * r, k) || blocks > GRID_ROWS) continue;
     if (rpt == 0 || padded < least) rpt = r, least = padded;
   }
   return rpt;

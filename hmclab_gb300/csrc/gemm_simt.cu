@@ -285,7 +285,6 @@ int gemm_f32(unsigned splits, int64_t m, int64_t n, int64_t k, float alpha, cons
     rows = 16 * rpt, columns = 32, threads = 128;
   }
   const dim3 grid((unsigned)((n + columns - 1) / columns), (unsigned)((m + rows - 1) / rows), splits);
-  HMC_REQUIRE(grid.y <= 65535, "hmc_gemm: matrix too large");
   kern<<<grid, threads, 0, st>>>(m, n, k, alpha, (const float*)A, (const float*)B, (const float*)bias, bias_scale,
                                  (const float*)row_scale, (float*)out, accumulate, k_chunk, (float*)partial);
   return check_launch("gemm_f32_kernel");
@@ -350,7 +349,7 @@ int gemm_ex(int dtype, int64_t m, int64_t n, int64_t k, double alpha, const void
   HMC_REQUIRE(m >= 0 && n >= 0 && k >= 0, "hmc_gemm: negative size");
   if (m == 0 || n == 0) return HMC_OK;
   HMC_REQUIRE(A && B && out, "hmc_gemm: null operand");
-  HMC_REQUIRE((n + BN - 1) / BN <= 0x7FFFFFFF && (m + BM - 1) / BM <= 65535, "hmc_gemm: matrix too large");
+  HMC_REQUIRE((n + BN - 1) / BN <= 0x7FFFFFFF && (m + BM - 1) / BM <= GRID_ROWS, "hmc_gemm: matrix too large");
   const dim3 grid((unsigned)((n + BN - 1) / BN), (unsigned)((m + BM - 1) / BM));
   const int64_t kc = k > 0 ? k : 1;
   // FP64 products of up to one tile of columns that leave SMs without a tile
@@ -379,7 +378,7 @@ int gemm_splitk(int dtype, int64_t m, int64_t n, int64_t k, double alpha, const 
   HMC_REQUIRE(A && B && out && work, "hmc_gemm_splitk: null operand");
   HMC_REQUIRE(work_elems >= m * n, "hmc_gemm_splitk: work holds fewer than m * n elements");
   HMC_REQUIRE(dtype == HMC_F32 || dtype == HMC_F64, "hmc_gemm_splitk: unknown dtype %d", dtype);
-  HMC_REQUIRE((m + BM - 1) / BM <= 65535, "hmc_gemm_splitk: matrix too large");
+  HMC_REQUIRE((m + BM - 1) / BM <= GRID_ROWS, "hmc_gemm_splitk: matrix too large");
   const int64_t tiles = ((n + BN - 1) / BN) * ((m + BM - 1) / BM);
   // about four CTAs per SM in total, at least 256 k per split
   int64_t splits = (4 * 152 + tiles - 1) / tiles;

@@ -50,6 +50,41 @@ def test_offsets_of_a_block_stay_within_32_bits(rules):
         assert rules.few_columns_fit(k) == (64 * k < 2**32 - 64)
 
 
+TALL = 65535 * 64  # rows a product may have
+
+
+def test_tall_matrices_fit_the_grid(rules):
+    for m in (1, 2_097_120, 2_097_121, 2_097_153, 2_131_600, 3_000_000, 3_000_001, 4_194_177, TALL):
+        r = rules.rows_per_thread(m, 8)
+        assert r > 0 and -(-m // (16 * r)) <= 65535, (m, r)
+
+
+def test_tall_matrices_are_not_refused():
+    """Without a device the launch fails, but no size is refused before it."""
+    lib, one = _lib.load(), ctypes.c_void_p(16)
+    torch = pytest.importorskip("torch")
+    if torch.cuda.is_available():
+        pytest.skip("a device would run the products on these addresses")
+    for n in (1, 4, 5, 64):
+        for m in (2_097_153, 3_000_001, TALL):
+            assert lib.hmc_gemm(_lib.HMC_F32, m, n, 1, 1.0, one, one, None, one, 0, None) != _lib.HMC_ERR_INVALID_ARG
+        assert lib.hmc_gemm(_lib.HMC_F32, TALL + 1, n, 1, 1.0, one, one, None, one, 0, None) == _lib.HMC_ERR_INVALID_ARG
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n", [(2_097_153, 5), (3_000_001, 64), (TALL, 8), (TALL, 3)])
+def test_tall_matrices(m, n):
+    torch = _cuda()
+    k = 3
+    A = torch.from_numpy(np.random.default_rng(n).integers(-9, 9, size=(m, k)).astype(np.float32)).cuda()
+    B = torch.from_numpy(np.random.default_rng(k).integers(-9, 9, size=(k, n)).astype(np.float32)).cuda()
+    out = torch.full((m, n), float("nan"), device="cuda")
+    _lib.call("hmc_gemm", _lib.HMC_F32, m, n, k, 1.0, A.data_ptr(), B.data_ptr(), None, out.data_ptr(), 0,
+              torch.cuda.current_stream().cuda_stream)
+    want = sum(A[:, j:j + 1] * B[j:j + 1] for j in range(k))  # whole numbers: exact
+    assert torch.equal(out, want)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [(144, 8, 30_200_000), (64, 2, 68_000_000), (31, 8, 139_000_000)])
 def test_long_rows(m, n, k):
