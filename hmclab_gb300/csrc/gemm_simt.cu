@@ -261,7 +261,7 @@ int gemm_f32(unsigned splits, int64_t m, int64_t n, int64_t k, float alpha, cons
              void* partial, cudaStream_t st) {
   const bool b16 = n % 4 == 0 && ((uintptr_t)B & 15) == 0;
   const bool few = n <= F32_FEW_COLUMNS;
-  const int rpt = few ? f32_offsets_fit(F32_FEW_ROWS, k) : f32_rows_per_thread(m, k);
+  const int rpt = few ? f32_offsets_fit(F32_FEW_ROWS, k) : f32_rows_per_thread(m, n, k);
   if (rpt == 0) {
     const dim3 tiles((unsigned)((n + BN - 1) / BN), (unsigned)((m + BM - 1) / BM), splits);
     gemm_kernel<float><<<tiles, 256, 0, st>>>(m, n, k, alpha, (const float*)A, (const float*)B, (const float*)bias,

@@ -13,7 +13,7 @@ from hmclab_gb300 import _lib
 _SOURCE = r"""
 #include "gemm_shape.cuh"
 extern "C" {
-int rows_per_thread(int64_t m, int64_t k) { return hmc::f32_rows_per_thread(m, k); }
+int rows_per_thread(int64_t m, int64_t n, int64_t k) { return hmc::f32_rows_per_thread(m, n, k); }
 int few_columns_fit(int64_t k) { return hmc::f32_offsets_fit(hmc::F32_FEW_ROWS, k); }
 }
 """
@@ -28,7 +28,7 @@ def rules(tmp_path_factory):
                    check=True)
     lib = ctypes.CDLL(str(d / "r.so"))
     for f in (lib.rows_per_thread, lib.few_columns_fit):
-        f.argtypes = [ctypes.c_int64] * (2 if f is lib.rows_per_thread else 1)
+        f.argtypes = [ctypes.c_int64] * (3 if f is lib.rows_per_thread else 1)
     return lib
 
 
@@ -44,9 +44,10 @@ def test_offsets_of_a_block_stay_within_32_bits(rules):
     the kernel with 64-bit offsets (0)."""
     for k in (1, 600, 29_800_000, 29_826_162, 30_200_000, 33_600_000, 40_000_000, 134_000_000, 135_000_000, 2**33):
         for m in (1, 33, 129, 144, 1000):
-            r = rules.rows_per_thread(m, k)
-            assert r in (0, 2, 4, 6, 8, 9) and 16 * r * k < 2**32, (m, k, r)
-            assert r > 0 or 32 * k >= 2**32 - 32
+            for n in (5, 64, 8192):
+                r = rules.rows_per_thread(m, n, k)
+                assert r in (0, 2, 4, 6, 8, 9) and 16 * r * k < 2**32, (m, n, k, r)
+                assert r > 0 or 32 * k >= 2**32 - 32
         assert rules.few_columns_fit(k) == (64 * k < 2**32 - 64)
 
 
@@ -55,8 +56,18 @@ TALL = 65535 * 64  # rows a product may have
 
 def test_tall_matrices_fit_the_grid(rules):
     for m in (1, 2_097_120, 2_097_121, 2_097_153, 2_131_600, 3_000_000, 3_000_001, 4_194_177, TALL):
-        r = rules.rows_per_thread(m, 8)
-        assert r > 0 and -(-m // (16 * r)) <= 65535, (m, r)
+        for n in (5, 64, 8192):
+            r = rules.rows_per_thread(m, n, 8)
+            assert r > 0 and -(-m // (16 * r)) <= 65535, (m, n, r)
+
+
+def test_two_rows_per_thread_where_blocks_are_missing(rules):
+    """Padding alone took two rows per thread for each of these; where the chip is
+    full that was slower than the tiles the kernel replaced."""
+    for m, n, want in ((20_000, 1024, 4), (100_000, 1024, 4), (4000, 8192, 4), (2080, 8192, 9), (2080, 200, 2), (200, 8192, 2),
+                       (20_000, 8, 9), (33, 64, 4), (129, 8192, 9), (160, 64, 2)):
+        r = rules.rows_per_thread(m, n, 60)
+        assert (r == 2) == (want == 2), (m, n, r)
 
 
 def test_tall_matrices_are_not_refused():
