@@ -34,4 +34,23 @@ inline int f32_rows_per_thread(int64_t m, int64_t n, int64_t k) {
   return rpt;
 }
 
+// FP64 products of up to 64 columns and 9664 rows (a tile of 64 x 64 for each SM at
+// most): gemv_kernel (true) or gemm_kernel.  Both are bound by FP64 lanes.  A tile
+// costs its SM 64 x 64 of them for each k, however few columns are real; the row
+// kernel, over all SMs, one for each product of groups of eight columns, and for
+// each such group of a row 5 x 8 adds of 32 lanes that sum over the warp.  Its factors were
+// measured over 1000 .. 9700 rows, 5 .. 64 columns, k of 16 .. 4000: 1.2, and 1.7 where
+// the rows of B are whole 128-byte lines and B exceeds an SM's L1 (a warp's loads
+// of a column, one per row of B, then fall into few of its sets).  9000 rows, k = 60:
+// 32 columns 137 us by rows and 76 us in tiles, 8 columns 37 and 76; 9000 x 1000, 64
+// columns 1901 and 1203; 1000 x 1000, 64 columns 241 and 1134.  Up to four columns
+// the row kernel was faster at every size.
+inline bool f64_by_rows(int64_t m, int64_t n, int64_t k) {
+  if (n > 64 || (m + 63) / 64 >= 152) return false;
+  if (n <= 4) return true;
+  const double factor = n % 16 == 0 && n * k > 16384 ? 1.7 : 1.2;
+  const double lanes = factor * (double)m * (double)((n + 7) / 8 * 8) * 32.0 * (double)((k + 31) / 32 + 5);
+  return lanes <= 152.0 * 64.0 * 64.0 * (double)((k + 15) / 16 * 16);
+}
+
 }  // namespace hmc

@@ -352,9 +352,8 @@ int gemm_ex(int dtype, int64_t m, int64_t n, int64_t k, double alpha, const void
   HMC_REQUIRE((n + BN - 1) / BN <= 0x7FFFFFFF && (m + BM - 1) / BM <= GRID_ROWS, "hmc_gemm: matrix too large");
   const dim3 grid((unsigned)((n + BN - 1) / BN), (unsigned)((m + BM - 1) / BM));
   const int64_t kc = k > 0 ? k : 1;
-  // FP64 products of up to one tile of columns that leave SMs without a tile
-  // go to the row kernel (FP64 only: FP32 sums keep their order in k)
-  if (dtype == HMC_F64 && n <= BN && grid.y < 152) {
+  // (FP64 only: FP32 sums keep their order in k)
+  if (dtype == HMC_F64 && f64_by_rows(m, n, k)) {
     if (n == 1) return gemv<double, 1>(m, n, k, alpha, A, B, bias, bias_scale, row_scale, out, accumulate, stream);
     if (n <= 4) return gemv<double, 4>(m, n, k, alpha, A, B, bias, bias_scale, row_scale, out, accumulate, stream);
     return gemv<double, 8>(m, n, k, alpha, A, B, bias, bias_scale, row_scale, out, accumulate, stream);

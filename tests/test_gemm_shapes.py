@@ -14,6 +14,7 @@ _SOURCE = r"""
 #include "gemm_shape.cuh"
 extern "C" {
 int rows_per_thread(int64_t m, int64_t n, int64_t k) { return hmc::f32_rows_per_thread(m, n, k); }
+int by_rows(int64_t m, int64_t n, int64_t k) { return hmc::f64_by_rows(m, n, k); }
 int few_columns_fit(int64_t k) { return hmc::f32_offsets_fit(hmc::F32_FEW_ROWS, k); }
 }
 """
@@ -27,8 +28,8 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", csrc, str(d / "r.cpp"), "-o", str(d / "r.so")],
                    check=True)
     lib = ctypes.CDLL(str(d / "r.so"))
-    for f in (lib.rows_per_thread, lib.few_columns_fit):
-        f.argtypes = [ctypes.c_int64] * (3 if f is lib.rows_per_thread else 1)
+    for f, args in ((lib.rows_per_thread, 3), (lib.by_rows, 3), (lib.few_columns_fit, 1)):
+        f.argtypes = [ctypes.c_int64] * args
     return lib
 
 
@@ -68,6 +69,16 @@ def test_two_rows_per_thread_where_blocks_are_missing(rules):
                        (20_000, 8, 9), (33, 64, 4), (129, 8192, 9), (160, 64, 2)):
         r = rules.rows_per_thread(m, n, 60)
         assert (r == 2) == (want == 2), (m, n, r)
+
+
+def test_fp64_rows_only_where_the_tiles_are_slower(rules):
+    """(m, n, k) on either side of the line, by the kernel that was faster."""
+    for m, n, k in ((50, 64, 50), (1000, 1, 1000), (1000, 64, 1000), (9000, 8, 60), (9000, 32, 1000), (4000, 64, 4000),
+                    (9664, 4, 16), (7500, 56, 1600), (6000, 32, 200)):
+        assert rules.by_rows(m, n, k), (m, n, k)
+    for m, n, k in ((9000, 48, 1000), (9000, 64, 1000), (9000, 32, 60), (9000, 64, 200), (7500, 64, 16), (6000, 64, 4000),
+                    (9665, 1, 1000), (50, 65, 50)):
+        assert not rules.by_rows(m, n, k), (m, n, k)
 
 
 def test_tall_matrices_are_not_refused():
@@ -113,3 +124,18 @@ def test_long_rows(m, n, k):
     _lib.call("hmc_gemm_splitk", _lib.HMC_F32, m, n, k, 1.0, A.data_ptr(), B.data_ptr(), out.data_ptr(), 0, work.data_ptr(),
               work.numel(), torch.cuda.current_stream().cuda_stream)
     assert np.array_equal(out.cpu().numpy(), np.arange(1.0, m + 1)[:, None] * b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(9000, 32, 60), (7500, 64, 16), (9000, 48, 1000), (6000, 56, 200)])
+def test_fp64_product_on_either_side_of_the_line(m, n, k):
+    torch = _cuda()
+    rng = np.random.default_rng(m + n + k)
+    A, B, bias = rng.normal(size=(m, k)), rng.normal(size=(k, n)), rng.normal(size=m)
+    tA, tB, tb = (torch.from_numpy(a).cuda() for a in (A, B, bias))
+    out = torch.full((m, n), float("nan"), dtype=torch.float64, device="cuda")
+    _lib.call("hmc_gemm", _lib.HMC_F64, m, n, k, 1.5, tA.data_ptr(), tB.data_ptr(), tb.data_ptr(), out.data_ptr(), 0,
+              torch.cuda.current_stream().cuda_stream)
+    # k products and a sum of them: k ulp of the sum of their sizes
+    bound = 2.3e-16 * (k + 4) * (1.5 * np.abs(A) @ np.abs(B) + np.abs(bias)[:, None])
+    assert np.all(np.abs(out.cpu().numpy() - (1.5 * A @ B + bias[:, None])) <= bound)
