@@ -26,6 +26,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "halo_exit.cuh"
 
 namespace hmc {
 namespace fwi {
@@ -143,17 +144,17 @@ __device__ __forceinline__ void halo_wait(const HaloBarriers& h, int k, uint32_t
   }
 }
 
-// After a wait that ran out, edge rows may still be on their way when their sender
-// reaches the end: 20 us, long past their arrival, before the last barrier.
-__device__ __forceinline__ void halo_drain(bool dead) {
-  if (!dead) return;
+// At the end of a launch: edge rows of a launch with a wait that ran out arrive
+// before any block leaves.
+__device__ __forceinline__ void halo_drain(bool dead, const int* status) {
+  if (!halo_must_drain(dead, *(const volatile int*)status)) return;
   uint64_t t0, t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
   do asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  while (t - t0 < 20000);
+  while (t - t0 < HALO_DRAIN_NS);
 }
 
-// Rows of shared memory (one float per column) of shared memory a block needs.
+// Rows of shared memory (one float per column) a block needs.
 constexpr int forward_rows(int rz) { return 10 * rz + 12; }
 // (strips above 11 rows fit only if t4 shares the rows of t1, which takes two
 // more barriers of the block: 1.8 % of a single model's pass)

@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
       g.g_bz[k] = gbz[z];
     }
   }
-  halo_drain(dead);
+  halo_drain(dead, g.status);
   cluster_barrier();  // no block leaves while a neighbour may push to it
 #undef SETTLE
 #undef PUSH

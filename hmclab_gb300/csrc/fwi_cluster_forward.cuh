@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
         g.sxz[k] = sxz[z];
       }
   }
-  halo_drain(dead);
+  halo_drain(dead, g.status);
   cluster_barrier();  // no block leaves while a neighbour may push to it
 #undef PUSH
 #undef PUBLISH
