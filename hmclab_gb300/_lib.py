@@ -292,6 +292,7 @@ SIGNATURES = {
     "hmc_pot_weighted_colsum": [I64, I64, P, I64, P, P, S],
     "hmc_pot_scale_columns": [I64, I64, P, I64, P, P, I64, S],
     "hmc_fwi_prepare": [P, S],
+    "hmc_fwi_strips": [P, I, P, P],
     "hmc_fwi_forward_shot": [P, I, I, I, I, S],
     "hmc_fwi_forward_shot_sources": [P, I, P, I, I, S],
     "hmc_fill_zero": [P, I64, S],

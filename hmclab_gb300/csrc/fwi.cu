@@ -948,19 +948,19 @@ static StoreSlot store_slot(const hmc_fwi* s, int n) {
   return {base, base + 2 * cells, 4ll * (n / k) * s->nz};
 }
 
-static int cluster_forward(const ShotForward& a, const Waves& w, bool dry, bool* ran, cudaStream_t st) {
-  *ran = false;
+static int cluster_forward(const ShotForward& a, const Waves& w, bool dry, int* rows, cudaStream_t st) {
+  *rows = 0;
   if (a.nx > CLUSTER_COLUMNS || a.C > 0x7FFFFFFF / CLUSTER_MAX) return HMC_OK;
-  return a.nx <= 128   ? cluster_forward_at<128>(a, w, dry, ran, st)
-         : a.nx <= 192 ? cluster_forward_at<192>(a, w, dry, ran, st)
-                       : cluster_forward_at<256>(a, w, dry, ran, st);
+  return a.nx <= 128   ? cluster_forward_at<128>(a, w, dry, rows, st)
+         : a.nx <= 192 ? cluster_forward_at<192>(a, w, dry, rows, st)
+                       : cluster_forward_at<256>(a, w, dry, rows, st);
 }
-static int cluster_adjoint(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st) {
-  *ran = false;
+static int cluster_adjoint(const ShotAdjoint& a, bool dry, int* rows, cudaStream_t st) {
+  *rows = 0;
   if (a.nx > CLUSTER_COLUMNS || a.C > 0x7FFFFFFF / CLUSTER_MAX) return HMC_OK;
-  return a.nx <= 128   ? cluster_adjoint_at<128>(a, dry, ran, st)
-         : a.nx <= 192 ? cluster_adjoint_at<192>(a, dry, ran, st)
-                       : cluster_adjoint_at<256>(a, dry, ran, st);
+  return a.nx <= 128   ? cluster_adjoint_at<128>(a, dry, rows, st)
+         : a.nx <= 192 ? cluster_adjoint_at<192>(a, dry, rows, st)
+                       : cluster_adjoint_at<256>(a, dry, rows, st);
 }
 static ShotForward forward_args(const hmc_fwi* s, int shot, int store) {
   ShotForward a = {};
@@ -1033,16 +1033,25 @@ static ShotAdjoint adjoint_args(const hmc_fwi* s) {
 // 82 us (misfit and gradient) for 1 / 16 / 64 chains, these 2.9 / 5.5 / 15.3 us
 // and 10 / 24 / 62 us; at 160 x 100 cells and 64 chains it is 11.8 and 37.9 us
 // against 8.1 and 34.7 us, the narrowest margin of the grids tried.
-static int on_chip(const hmc_fwi* s, int store, bool* yes) {
-  *yes = false;
+// Strip heights of the shot's passes, 0 where the per-step kernels run.
+static int on_chip(const hmc_fwi* s, int store, int* forward, int* adjoint) {
+  *forward = *adjoint = 0;
   if (!s->status || (wait_limits().withhold && s->chains % 32 == 0)) return HMC_OK;
   static const Waves none = {};
-  HMC_TRY(cluster_forward(forward_args(s, 0, store), none, true, yes, nullptr));
-  if (*yes && store) HMC_TRY(cluster_adjoint(adjoint_args(s), true, yes, nullptr));
+  HMC_TRY(cluster_forward(forward_args(s, 0, store), none, true, forward, nullptr));
+  if (!store || *forward == 0) return HMC_OK;
+  HMC_TRY(cluster_adjoint(adjoint_args(s), true, adjoint, nullptr));
+  if (*adjoint == 0) *forward = 0;
   return HMC_OK;
 }
 
 extern "C" {
+
+HMC_API int hmc_fwi_strips(const hmc_fwi* s, int store, int* forward, int* adjoint) {
+  HMC_TRY(check_fwi(s, "hmc_fwi_strips"));
+  HMC_REQUIRE(forward && adjoint, "hmc_fwi_strips: null output");
+  return on_chip(s, store, forward, adjoint);
+}
 
 HMC_API int hmc_fwi_prepare(const hmc_fwi* s, void* stream) {
   HMC_TRY(check_fwi(s, "hmc_fwi_prepare"));
@@ -1106,9 +1115,9 @@ HMC_API int hmc_fwi_forward_shot_sources(const hmc_fwi* s, int shot, const hmc_f
     return ss;
   };
   cudaStream_t st = as_stream(stream);
-  bool chip = false;
-  if (n_src <= WAVE_SAMPLES) HMC_TRY(on_chip(s, store, &chip));
-  if (chip) {
+  int strip = 0, adjoint_strip = 0;
+  if (n_src <= WAVE_SAMPLES) HMC_TRY(on_chip(s, store, &strip, &adjoint_strip));
+  if (strip) {
     ShotForward a = forward_args(s, shot, store);
     Waves w = {};
     auto term = [&](int q, int i, int j, float xx, float zz, float xz) {
@@ -1142,9 +1151,8 @@ HMC_API int hmc_fwi_forward_shot_sources(const hmc_fwi* s, int shot, const hmc_f
       for (int t = 0; t < w.n_terms; ++t) w.first[t] = sources.first[t] * steps;
       for (int q = 0; q < n_src; ++q)
         for (int n = 0; n < steps; ++n) w.s[q * steps + n] = src[q].stf_host[n0 + n] * src_scale;
-      bool ran = false;
-      HMC_TRY(cluster_forward(a, w, false, &ran, st));
-      HMC_REQUIRE(ran, "hmc_fwi_forward_shot_sources: no strip height fits");
+      HMC_TRY(cluster_forward(a, w, false, &strip, st));
+      HMC_REQUIRE(strip, "hmc_fwi_forward_shot_sources: no strip height fits");
     }
     return HMC_OK;
   }
@@ -1225,9 +1233,9 @@ HMC_API int hmc_fwi_adjoint_shot(const hmc_fwi* s, int shot, void* stream) {
   residual_kernel<<<grid_for(rows * s->chains), 256, 0, st>>>(rows, s->chains, s->rec + shot_off * s->chains,
                                                               s->obs + shot_off, s->w, s->resid);
   HMC_TRY(check_launch("residual_kernel"));
-  bool chip = false;
-  HMC_TRY(on_chip(s, 1, &chip));
-  if (chip) return cluster_adjoint(adjoint_args(s), false, &chip, st);
+  int forward_strip = 0, strip = 0;
+  HMC_TRY(on_chip(s, 1, &forward_strip, &strip));
+  if (strip) return cluster_adjoint(adjoint_args(s), false, &strip, st);
   const Grid g = grid_of(s);
   const int64_t cells = (int64_t)s->nx * s->nz * s->chains;
   const size_t fb = (size_t)cells * sizeof(float);

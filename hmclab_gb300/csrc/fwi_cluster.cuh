@@ -165,17 +165,17 @@ constexpr int adjoint_rows(int rz) { return adjoint_shares(rz) ? 14 * rz + 24 : 
 #define HMC_FORWARD_STRIPS(X) X(4) X(5) X(7) X(9) X(10) X(14)
 #define HMC_ADJOINT_STRIPS(X) X(4) X(5) X(7) X(9) X(11) X(14)
 
-// Launch one shot; false when no strip height fits (the caller then runs the
-// per-step kernels).  dry: only tell whether it would run.  The pitch of a row
+// Launch one shot; *rows is the strip height, 0 when none fits (the caller then
+// runs the per-step kernels).  dry: only tell the height.  The pitch of a row
 // in shared memory is a constant, so that offsets are immediates; a narrow grid
 // takes a narrow one, which lets several blocks share an SM: 64 chains of 100 x
 // 70 cells take 21.4 us per step of misfit and gradient with 256 columns and 15.0
 // with 128 (compiled in fwi_cluster_128.cu, fwi_cluster_192.cu and
 // fwi_cluster_256.cu).
 template <int PITCH>
-int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, bool* ran, cudaStream_t st);
+int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, int* rows, cudaStream_t st);
 template <int PITCH>
-int cluster_adjoint_at(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st);
+int cluster_adjoint_at(const ShotAdjoint& a, bool dry, int* rows, cudaStream_t st);
 
 // The strip height for C chains: the cheapest number of waves of resident
 // clusters, a step of a wave costing its rows' instructions (those of all

@@ -345,16 +345,15 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
 #undef HMC_DP
 
 template <int PITCH>
-int cluster_adjoint_at(const ShotAdjoint& a, bool dry, bool* ran, cudaStream_t st) {
-  *ran = false;
+int cluster_adjoint_at(const ShotAdjoint& a, bool dry, int* rows, cudaStream_t st) {
+  *rows = 0;
   ClusterChoice best;
 #define HMC_STRIP(RZ) \
   consider_strip(best, cluster_adjoint_kernel<RZ, PITCH>, RZ, adjoint_rows(RZ) * PITCH, a.nx, a.nz, a.C, 210.0);
   HMC_ADJOINT_STRIPS(HMC_STRIP)
 #undef HMC_STRIP
-  if (best.rz == 0) return HMC_OK;
-  *ran = true;
-  if (dry) return HMC_OK;
+  *rows = best.rz;
+  if (dry || best.rz == 0) return HMC_OK;
   ShotAdjoint g = a;
   g.R = best.R;
   switch (best.rz) {

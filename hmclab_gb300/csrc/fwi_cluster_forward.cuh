@@ -262,16 +262,15 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
 #undef HMC_DP
 
 template <int PITCH>
-int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, bool* ran, cudaStream_t st) {
-  *ran = false;
+int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, int* rows, cudaStream_t st) {
+  *rows = 0;
   ClusterChoice best;
 #define HMC_STRIP(RZ) \
   consider_strip(best, cluster_forward_kernel<RZ, PITCH>, RZ, forward_rows(RZ) * PITCH, a.nx, a.nz, a.C, 75.0);
   HMC_FORWARD_STRIPS(HMC_STRIP)
 #undef HMC_STRIP
-  if (best.rz == 0) return HMC_OK;
-  *ran = true;
-  if (dry) return HMC_OK;
+  *rows = best.rz;
+  if (dry || best.rz == 0) return HMC_OK;
   ShotForward g = a;
   g.R = best.R;
   switch (best.rz) {

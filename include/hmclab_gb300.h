@@ -654,6 +654,11 @@ typedef struct hmc_fwi {
 
 /* rho, vp, vs -> buoyancies and moduli on the staggered grid.               */
 HMC_API int hmc_fwi_prepare(const hmc_fwi* s, void* stream);
+/* How shots of this descriptor run: the rows of the grid that a block of a
+ * chain's cluster owns in the forward pass and (with store) in the adjoint, both 0
+ * where the per-step kernels run.                                           */
+HMC_API int hmc_fwi_strips(const hmc_fwi* s, int store, int* forward,
+                           int* adjoint);
 /* One shot with an explosive source at (src_x, src_z) and the wavelet
  * stf_host; records into rec[shot]; stores the velocities of every step when
  * store != 0.  (psvWave fdModel.forward_simulate, called at
