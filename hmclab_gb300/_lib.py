@@ -385,7 +385,8 @@ class wait_limits:
     """Context manager around hmc_set_wait_limits (a test hook): inside it,
     bounded device waits give up after `wait_ns`, and with `withhold` block 0
     of every launch that stages tiles through tensor-copy barriers skips its
-    arrival, so its wait runs out and the kernel reports a time-out.  The
+    arrival, and a thread of block 0 of an on-chip elastic shot sends no edge
+    rows, so a wait runs out and the kernel reports a time-out.  The
     production limits (2 s, nothing withheld) are restored on exit."""
 
     DEFAULT_NS = 2_000_000_000

@@ -1025,9 +1025,8 @@ static ShotAdjoint adjoint_args(const hmc_fwi* s) {
 // Whether a shot runs with the wavefield on chip (fwi_cluster.cuh): grids of up
 // to 256 columns whose strips fit a cluster.  A stored wavefield has another
 // layout there ([chain][plane] instead of [plane][chain]), so the forward pass
-// that stores it and the adjoint that reads it decide together.  A null status
-// word keeps the direct-load kernels, and the wait-limit test hook the staged
-// ones for multiples of 32 chains, so that their waits can be tested too.  Per
+// that stores it and the adjoint that reads it decide together, from the descriptor
+// alone.  A null status word keeps the direct-load kernels.  Per
 // time step of 240 x 140 cells the staged
 // and direct-load kernels take 16.8 / 17.1 / 21.7 us (misfit) and 45 / 46 /
 // 82 us (misfit and gradient) for 1 / 16 / 64 chains, these 2.9 / 5.5 / 15.3 us
@@ -1036,7 +1035,7 @@ static ShotAdjoint adjoint_args(const hmc_fwi* s) {
 // Strip heights of the shot's passes, 0 where the per-step kernels run.
 static int on_chip(const hmc_fwi* s, int store, int* forward, int* adjoint) {
   *forward = *adjoint = 0;
-  if (!s->status || (wait_limits().withhold && s->chains % 32 == 0)) return HMC_OK;
+  if (!s->status) return HMC_OK;
   static const Waves none = {};
   HMC_TRY(cluster_forward(forward_args(s, 0, store), none, true, forward, nullptr));
   if (!store || *forward == 0) return HMC_OK;

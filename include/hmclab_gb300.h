@@ -59,11 +59,11 @@ HMC_API const char* hmc_last_error(void);
 HMC_API int64_t hmc_launch_count(void);
 /* Limits of the bounded waits of the kernels that stage operands through
  * tensor-copy barriers (tensor-core contractions, staged elastic stencils) and
- * of the on-chip elastic shots, whose first block then sends no halos
- * (withholding selects the staged stencils for multiples of 32 chains).  The
- * default is 2 s with nothing withheld.  A test hook: with withhold = 1,
- * block 0 of every such launch skips its first barrier arrival, so its wait
- * runs out after wait_ns (1 us .. 2 s); the kernel then sets its status word
+ * of the on-chip elastic shots.  The default is 2 s with nothing withheld.  A
+ * test hook: with withhold = 1, block 0 of every such launch skips its first
+ * barrier arrival (on chip, a thread of block 0 sends no edge rows), so its or
+ * its neighbour's wait runs out after wait_ns (1 us .. 2 s); which kernels run
+ * does not change.  The kernel then sets its status word
  * (HMC_ERR_TIMEOUT, or 1 for the stencils), frees what it holds and returns.
  * Launches captured in a CUDA graph keep the limits of their capture.
  * Reference counterpart: none (the reference has no device code); it stands
