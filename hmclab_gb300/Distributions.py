@@ -45,9 +45,16 @@ def _column(coordinates, dimensions):
 def _fills_output(method):
     """Mark a `_device_misfit` / `_device_gradient` that writes every element of
     `out` when it does not accumulate, so that callers need not clear it first.
-    An override in a subclass is a function of its own, without the mark."""
+    An override, in a subclass or on an object, is a function of its own, without
+    the mark."""
     method.fills_output = True
     return method
+
+
+def _keeps(target, cls, method):
+    """Whether `target` has `cls`'s own `method`: overridden neither in a subclass
+    nor on the object."""
+    return getattr(getattr(target, method), "__func__", None) is getattr(cls, method)
 
 
 class _AbstractDistribution:
@@ -116,7 +123,7 @@ class _AbstractDistribution:
         return _dev.normalise_dtype(M.dtype)
 
     def _fills(self, method):
-        return getattr(getattr(type(self), method), "fills_output", False)
+        return getattr(getattr(self, method), "fills_output", False)
 
     def _new_output(self, method, accumulate):
         return _dev.empty if not accumulate and self._fills(method) else _dev.zeros
@@ -317,7 +324,7 @@ class Normal(_AbstractDistribution):
                       p["icov"].data_ptr(), work.data_ptr(), out.data_ptr(), int(accumulate), stream)
 
     def _row_prior(self, dtype):
-        if not self.diagonal or type(self)._device_gradient is not Normal._device_gradient:
+        if not self.diagonal or not _keeps(self, Normal, "_device_gradient"):
             return None
         p = self._params(dtype)
         return 1, p["mean"], p["iv"]
@@ -380,7 +387,7 @@ class Laplace(_AbstractDistribution):
                   p["mean"].data_ptr(), p["iw"].data_ptr(), out.data_ptr(), int(accumulate), stream)
 
     def _row_prior(self, dtype):
-        if type(self)._device_gradient is not Laplace._device_gradient:
+        if not _keeps(self, Laplace, "_device_gradient"):
             return None
         p = self._params(dtype)
         return 2, p["mean"], p["iw"]
@@ -697,7 +704,7 @@ class LinearMatrix(_AbstractDistribution):
     def _gradient_with_prior(self, prior, M, out, dtype, stream):
         # (an unaligned M keeps the two passes: the four-chain product reads it in 16 bytes)
         if (self.dense or self.premultiplication or dtype != "float32" or M.data_ptr() % 16
-                or type(self)._device_gradient is not LinearMatrix._device_gradient):
+                or not _keeps(self, LinearMatrix, "_device_gradient")):
             return False
         row = prior._row_prior(dtype)
         if row is None:
