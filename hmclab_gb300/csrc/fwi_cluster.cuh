@@ -26,7 +26,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
-#include "halo_exit.cuh"
+#include "halo_rules.cuh"
 
 namespace hmc {
 namespace fwi {

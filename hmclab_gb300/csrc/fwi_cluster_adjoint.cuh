@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
                  down_bar = remote_of(smem_of(&bars), has_down ? rank + 1 : rank);
   uint32_t parity = 0;
   bool dead = false;
-  const bool sends = column && !(g.withhold && blockIdx.x == 0 && i == 0);
+  const bool sends = halo_sends(column) && !(g.withhold && blockIdx.x == 0 && i == 0);
+  const bool awaits = halo_awaits(column) && bytes;  // some neighbour
   // edge rows of the operands a (rows -1, RZ, RZ + 1) and b (rows -2, -1, RZ) to
   // the neighbours; k numbers the barrier
 #define PUSH(k, a, b)                                                             \
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
   }
 #define SETTLE(k)                                          \
   __syncthreads();                                         \
-  if (bytes) { /* some neighbour */                        \
+  if (awaits) {                                            \
     halo_wait(bars, k, parity, g.wait_ns, g.status, dead); \
     if (i == 0 && !dead) halo_arm(bars, k, bytes);         \
   }

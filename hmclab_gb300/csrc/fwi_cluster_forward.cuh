@@ -83,7 +83,8 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
                  down_bar = remote_of(smem_of(&bars), has_down ? rank + 1 : rank);
   uint32_t parity = 0;
   bool dead = false;
-  const bool sends = column && !(g.withhold && blockIdx.x == 0 && i == 0);
+  const bool sends = halo_sends(column) && !(g.withhold && blockIdx.x == 0 && i == 0);
+  const bool awaits = halo_awaits(column) && bytes;  // some neighbour
 
   // Edge rows to the neighbours: fa is differentiated downwards (rows -2, -1,
   // RZ) and fb upwards (rows -1, RZ, RZ + 1); k numbers the barrier.
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
     }                                                        \
   }                                                          \
   __syncthreads();                                           \
-  if (bytes) { /* some neighbour */                          \
+  if (awaits) {                                              \
     halo_wait(bars, k, parity, g.wait_ns, g.status, dead);   \
     if (i == 0 && !dead) halo_arm(bars, k, bytes);           \
   }

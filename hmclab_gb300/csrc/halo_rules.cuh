@@ -1,5 +1,10 @@
-// When a block of an elastic shot on chip may leave (fwi_cluster.cuh).
+// Rules of the edge rows' exchange in elastic shots on chip (fwi_cluster.cuh).
 //
+// Who takes part: the lanes of the grid's columns send, and only they wait.  A lane
+// that waited without sending would hold nobody up: the barrier could pass two phases
+// while it still asks for the first, and two phases look like none to it.
+//
+// When a block may leave.
 // A block whose halo waits all succeeded holds every edge row that was sent to it.
 // One that gave up does not: a late neighbour may send its last rows only then,
 // and its own wait succeeds, as the block that gave up had sent before it waited.
@@ -18,6 +23,9 @@
 
 namespace hmc {
 namespace fwi {
+
+HMC_HALO_HD bool halo_sends(bool column) { return column; }
+HMC_HALO_HD bool halo_awaits(bool column) { return column; }
 
 constexpr unsigned long long HALO_DRAIN_NS = 20000;
 // gave_up: a wait of this thread ran out; status: the word, read after its last send.
