@@ -108,6 +108,30 @@ def test_tall_matrices(m, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m", [97, 127, 128])
+@pytest.mark.parametrize("n,offset", [(5, 0), (32, 0), (36, 0), (32, 1)])
+def test_eight_rows_per_thread(rules, m, n, offset):
+    torch = _cuda()
+    k = 33
+    assert rules.rows_per_thread(m, n, k) == 8
+    rng = np.random.default_rng(m + n)
+    A, B, bias = (rng.normal(size=s).astype(np.float32) for s in ((m, k), (k, n), (m,)))
+
+    def put(a):  # offset: four bytes past a 16-byte boundary
+        t = torch.zeros(a.size + offset, device="cuda")
+        t[offset:] = torch.from_numpy(a.ravel()).cuda()
+        return t[offset:]
+
+    tA, tB, tb = put(A), put(B), put(bias)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    _lib.call("hmc_gemm", _lib.HMC_F32, m, n, k, 1.5, tA.data_ptr(), tB.data_ptr(), tb.data_ptr(), out.data_ptr(), 0,
+              torch.cuda.current_stream().cuda_stream)
+    A, B, bias = (a.astype(np.float64) for a in (A, B, bias))
+    bound = 2.0**-24 * (k + 4) * (1.5 * np.abs(A) @ np.abs(B) + np.abs(bias)[:, None])
+    assert np.all(np.abs(out.cpu().numpy() - (1.5 * A @ B + bias[:, None])) <= bound)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [(144, 8, 30_200_000), (64, 2, 68_000_000), (31, 8, 139_000_000)])
 def test_long_rows(m, n, k):
     """Rows whose offsets pass 2^32 (17 GB): one entry per row, so every product is
