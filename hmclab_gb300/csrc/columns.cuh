@@ -12,39 +12,10 @@
 
 #include <cooperative_groups.h>
 
+#include "column_shape.cuh"
 #include "common.cuh"
 
 namespace hmc {
-
-constexpr int COL_THREADS = 512;
-
-struct ColumnShape {
-  int log_x;    // a tile holds 1 << log_x chains
-  int cluster;  // blocks that share a tile's rows
-};
-
-// Tile width: 32 chains (one 128-byte FP32 row segment per warp), or the next
-// power of two for fewer chains, whose idle lanes then take rows instead.
-// Cluster: doubled while the grid stays within one resident wave (two blocks on
-// an SM) and every lane keeps four rows: a block sums, waits for the cluster and
-// then moves rows, and a second wave pays these latencies again (a pass of two
-// proposals of 20 steps, d = 1000, 4096 chains: 2052 us at up to 256 blocks, 2063
-// at 512, 2113 at 1024, 2116 at 128); fewer than 32 chains always spread over eight
-// SMs, because a warp alone on its scheduler issues FP64 at half the SM's rate
-// (d = 1000, one chain: momenta in 13 us on eight SMs,
-// 418 us in one lane of one block's warps).
-inline ColumnShape column_shape(int64_t C, int64_t rows) {
-  ColumnShape s{0, 1};
-  while (s.log_x < 5 && (1ll << s.log_x) < C) ++s.log_x;
-  const int64_t tiles = (C + (1 << s.log_x) - 1) >> s.log_x;
-  const int64_t lanes = COL_THREADS >> s.log_x;
-  if (s.log_x < 5) {
-    while (s.cluster < 8 && rows >= 16 * s.cluster) s.cluster *= 2;
-  } else {
-    while (s.cluster < 8 && 2 * s.cluster * tiles <= 256 && rows >= 4 * lanes * 2 * s.cluster) s.cluster *= 2;
-  }
-  return s;
-}
 
 struct ColumnTile {
   int64_t c;   // this thread's chain
@@ -63,7 +34,7 @@ __device__ __forceinline__ ColumnTile column_tile(const ColumnShape& s, int64_t 
   t.first = rank == 0 && (int)threadIdx.x < (1 << s.log_x);
   // consecutive rows go to different blocks, so few rows still use every SM
   t.row = (int64_t)(threadIdx.x >> s.log_x) * s.cluster + rank;
-  t.rows = (int64_t)(COL_THREADS >> s.log_x) * s.cluster;
+  t.rows = (int64_t)(s.threads >> s.log_x) * s.cluster;
   return t;
 }
 
@@ -92,7 +63,7 @@ __device__ __forceinline__ double column_total(const ColumnShape& s, double v, C
   __syncthreads();
   double total = 0.0;
   if ((int)threadIdx.x < X) {
-    for (int k = 0; k < COL_THREADS / 32; ++k) total += sh.warp[k][threadIdx.x];
+    for (int k = 0; k < s.threads / 32; ++k) total += sh.warp[k][threadIdx.x];
     sh.block[threadIdx.x] = total;
   }
   column_sync(s);
@@ -114,7 +85,7 @@ int launch_columns(const char* who, void (*kernel)(P...), const ColumnShape& s, 
   HMC_REQUIRE(tiles * s.cluster <= 0x7FFFFFFF, "%s: too many chains", who);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(tiles * s.cluster));
-  cfg.blockDim = dim3(COL_THREADS);
+  cfg.blockDim = dim3((unsigned)s.threads);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -548,7 +548,7 @@ template <typename T>
 int end_impl(const hmc_chains* s, cudaStream_t st) {
   HMC_TRY(check_state<T>(s, "hmc_end_trajectory"));
   ChainView<T> v = view<T>(s);
-  const ColumnShape shape = column_shape(s->chains, s->dims);
+  const ColumnShape shape = column_shape(s->chains, s->dims, 320);
   const char* who = "end_kernel";
   switch (s->mass_kind) {
     case HMC_MASS_UNIT:
