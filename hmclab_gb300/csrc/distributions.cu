@@ -79,6 +79,7 @@ template <typename T, int VEC>
 struct alignas(sizeof(T) * VEC) Pack {
   T v[VEC];
 };
+constexpr int PRIOR_ROWS = 4;  // rows of a thread loaded together
 template <typename T, int KIND, int VEC>
 __global__ void __launch_bounds__(256) prior_gradient_kernel(int64_t d, int64_t C, const T* __restrict__ M,
                                                              const T* __restrict__ mean, const T* __restrict__ w,
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(256) prior_gradient_kernel(int64_t d, int64_t 
   using V = Pack<T, VEC>;
   const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * VEC;
   if (c >= C) return;
-  constexpr int U = 4;  // rows loaded together
+  constexpr int U = PRIOR_ROWS;
   const int64_t stride = (int64_t)gridDim.y * blockDim.y;
   for (int64_t r0 = blockIdx.y * (int64_t)blockDim.y + threadIdx.y; r0 < d; r0 += U * stride) {
     V m[U], o[U];
@@ -117,14 +118,14 @@ __global__ void __launch_bounds__(256) prior_gradient_kernel(int64_t d, int64_t 
 }
 
 template <typename T, int KIND, int VEC>
-int prior_gradient_launch(int64_t d, int64_t C, const T* M, const T* mean, const T* w, T* out, int accumulate,
+int prior_gradient_launch(int64_t d, int64_t C, int rows, const T* M, const T* mean, const T* w, T* out, int accumulate,
                           cudaStream_t st, const char* who) {
   const int64_t cols = (C + VEC - 1) / VEC;
   unsigned bx = 1;
   while (bx < 256 && bx < cols) bx *= 2;
   const dim3 block(bx, 256 / bx);
   const int64_t gx = (cols + bx - 1) / bx;
-  int64_t gy = (d + 4 * block.y - 1) / (4 * block.y);  // the four rows a thread loads together
+  int64_t gy = (d + rows * block.y - 1) / (rows * block.y);
   while (gy > 1 && gx * gy > 152 * 16) gy = (gy + 1) / 2;
   HMC_REQUIRE(gx <= 0x7FFFFFFF, "%s: too many chains", who);
   const dim3 grid((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535));
@@ -149,11 +150,11 @@ int prior_gradient(int64_t d, int64_t C, const void* M, const void* mean, const 
   HMC_REQUIRE(d > 0 && C >= 0, "%s: bad sizes", who);
   if (C == 0) return HMC_OK;
   HMC_REQUIRE(M && mean && w && out, "%s: null argument", who);
-  constexpr int VEC = 16 / (int)sizeof(T);
   const T *Mt = (const T*)M, *mt = (const T*)mean, *wt = (const T*)w;
-  if (C % VEC == 0 && ((uintptr_t)M | (uintptr_t)out) % 16 == 0)
-    return prior_gradient_launch<T, KIND, VEC>(d, C, Mt, mt, wt, (T*)out, accumulate, st, who);
-  return prior_gradient_launch<T, KIND, 1>(d, C, Mt, mt, wt, (T*)out, accumulate, st, who);
+  const ElementShape e =
+      element_shape(d, C, (int)sizeof(T), ((uintptr_t)M | (uintptr_t)out) % 16 == 0, PRIOR_ROWS);
+  return e.vec ? prior_gradient_launch<T, KIND, 16 / (int)sizeof(T)>(d, C, e.rows, Mt, mt, wt, (T*)out, accumulate, st, who)
+               : prior_gradient_launch<T, KIND, 1>(d, C, e.rows, Mt, mt, wt, (T*)out, accumulate, st, who);
 }
 
 // ---- per-chain quadratic forms ---------------------------------------------

@@ -486,16 +486,16 @@ int begin_impl(const hmc_chains* s, double drift, cudaStream_t st) {
   }
 }
 
-// Threads (x over chains, y over rows) and grid of the kick: at least the
-// rows a thread loads together, which also share the per-chain work.
+// Threads (x over chains, y over rows) and grid of the kick: `rows` at least per
+// thread (element_shape), KICK_ROWS of them loaded together.
 template <typename T, int MASS, int VEC>
-int kick_drift_launch(const ChainView<T>& v, bool do_kick, bool do_drift, double kick, double drift,
+int kick_drift_launch(const ChainView<T>& v, int rows, bool do_kick, bool do_drift, double kick, double drift,
                       cudaStream_t st) {
   const int64_t cols = (v.C + VEC - 1) / VEC;
   unsigned bx = 1;
   while (bx < 256 && bx < cols) bx *= 2;
   const dim3 block(bx, 256 / bx);
-  int64_t gy = (v.d + KICK_ROWS * block.y - 1) / (KICK_ROWS * block.y);
+  int64_t gy = (v.d + rows * block.y - 1) / (rows * block.y);
   const int64_t gx = (cols + bx - 1) / bx;
   while (gy > 1 && gx * gy > 152 * 16) gy = (gy + 1) / 2;
   HMC_REQUIRE(gx <= 0x7FFFFFFF, "hmc_kick_drift: too many chains");
@@ -512,11 +512,11 @@ int kick_drift_launch(const ChainView<T>& v, bool do_kick, bool do_drift, double
 
 template <typename T, int MASS>
 int kick_drift_any(const ChainView<T>& v, bool do_kick, bool do_drift, double kick, double drift, cudaStream_t st) {
-  constexpr int VEC = 16 / (int)sizeof(T);
   // 16-byte accesses need every row of the [d][C] state on a 16-byte boundary
-  const bool vec = v.C % VEC == 0 && ((uintptr_t)v.q | (uintptr_t)v.p | (uintptr_t)v.g | (uintptr_t)v.v) % 16 == 0;
-  return vec ? kick_drift_launch<T, MASS, VEC>(v, do_kick, do_drift, kick, drift, st)
-             : kick_drift_launch<T, MASS, 1>(v, do_kick, do_drift, kick, drift, st);
+  const bool aligned = ((uintptr_t)v.q | (uintptr_t)v.p | (uintptr_t)v.g | (uintptr_t)v.v) % 16 == 0;
+  const ElementShape e = element_shape(v.d, v.C, (int)sizeof(T), aligned, KICK_ROWS);
+  return e.vec ? kick_drift_launch<T, MASS, 16 / (int)sizeof(T)>(v, e.rows, do_kick, do_drift, kick, drift, st)
+               : kick_drift_launch<T, MASS, 1>(v, e.rows, do_kick, do_drift, kick, drift, st);
 }
 
 template <typename T>

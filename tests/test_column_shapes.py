@@ -13,6 +13,10 @@ D = H.Distributions
 
 _SOURCE = r"""
 #include "column_shape.cuh"
+extern "C" int element(int64_t d, int64_t C, int bytes, int aligned, int most) {
+  const hmc::ElementShape s = hmc::element_shape(d, C, bytes, aligned != 0, most);
+  return s.vec ? 100 + s.rows : s.rows;
+}
 extern "C" void shape(int64_t C, int64_t rows, int64_t narrow, int* out) {
   const hmc::ColumnShape s = narrow > 0 ? hmc::column_shape(C, rows, narrow) : hmc::column_shape(C, rows);
   out[0] = 1 << s.log_x;
@@ -36,6 +40,7 @@ def shape(tmp_path_factory):
         lib.shape(ctypes.c_int64(C), ctypes.c_int64(rows), ctypes.c_int64(narrow), out)
         return tuple(out)
 
+    call.element = lambda d, C, nbytes, aligned, most: lib.element(ctypes.c_int64(d), ctypes.c_int64(C), nbytes, aligned, most)
     return call
 
 
@@ -59,6 +64,36 @@ def test_few_rows_take_few_threads(shape):
     # layouts that the sums of many rows were measured with
     assert shape(1, 1000) == (1, 8, 512) and shape(1024, 4096) == (32, 8, 512) and shape(4096, 1000) == (32, 2, 512)
     assert shape(8192, 129) == (32, 1, 512)
+
+
+def test_elements_take_few_threads_only_on_a_full_chip(shape):
+    """Two to four rows and 16 bytes per thread made small FP64 updates up to 1.8 times as slow."""
+    for d, C in ((40, 512), (4096, 4), (16, 1024), (1, 1), (9, 4096)):
+        assert shape.element(d, C, 8, 1, 2) == shape.element(d, C, 8, 1, 4) == shape.element(d, C, 4, 1, 4) == 1
+    assert shape.element(1500, 20_000, 8, 1, 4) == 102 and shape.element(600, 1024, 4, 1, 2) == 102
+    assert shape.element(4096, 1024, 4, 1, 2) == 102 and shape.element(4096, 1024, 4, 1, 4) == 104
+    assert shape.element(4096, 1024, 4, 0, 4) == 4 and shape.element(4096, 1023, 4, 1, 2) == 2  # no 16-byte rows
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,C", [(125, 512), (124, 516), (250, 256), (1000, 2000), (1001, 2000), (80, 501), (80, 499), (1, 64_000),
+                                 (40, 2048), (300, 1027)])
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("kind", ["normal", "laplace"])
+def test_prior_gradients(d, C, dtype, kind):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    rng = np.random.default_rng(d + C)
+    mean, w = rng.normal(size=(d, 1)).astype(dtype), rng.uniform(0.5, 2.0, size=(d, 1)).astype(dtype)
+    q = rng.normal(size=(d, C)).astype(dtype)
+    make = D.Normal if kind == "normal" else D.Laplace
+    iw = (1.0 / w.astype(float)).astype(dtype)
+    want = -(iw * (mean - q)) if kind == "normal" else np.sign(q - mean) * iw
+    post, M = make(mean.astype(float), w.astype(float)), torch.from_numpy(q).cuda()
+    assert np.array_equal(post.gradient_batch(M).cpu().numpy(), want)
+    twice = post.gradient_batch(M, out=torch.from_numpy(want.copy()).cuda(), accumulate=True)
+    assert np.array_equal(twice.cpu().numpy(), want + want)
 
 
 @pytest.mark.gpu
