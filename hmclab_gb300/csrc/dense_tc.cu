@@ -32,13 +32,11 @@
 
 #include "common.cuh"
 #include "gelu.cuh"
+#include "tc_tiles.cuh"
 
 namespace hmc {
 namespace tc {
 
-constexpr int BM = 128;                   // chains per tile (UMMA M)
-constexpr int BN = 256;                   // matrix rows per tile (UMMA N), many tiles
-constexpr int BN_FEW = 32;                // the same where 256 would leave most SMs idle
 constexpr int SWZ = 64;                   // swizzle span in bytes (64 or 128)
 constexpr int BK = SWZ / 2;               // k per stage = one swizzle row of bf16
 constexpr int UK = 16;                    // k per tcgen05.mma (kind::f16)
@@ -931,21 +929,16 @@ int launch_tiles(int64_t C, int64_t rows, int64_t K, const void* q_hi, const voi
   return check_launch("chain_gemm_kernel");
 }
 
-// Tiles of 256 matrix rows read the operands least often; where they are so few
-// that most SMs would idle, eight times as many of 32 rows (512 x 256 outputs,
-// 512 products: 37 us with 4 wide tiles, 8.6 us with 32; the line is where the
-// narrow ones fill the SMs twice).
 template <int EPI, int NPROD = 3>
 int launch(int64_t C, int64_t rows, int64_t K, const void* q_hi, const void* q_lo, int64_t ldq, const void* a_hi,
            const void* a_lo, int64_t lda, const EpiParams& ep, cudaStream_t st) {
   HMC_REQUIRE(C > 0 && rows > 0 && K > 0, "tensor-core contraction: bad sizes");
   HMC_REQUIRE(C < (1ll << 31) && rows < (1ll << 31) && K < (1ll << 31), "tensor-core contraction: too large");
   HMC_REQUIRE(ep.status != nullptr, "tensor-core contraction: null status word");
-  const int64_t tiles = (C + BM - 1) / BM * ((rows + BN - 1) / BN);
   HMC_REQUIRE((rows + BN - 1) / BN <= 65535, "tensor-core contraction: too many rows");
   // (the fused step and the misfit, whose partial sums are per 256 rows, keep the wide tiles)
   if constexpr (EPI != EPI_STEP && EPI != EPI_MISFIT) {
-    if (tiles <= 38) return launch_tiles<EPI, NPROD, BN_FEW>(C, rows, K, q_hi, q_lo, ldq, a_hi, a_lo, lda, ep, st);
+    if (narrow_tiles(C, rows, K, NPROD)) return launch_tiles<EPI, NPROD, BN_FEW>(C, rows, K, q_hi, q_lo, ldq, a_hi, a_lo, lda, ep, st);
   }
   return launch_tiles<EPI, NPROD, BN>(C, rows, K, q_hi, q_lo, ldq, a_hi, a_lo, lda, ep, st);
 }
