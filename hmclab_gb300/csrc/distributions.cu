@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "columns.cuh"
+#include "srcloc_shape.cuh"
 
 namespace hmc {
 int gemm_ex(int dtype, int64_t m, int64_t n, int64_t k, double alpha, const void* A, const void* B, const void* bias,
@@ -753,13 +754,13 @@ __device__ __forceinline__ float x2_sum(f32x2 v) {
   return a + b;
 }
 
-// Blocks of 32 chains and 8 events; the blocks of a cluster share a tile's
-// events and add their FP64 parts in block 0.  FP32 arithmetic bounds it (57 % of
-// the pipe over the chip with 16 events per block and a loop over events: 256
-// blocks on 152 SMs left a sixth of it waiting).  32 events, 200 stations,
-// 8192 chains, four proposals of five steps: 1706 us, now 1582.
-constexpr int SL_BY = 8;  // event lanes per block
-template <bool GRAD>
+// Blocks of 32 chains and up to 8 events (LANES; 0: blockDim.y); the blocks of a
+// cluster share a tile's events and add their FP64 parts in block 0 (srcloc_shape).
+// FP32 arithmetic bounds it (57 % of the pipe over the chip with 16 events per
+// block and a loop over events: 256 blocks on 152 SMs left a sixth of it waiting).
+// 32 events, 200 stations, 8192 chains, four proposals of five steps: 1706 us, now
+// 1582.
+template <bool GRAD, int LANES>
 __global__ void __launch_bounds__(RED_X * SL_BY, 4)
     srcloc_f32_kernel(int64_t E, int64_t S, int64_t C, const float* __restrict__ M, const float* __restrict__ rx,
                       const float* __restrict__ ry, const float* __restrict__ rz, const float* __restrict__ obs,
@@ -767,11 +768,12 @@ __global__ void __launch_bounds__(RED_X * SL_BY, 4)
                       int accumulate, int pairs, int blocks) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ulonglong2* sxy = (ulonglong2*)smem_raw;  // [pairs] (x_a, x_b), (y_a, y_b)
-  ulonglong2* swo = sxy + pairs;            // [SL_BY][pairs] (w_a, w_b), (o_a, o_b)
-  f32x2* sz = (f32x2*)(swo + SL_BY * pairs);  // [pairs] (z_a, z_b)
+  ulonglong2* swo = sxy + pairs;            // [event lanes][pairs] (w_a, w_b), (o_a, o_b)
+  const int by = LANES ? LANES : blockDim.y;
+  f32x2* sz = (f32x2*)(swo + by * pairs);  // [pairs] (z_a, z_b)
   __shared__ double red[SL_BY][RED_X + 1];
   __shared__ double part[RED_X];
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = RED_X * SL_BY;
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = RED_X * by;
   const int rank = (int)(blockIdx.x % (unsigned)blocks);
   const int64_t c = blockIdx.x / (unsigned)blocks * (int64_t)RED_X + threadIdx.x;
   const bool live = c < C;
@@ -779,7 +781,7 @@ __global__ void __launch_bounds__(RED_X * SL_BY, 4)
   const float inv_v = 1.f / v;
   const f32x2 IV = x2_pack(inv_v, inv_v), EPS = x2_pack(1e-30f, 1e-30f);
   double mis = 0.0, gvd_total = 0.0;
-  for (int64_t e0 = rank * SL_BY; e0 < E; e0 += blocks * SL_BY) {
+  for (int64_t e0 = rank * by; e0 < E; e0 += blocks * by) {
     const int64_t e = e0 + threadIdx.y;
     const bool ev = live && e < E;
     float x = 0.f, y = 0.f, z = 0.f, t0 = 0.f;
@@ -867,7 +869,7 @@ __global__ void __launch_bounds__(RED_X * SL_BY, 4)
   __syncthreads();
   double sum = 0.0;
   if (threadIdx.y == 0) {
-    for (int yy = 0; yy < SL_BY; ++yy) sum += red[yy][threadIdx.x];
+    for (int yy = 0; yy < by; ++yy) sum += red[yy][threadIdx.x];
     part[threadIdx.x] = sum;
   }
   if (blocks > 1) {
@@ -903,21 +905,23 @@ int srcloc(bool grad, int64_t E, int64_t S, int64_t C, const void* M, const void
   if (sizeof(T) == 4) {
     // stations staged at a time, and blocks that share a tile's events
     const int pairs = S < SL_CHUNK ? (int)(S + 1) / 2 : SL_PAIRS;
-    const int64_t groups = (E + SL_BY - 1) / SL_BY;
-    const int blocks = groups < 8 ? (int)groups : 8;
+    const SrclocShape shape = srcloc_shape(E, S, C);
+    const int blocks = shape.blocks, by = shape.lanes;
     const int64_t tiles = (C + RED_X - 1) / RED_X;
     HMC_REQUIRE(tiles * blocks <= 0x7FFFFFFF, "%s: too many chains", who);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * blocks));
-    cfg.blockDim = dim3(RED_X, SL_BY);
-    cfg.dynamicSmemBytes = (size_t)pairs * ((1 + SL_BY) * sizeof(ulonglong2) + sizeof(f32x2));
+    cfg.blockDim = dim3(RED_X, (unsigned)by);
+    cfg.dynamicSmemBytes = (size_t)pairs * ((1 + by) * sizeof(ulonglong2) + sizeof(f32x2));
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim = {(unsigned)blocks, 1, 1};
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, grad ? srcloc_f32_kernel<true> : srcloc_f32_kernel<false>, E, S, C,
+    auto k32 = by == SL_BY ? (grad ? srcloc_f32_kernel<true, SL_BY> : srcloc_f32_kernel<false, SL_BY>)
+                           : (grad ? srcloc_f32_kernel<true, 0> : srcloc_f32_kernel<false, 0>);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k32, E, S, C,
                                        (const float*)M, (const float*)rx, (const float*)ry, (const float*)rz,
                                        (const float*)obs, (const float*)iv, infer_v, (float)v_fixed, out_x,
                                        (float*)out_g, accumulate, pairs, blocks);
