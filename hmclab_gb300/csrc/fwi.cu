@@ -948,19 +948,19 @@ static StoreSlot store_slot(const hmc_fwi* s, int n) {
   return {base, base + 2 * cells, 4ll * (n / k) * s->nz};
 }
 
-static int cluster_forward(const ShotForward& a, const Waves& w, bool dry, int* rows, cudaStream_t st) {
-  *rows = 0;
+static int cluster_forward(const ShotForward& a, const Waves& w, bool dry, Strip* strip, cudaStream_t st) {
+  *strip = Strip{};
   if (a.nx > CLUSTER_COLUMNS || a.C > 0x7FFFFFFF / CLUSTER_MAX) return HMC_OK;
-  return a.nx <= 128   ? cluster_forward_at<128>(a, w, dry, rows, st)
-         : a.nx <= 192 ? cluster_forward_at<192>(a, w, dry, rows, st)
-                       : cluster_forward_at<256>(a, w, dry, rows, st);
+  return a.nx <= 128   ? cluster_forward_at<128>(a, w, dry, strip, st)
+         : a.nx <= 192 ? cluster_forward_at<192>(a, w, dry, strip, st)
+                       : cluster_forward_at<256>(a, w, dry, strip, st);
 }
-static int cluster_adjoint(const ShotAdjoint& a, bool dry, int* rows, cudaStream_t st) {
-  *rows = 0;
+static int cluster_adjoint(const ShotAdjoint& a, bool dry, Strip* strip, cudaStream_t st) {
+  *strip = Strip{};
   if (a.nx > CLUSTER_COLUMNS || a.C > 0x7FFFFFFF / CLUSTER_MAX) return HMC_OK;
-  return a.nx <= 128   ? cluster_adjoint_at<128>(a, dry, rows, st)
-         : a.nx <= 192 ? cluster_adjoint_at<192>(a, dry, rows, st)
-                       : cluster_adjoint_at<256>(a, dry, rows, st);
+  return a.nx <= 128   ? cluster_adjoint_at<128>(a, dry, strip, st)
+         : a.nx <= 192 ? cluster_adjoint_at<192>(a, dry, strip, st)
+                       : cluster_adjoint_at<256>(a, dry, strip, st);
 }
 static ShotForward forward_args(const hmc_fwi* s, int shot, int store) {
   ShotForward a = {};
@@ -1023,24 +1023,25 @@ static ShotAdjoint adjoint_args(const hmc_fwi* s) {
   return a;
 }
 // Whether a shot runs with the wavefield on chip (fwi_cluster.cuh): grids of up
-// to 256 columns whose strips fit a cluster.  A stored wavefield has another
+// to 256 columns whose strips fit a cluster, where a step is expected to take less time
+// there (fwi_choice.cuh).  A stored wavefield has another
 // layout there ([chain][plane] instead of [plane][chain]), so the forward pass
 // that stores it and the adjoint that reads it decide together, from the descriptor
 // alone.  A null status word keeps the direct-load kernels.  Per
 // time step of 240 x 140 cells the staged
 // and direct-load kernels take 16.8 / 17.1 / 21.7 us (misfit) and 45 / 46 /
 // 82 us (misfit and gradient) for 1 / 16 / 64 chains, these 2.9 / 5.5 / 15.3 us
-// and 10 / 24 / 62 us; at 160 x 100 cells and 64 chains it is 11.8 and 37.9 us
-// against 8.1 and 34.7 us, the narrowest margin of the grids tried.
-// Strip heights of the shot's passes, 0 where the per-step kernels run.
-static int on_chip(const hmc_fwi* s, int store, int* forward, int* adjoint) {
-  *forward = *adjoint = 0;
+// and 10 / 24 / 62 us.
+static int on_chip(const hmc_fwi* s, int store, Strip* forward, Strip* adjoint) {
+  *forward = *adjoint = Strip{};
   if (!s->status) return HMC_OK;
   static const Waves none = {};
   HMC_TRY(cluster_forward(forward_args(s, 0, store), none, true, forward, nullptr));
-  if (!store || *forward == 0) return HMC_OK;
-  HMC_TRY(cluster_adjoint(adjoint_args(s), true, adjoint, nullptr));
-  if (*adjoint == 0) *forward = 0;
+  if (store && forward->rows) HMC_TRY(cluster_adjoint(adjoint_args(s), true, adjoint, nullptr));
+  const bool fits = forward->rows && (!store || adjoint->rows);
+  if (!fits || forward->step_us + adjoint->step_us >=
+                   stencil_step_us((int64_t)s->nx * s->nz, s->chains, s->chains % 32 == 0, store != 0))
+    *forward = *adjoint = Strip{};
   return HMC_OK;
 }
 
@@ -1049,7 +1050,11 @@ extern "C" {
 HMC_API int hmc_fwi_strips(const hmc_fwi* s, int store, int* forward, int* adjoint) {
   HMC_TRY(check_fwi(s, "hmc_fwi_strips"));
   HMC_REQUIRE(forward && adjoint, "hmc_fwi_strips: null output");
-  return on_chip(s, store, forward, adjoint);
+  Strip f, a;
+  HMC_TRY(on_chip(s, store, &f, &a));
+  *forward = f.rows;
+  *adjoint = a.rows;
+  return HMC_OK;
 }
 
 HMC_API int hmc_fwi_prepare(const hmc_fwi* s, void* stream) {
@@ -1114,9 +1119,9 @@ HMC_API int hmc_fwi_forward_shot_sources(const hmc_fwi* s, int shot, const hmc_f
     return ss;
   };
   cudaStream_t st = as_stream(stream);
-  int strip = 0, adjoint_strip = 0;
+  Strip strip, adjoint_strip;
   if (n_src <= WAVE_SAMPLES) HMC_TRY(on_chip(s, store, &strip, &adjoint_strip));
-  if (strip) {
+  if (strip.rows) {
     ShotForward a = forward_args(s, shot, store);
     Waves w = {};
     auto term = [&](int q, int i, int j, float xx, float zz, float xz) {
@@ -1151,7 +1156,7 @@ HMC_API int hmc_fwi_forward_shot_sources(const hmc_fwi* s, int shot, const hmc_f
       for (int q = 0; q < n_src; ++q)
         for (int n = 0; n < steps; ++n) w.s[q * steps + n] = src[q].stf_host[n0 + n] * src_scale;
       HMC_TRY(cluster_forward(a, w, false, &strip, st));
-      HMC_REQUIRE(strip, "hmc_fwi_forward_shot_sources: no strip height fits");
+      HMC_REQUIRE(strip.rows, "hmc_fwi_forward_shot_sources: no strip height fits");
     }
     return HMC_OK;
   }
@@ -1232,9 +1237,9 @@ HMC_API int hmc_fwi_adjoint_shot(const hmc_fwi* s, int shot, void* stream) {
   residual_kernel<<<grid_for(rows * s->chains), 256, 0, st>>>(rows, s->chains, s->rec + shot_off * s->chains,
                                                               s->obs + shot_off, s->w, s->resid);
   HMC_TRY(check_launch("residual_kernel"));
-  int forward_strip = 0, strip = 0;
+  Strip forward_strip, strip;
   HMC_TRY(on_chip(s, 1, &forward_strip, &strip));
-  if (strip) return cluster_adjoint(adjoint_args(s), false, &strip, st);
+  if (strip.rows) return cluster_adjoint(adjoint_args(s), false, &strip, st);
   const Grid g = grid_of(s);
   const int64_t cells = (int64_t)s->nx * s->nz * s->chains;
   const size_t fb = (size_t)cells * sizeof(float);

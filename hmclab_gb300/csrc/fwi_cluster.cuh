@@ -26,6 +26,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "fwi_choice.cuh"
 #include "halo_rules.cuh"
 
 namespace hmc {
@@ -165,27 +166,31 @@ constexpr int adjoint_rows(int rz) { return adjoint_shares(rz) ? 14 * rz + 24 : 
 #define HMC_FORWARD_STRIPS(X) X(4) X(5) X(7) X(9) X(10) X(14)
 #define HMC_ADJOINT_STRIPS(X) X(4) X(5) X(7) X(9) X(11) X(14)
 
-// Launch one shot; *rows is the strip height, 0 when none fits (the caller then
-// runs the per-step kernels).  dry: only tell the height.  The pitch of a row
+struct Strip {
+  int rows = 0;          // of a block; 0: no strip fits, the per-step kernels run
+  double step_us = 0.0;  // expected time of a step
+};
+// Launch one shot.  dry: only tell the strip.  The pitch of a row
 // in shared memory is a constant, so that offsets are immediates; a narrow grid
 // takes a narrow one, which lets several blocks share an SM: 64 chains of 100 x
 // 70 cells take 21.4 us per step of misfit and gradient with 256 columns and 15.0
 // with 128 (compiled in fwi_cluster_128.cu, fwi_cluster_192.cu and
 // fwi_cluster_256.cu).
 template <int PITCH>
-int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, int* rows, cudaStream_t st);
+int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, Strip* strip, cudaStream_t st);
 template <int PITCH>
-int cluster_adjoint_at(const ShotAdjoint& a, bool dry, int* rows, cudaStream_t st);
+int cluster_adjoint_at(const ShotAdjoint& a, bool dry, Strip* strip, cudaStream_t st);
 
 // The strip height for C chains: the cheapest number of waves of resident
 // clusters, a step of a wave costing its rows' instructions (those of all
 // blocks of an SM) or, if that is more, one block's and two halo exchanges.
 struct ClusterChoice {
   int rz = 0, R = 0;
-  double cost = 0.0;
+  double cost = 0.0, step_us = 0.0;
 };
 template <typename Kernel>
-void consider_strip(ClusterChoice& best, Kernel kern, int rz, int floats, int nx, int nz, int64_t C, double row_instr) {
+void consider_strip(ClusterChoice& best, Kernel kern, int rz, int floats, int nx, int nz, int64_t C, double row_instr,
+                    const StripModel& model) {
   const int R = (nz + rz - 1) / rz;
   const size_t smem = (size_t)floats * sizeof(float);
   if (R > CLUSTER_MAX || smem > 227 * 1024 - 64) return;
@@ -215,7 +220,8 @@ void consider_strip(ClusterChoice& best, Kernel kern, int rz, int floats, int nx
   const double work = rz * row_instr * (threads / 32) / 4;
   const double step = work * per_sm > work + 900 ? work * per_sm : work + 900;
   const double cost = step * (double)((C + n - 1) / n);
-  if (best.rz == 0 || cost < best.cost) best = ClusterChoice{rz, R, cost};
+  if (best.rz == 0 || cost < best.cost)
+    best = ClusterChoice{rz, R, cost, strip_step_us(model, rz, R, n, threads / 32, C)};
 }
 
 template <typename Kernel, typename... A>

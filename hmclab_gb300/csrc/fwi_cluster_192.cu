@@ -4,7 +4,7 @@
 
 namespace hmc {
 namespace fwi {
-template int cluster_forward_at<192>(const ShotForward&, const Waves&, bool, int*, cudaStream_t);
-template int cluster_adjoint_at<192>(const ShotAdjoint&, bool, int*, cudaStream_t);
+template int cluster_forward_at<192>(const ShotForward&, const Waves&, bool, Strip*, cudaStream_t);
+template int cluster_adjoint_at<192>(const ShotAdjoint&, bool, Strip*, cudaStream_t);
 }  // namespace fwi
 }  // namespace hmc

@@ -346,14 +346,14 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
 #undef HMC_DP
 
 template <int PITCH>
-int cluster_adjoint_at(const ShotAdjoint& a, bool dry, int* rows, cudaStream_t st) {
-  *rows = 0;
+int cluster_adjoint_at(const ShotAdjoint& a, bool dry, Strip* strip, cudaStream_t st) {
   ClusterChoice best;
 #define HMC_STRIP(RZ) \
-  consider_strip(best, cluster_adjoint_kernel<RZ, PITCH>, RZ, adjoint_rows(RZ) * PITCH, a.nx, a.nz, a.C, 210.0);
+  consider_strip(best, cluster_adjoint_kernel<RZ, PITCH>, RZ, adjoint_rows(RZ) * PITCH, a.nx, a.nz, a.C, 210.0, \
+                 ADJOINT_STEP);
   HMC_ADJOINT_STRIPS(HMC_STRIP)
 #undef HMC_STRIP
-  *rows = best.rz;
+  *strip = Strip{best.rz, best.step_us};
   if (dry || best.rz == 0) return HMC_OK;
   ShotAdjoint g = a;
   g.R = best.R;

@@ -263,14 +263,14 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
 #undef HMC_DP
 
 template <int PITCH>
-int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, int* rows, cudaStream_t st) {
-  *rows = 0;
+int cluster_forward_at(const ShotForward& a, const Waves& w, bool dry, Strip* strip, cudaStream_t st) {
   ClusterChoice best;
 #define HMC_STRIP(RZ) \
-  consider_strip(best, cluster_forward_kernel<RZ, PITCH>, RZ, forward_rows(RZ) * PITCH, a.nx, a.nz, a.C, 75.0);
+  consider_strip(best, cluster_forward_kernel<RZ, PITCH>, RZ, forward_rows(RZ) * PITCH, a.nx, a.nz, a.C, 75.0, \
+                 a.store ? STORING_STEP : FORWARD_STEP);
   HMC_FORWARD_STRIPS(HMC_STRIP)
 #undef HMC_STRIP
-  *rows = best.rz;
+  *strip = Strip{best.rz, best.step_us};
   if (dry || best.rz == 0) return HMC_OK;
   ShotForward g = a;
   g.R = best.R;
