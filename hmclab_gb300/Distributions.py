@@ -829,9 +829,10 @@ class ElasticFullWaveform2D(_AbstractDistribution):
     # each shot is a CUDA graph of its own, replayed from the host
     graph_safe = False
     # shots run with the wavefield on chip (a cluster of blocks per chain), or,
-    # on grids too wide or tall for that, with stencil neighbourhoods staged
-    # by the tensor memory accelerator (chain counts that are a multiple of
-    # 32); False selects the direct-load kernels, which give the same records.
+    # on grids too wide or tall for that and where it would take longer, with
+    # stencil neighbourhoods staged by the tensor memory accelerator (chain
+    # counts that are a multiple of 32); False selects the direct-load
+    # kernels, which give the same records.
     # Set before the first evaluation.
     staged_tiles: bool = True
 
@@ -1010,8 +1011,8 @@ class ElasticFullWaveform2D(_AbstractDistribution):
                           p["bg"][f].data_ptr(), ws[name].data_ptr(), stream)
 
     def _shot_graph(self, ws, C, shot, store_and_adjoint):
-        """CUDA graph of one shot's 2*nt half-step launches (and its adjoint),
-        captured once per workspace on a private stream and replayed on the
+        """CUDA graph of one shot (and its adjoint): a launch per direction on
+        chip, one per half step in the per-step kernels; captured once per workspace on a private stream and replayed on the
         caller's stream."""
         import ctypes
 
@@ -1070,7 +1071,7 @@ class ElasticFullWaveform2D(_AbstractDistribution):
             st = ws.get("status") if isinstance(ws, dict) else None
             if st is not None and int(st.cpu()[0]) != 0:
                 st.zero_()
-                raise DeviceTimeoutError("elastic stencil tile load timed out (bounded wait expired)")
+                raise DeviceTimeoutError("elastic shot timed out: a tile load or a halo exchange (bounded wait expired)")
 
     @_fills_output
     def _device_misfit(self, M, out, accumulate, dtype, stream):

@@ -10,9 +10,10 @@
 // Q holds the chains' positions transposed to chain-major [C][ld] (K-major
 // operand), re-split by the epilogue of every fused step.
 //
-// Kernel structure (one 128-chain x 256-row output tile per CTA, 320 threads):
-//   warp 0  TMEM allocation; one lane issues TMA tile loads (128B swizzle)
-//   warp 1  one lane issues tcgen05.mma (M=128, N=256, K=16) and commits
+// Kernel structure (one output tile of 128 chains x 256 rows per CTA, or x 32 rows
+// where the tiles are few (tc_tiles.cuh); 320 threads):
+//   warp 0  TMEM allocation; one lane issues TMA tile loads (64B swizzle)
+//   warp 1  one lane issues tcgen05.mma (M=128, N=256 or 32, K=16) and commits
 //   warps 2-9  epilogue: tcgen05.ld of the accumulator (lane = chain),
 //           then one of:
 //             EPI_GRAD       g[r][c] (+)= D - bias[r]
@@ -20,6 +21,10 @@
 //                            q += drift*eps*M^-1 p; reflect; write p, q and
 //                            the next step's Q hi/lo operand
 //             EPI_MISFIT     partial[tile][c] = sum_r (D - data[r])^2 inv_var[r]
+//             EPI_MLP_*      a network's hidden layer, output or backward pass
+//             EPI_POT        a hidden layer or product of the scalar potential with
+//                            the element-wise step that follows it
+//           (the last two with plain BF16 operands, one product)
 // Every mbarrier wait is bounded (2 s of %globaltimer by default, see
 // hmc_set_wait_limits); on expiry the CTA sets
 // *status = HMC_ERR_TIMEOUT, stops issuing work, waits (bounded) for its own

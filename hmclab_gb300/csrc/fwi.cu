@@ -6,9 +6,9 @@
 // map_kernels_to_velocity), restated from Virieux (1986) / Levander (1988)
 // with a Cerjan et al. (1985) sponge.
 //
-// A shot runs with the wavefield on chip (fwi_cluster.cuh) wherever the grid
-// fits; the kernels of this file, one launch per half step, serve the others,
-// and everything around the time loops.
+// A shot runs with the wavefield on chip (fwi_cluster.cuh) where the grid fits
+// and a step takes less time there (fwi_choice.cuh); the kernels of this file, one
+// launch per half step, serve the others, and everything around the time loops.
 //
 // Layout: every field is [nz][nx][C] (chain fastest), so each warp reads 32
 // chains of one cell in one 128-byte transaction and the stencil neighbours

@@ -620,7 +620,10 @@ typedef struct hmc_fwi {
                                when snapshot_interval <= 1, else per
                                snapshot s = n / k of the steps n = 0, k, 2k,
                                ... [ceil(nt / k)][4][nz][nx][C] (vx, vz after
-                               step n, then after step n - 1)               */
+                               step n, then after step n - 1).  Shots on chip
+                               (hmc_fwi_strips) keep the same planes chain by
+                               chain, [C][nt][2][nz][nx] and
+                               [C][ceil(nt / k)][4][nz][nx]                 */
   float* rec;               /* [shots][nt][nrec][2][C] synthetic records    */
   const float* obs;         /* [shots][nt][nrec][2] observed records        */
   float* resid;             /* [nt][nrec][2][C] weighted residuals (work)   */
