@@ -125,9 +125,8 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
   const uint32_t up_bar = remote_of(smem_of(&bars), has_up ? rank - 1 : rank),
                  down_bar = remote_of(smem_of(&bars), has_down ? rank + 1 : rank);
   uint32_t parity = 0;
-  bool dead = false;
+  bool dead = !halo_awaits(column);  // neither waits, sends nor arms
   const bool sends = halo_sends(column) && !(g.withhold && blockIdx.x == 0 && i == 0);
-  const bool awaits = halo_awaits(column) && bytes;  // some neighbour
   // edge rows of the operands a (rows -1, RZ, RZ + 1) and b (rows -2, -1, RZ) to
   // the neighbours; k numbers the barrier
 #define PUSH(k, a, b)                                                             \
@@ -145,7 +144,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
   }
 #define SETTLE(k)                                          \
   __syncthreads();                                         \
-  if (awaits) {                                            \
+  if (bytes) { /* some neighbour */                        \
     halo_wait(bars, k, parity, g.wait_ns, g.status, dead); \
     if (i == 0 && !dead) halo_arm(bars, k, bytes);         \
   }
@@ -337,7 +336,7 @@ __global__ void __launch_bounds__(PITCH, PITCH == 128 || (PITCH == 192 && RZ <= 
       g.g_bz[k] = gbz[z];
     }
   }
-  halo_drain(dead, g.status);
+  halo_drain(dead && column, g.status);
   cluster_barrier();  // no block leaves while a neighbour may push to it
 #undef SETTLE
 #undef PUSH

@@ -82,9 +82,8 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
   const uint32_t up_bar = remote_of(smem_of(&bars), has_up ? rank - 1 : rank),
                  down_bar = remote_of(smem_of(&bars), has_down ? rank + 1 : rank);
   uint32_t parity = 0;
-  bool dead = false;
+  bool dead = !halo_awaits(column);  // neither waits, sends nor arms
   const bool sends = halo_sends(column) && !(g.withhold && blockIdx.x == 0 && i == 0);
-  const bool awaits = halo_awaits(column) && bytes;  // some neighbour
 
   // Edge rows to the neighbours: fa is differentiated downwards (rows -2, -1,
   // RZ) and fb upwards (rows -1, RZ, RZ + 1); k numbers the barrier.
@@ -111,7 +110,7 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
     }                                                        \
   }                                                          \
   __syncthreads();                                           \
-  if (awaits) {                                              \
+  if (bytes) { /* some neighbour */                          \
     halo_wait(bars, k, parity, g.wait_ns, g.status, dead);   \
     if (i == 0 && !dead) halo_arm(bars, k, bytes);           \
   }
@@ -254,7 +253,7 @@ __global__ void __launch_bounds__(PITCH, (RZ <= 10 ? 512 : 256) / PITCH)
         g.sxz[k] = sxz[z];
       }
   }
-  halo_drain(dead, g.status);
+  halo_drain(dead && column, g.status);
   cluster_barrier();  // no block leaves while a neighbour may push to it
 #undef PUSH
 #undef PUBLISH
